@@ -17,14 +17,20 @@ namespace {
 inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 constexpr int kLabBlocks = 148 * 8;
 
-// sums the per-block partials of bulk_lab_kernel in block order, times the cell volume
+// sums the per-block partials of bulk_lab_kernel in a fixed order (one warp:
+// each lane its blocks, then a tree), times the cell volume
 __global__ void lab_finish_kernel(const double* part, int n, double volume, double* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
   double e = 0.0, s = 0.0;
-  for (int b = 0; b < n; b++) {
+  for (int b = threadIdx.x; b < n; b += 32) {
     e += part[2 * b];
     s += part[2 * b + 1];
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    e += __shfl_down_sync(0xffffffffu, e, o);
+    s += __shfl_down_sync(0xffffffffu, s, o);
+  }
+  if (threadIdx.x != 0) return;
   out[0] = e * volume;
   out[1] = s * volume;
 }
@@ -49,18 +55,16 @@ int clv_bulk_slices(const clv_params* pp, const void* ev, const void* pi, void* 
                              4 * (X + Y + Z + X * Y + X * Z), 4 * (X + Y + Z + X * Y + X * Z + Y * Z),
                              4 * (X + Y + Z + X * Y + X * Z + Y * Z) + X * Y,
                              4 * (X + Y + Z + X * Y + X * Z + Y * Z) + 2 * X * Y, 0};
-  const int n = (int)std::max(X, std::max(Y, Z));
+  const unsigned int nb = (unsigned int)((X + Y + Z + X * Y + X * Z + Y * Z + 255) / 256);
   cudaStream_t s = S(stream);
   dim3 g2((p.ny + 127) / 128, p.nx);
   if (pp->precision == 4) {
     float* o = (float*)out;
-    clv::bulk_slices_kernel<float><<<(n + 127) / 128, 128, 0, s>>>(p, (const float*)ev, o + off[0], o + off[1],
-                                                                    o + off[2], o + off[3], o + off[4], o + off[5]);
+    clv::bulk_slices_kernel<float><<<nb, 256, 0, s>>>(p, (const float*)ev, o);
     if (pi) clv::bulk_pimn_kernel<float><<<g2, 128, 0, s>>>(p, (const float*)pi, o + off[6], o + off[7], o + off[8]);
   } else {
     double* o = (double*)out;
-    clv::bulk_slices_kernel<double><<<(n + 127) / 128, 128, 0, s>>>(p, (const double*)ev, o + off[0], o + off[1],
-                                                                     o + off[2], o + off[3], o + off[4], o + off[5]);
+    clv::bulk_slices_kernel<double><<<nb, 256, 0, s>>>(p, (const double*)ev, o);
     if (pi) clv::bulk_pimn_kernel<double><<<g2, 128, 0, s>>>(p, (const double*)pi, o + off[6], o + off[7], o + off[8]);
   }
   return clv_host::check_cuda("bulk_slices");
@@ -71,12 +75,12 @@ int clv_bulk_sums(const clv_params* pp, const void* ev, const void* pi, double* 
   int rc = clv_host::params_from_abi(pp, &p);
   if (rc) return rc;
   if (!ev || !out) return clv_host::set_error(CLV_ERR_INVALID, "bulk_sums: null buffer");
+  const int blocks = (p.nz + clv::BULK_KL - 1) / clv::BULK_KL * clv::BULK_CLUSTER;
+  constexpr int threads = clv::BULK_KL * clv::BULK_ROWS;
   if (pp->precision == 4)
-    clv::bulk_sums_kernel<float><<<p.nz, clv::BULK_SUM_THREADS, 0, S(stream)>>>(p, (const float*)ev,
-                                                                                (const float*)pi, out);
+    clv::bulk_sums_kernel<float><<<blocks, threads, 0, S(stream)>>>(p, (const float*)ev, (const float*)pi, out);
   else
-    clv::bulk_sums_kernel<double><<<p.nz, clv::BULK_SUM_THREADS, 0, S(stream)>>>(p, (const double*)ev,
-                                                                                 (const double*)pi, out);
+    clv::bulk_sums_kernel<double><<<blocks, threads, 0, S(stream)>>>(p, (const double*)ev, (const double*)pi, out);
   return clv_host::check_cuda("bulk_sums_kernel");
 }
 
