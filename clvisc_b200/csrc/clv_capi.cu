@@ -296,7 +296,7 @@ int hypersf_t(const clv::Params& p, int visc, double tau_old, double tau_new, co
   clv::hsf_mark_kernel<real><<<nb, 256, 0, s>>>(p, (const real*)ev_old, (const real*)ev_new, visc, mark, bcount);
   clv::hsf_scan_kernel<<<1, 1024, 0, s>>>(bcount, (int)nb, count);
   clv::hsf_compact_kernel<<<nb, 256, 0, s>>>(nc, mark, bcount, list);
-  clv::hsf_element_kernel<real><<<148 * 4, 128, 0, s>>>(
+  clv::hsf_element_kernel<real><<<148 * 24, 32 * clv::HSF_WARPS, 0, s>>>(
       p, (const real*)ev_old, (const real*)ev_new, (const real*)pi_old, (const real*)pi_new, (real)tau_old,
       (real)tau_new, visc, list, count, total, (real*)sf, (real*)txyz, (real*)pisf, capacity);
   clv::hsf_advance_kernel<<<1, 1, 0, s>>>(count, total);
