@@ -15,9 +15,12 @@ namespace {
 
 inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
-// surface chunks per rapidity: enough blocks to fill the GPU a few times
+// surface chunks per rapidity: the blocks fill two waves of two resident
+// blocks an SM (592 slots) and stay below them, so that no wave is nearly
+// empty; at least a tile of elements each
 int spectra_chunks(long long n, int ny) {
-  long long want = (148LL * 4 + ny - 1) / ny;
+  const long long slots = 148LL * 4;
+  long long want = std::max(1LL, slots / ny);
   long long most = std::max(1LL, (n + clv::SPEC_TILE - 1) / clv::SPEC_TILE);
   return (int)std::max(1LL, std::min(want, most));
 }
@@ -31,14 +34,15 @@ int spectra_t(const clv_spectra_args* a, void* out, void* scratch, cudaStream_t 
   clv::SpecHadron h{a->mass, a->gspin, a->fermi_boson, a->mu};
   dim3 grid(nchunk, a->ny);
   const int threads = ((a->npt * a->nphi + 31) / 32) * 32;
-  if (a->pisf)
-    clv::spectra_kernel<real, true><<<grid, threads, 0, s>>>(
-        (const real*)a->sf, (const real*)a->pisf, a->n, chunk, h, (real)a->tfrz, (real)a->tcoeff, (const real*)a->y,
-        (const real*)a->pt, (const real*)a->cphi, (const real*)a->sphi, a->npt, a->nphi, part);
+  auto launch = [&](auto kern) {
+    kern<<<grid, threads, 0, s>>>((const real*)a->sf, (const real*)a->pisf, a->n, chunk, h, (real)a->tfrz,
+                                  a->pisf ? (real)a->tcoeff : (real)0, (const real*)a->y, (const real*)a->pt,
+                                  (const real*)a->cphi, (const real*)a->sphi, a->npt, a->nphi, part);
+  };
+  if (threads <= 736)
+    a->pisf ? launch(clv::spectra_kernel<real, true, 736>) : launch(clv::spectra_kernel<real, false, 736>);
   else
-    clv::spectra_kernel<real, false><<<grid, threads, 0, s>>>(
-        (const real*)a->sf, nullptr, a->n, chunk, h, (real)a->tfrz, (real)0, (const real*)a->y, (const real*)a->pt,
-        (const real*)a->cphi, (const real*)a->sphi, a->npt, a->nphi, part);
+    a->pisf ? launch(clv::spectra_kernel<real, true, 1024>) : launch(clv::spectra_kernel<real, false, 1024>);
   clv::spectra_finish_kernel<real><<<(unsigned)((np + 255) / 256), 256, 0, s>>>(part, nchunk, np, (real*)out);
   return clv_host::check_cuda("spectra_kernel");
 }

@@ -15,6 +15,29 @@ BULK = dict(ZETAOS_MAX=0.12, ZETAOS_T0=0.2, ZETAOS_WIDTH=0.05, ZETAOS_SKEW=0.3)
 
 
 @pytest.mark.parametrize('use_float32', [True, False])
+@pytest.mark.parametrize('viscous', [False, True])
+@pytest.mark.parametrize('n', [1, 127, 128, 129, 1800])
+def test_spectra_element_counts(cuda_lib, oracle_mod, use_float32, viscous, n):
+    """One element, a tile's edges, and more chunks than one."""
+    from clvisc_b200.spectra import SmoothSpec
+    rng = np.random.default_rng(n)
+    sf = np.zeros((n, 8))
+    sf[:, 0] = rng.uniform(0.01, 0.02, n)
+    sf[:, 1:4] = rng.uniform(-0.005, 0.005, (n, 3))
+    sf[:, 4:6] = rng.uniform(-0.5, 0.5, (n, 2))
+    sf[:, 6] = rng.uniform(-0.05, 0.05, n)
+    sf[:, 7] = rng.uniform(-4.0, 4.0, n)
+    pi = rng.uniform(-0.006, 0.006, (n, 10)) if viscous else None
+    s = SmoothSpec(sf, 0.137, pi, 12.0, use_float32=use_float32)
+    got = s.calc(211, mu=0.02)
+    want = oracle_mod.spectra(sf, pi, 0.13957, 1.0, -1.0, 0.02, 0.137, 12.0 if viscous else 0.0, s.y, s.pt, s.phi,
+                              use_float32)
+    # the sums' scale: terms of both signs cancel
+    tol = 1e-5 if use_float32 else 1e-11
+    assert np.abs(got - want).max() <= tol * np.abs(want).max()
+
+
+@pytest.mark.parametrize('use_float32', [True, False])
 @pytest.mark.parametrize('grid', [(9, 7, 1), (17, 15, 7), (16, 33, 8), (13, 11, 9), (3, 70, 25)])
 def test_diagnostics_slice_edges(cuda_lib, use_float32, grid):
     """Sums per eta slice with fewer, as many and more slices than a cluster's
