@@ -40,6 +40,9 @@ int wgrad_splits(long long P, int Cin, int Cout) {
   return (int)s;
 }
 constexpr int kRowBlocks = 148 * 2;
+constexpr long long kIndex32 = 1ll << 31;   // the 8-channel kernels index in 32 bits
+// C / 8 channel groups that share a warp evenly
+inline bool group8(int C) { return C % 8 == 0 && C / 8 <= 32 && (C / 8 & (C / 8 - 1)) == 0; }
 
 // clv_unet_set_conv_path: 1 tcgen05 convolutions and weight gradient (default), 2 tcgen05 convolutions
 // with no-swizzle TMA operands and the mma.sync weight gradient, 3 tcgen05 convolutions and the mma.sync
@@ -181,7 +184,7 @@ int wgrad_tma(const WgradArgs& a, float* dw, int accumulate, int max_splits, cud
   int rc = clv_host::check_cuda("wgrad3x3_tma_kernel");
   if (rc) return rc;
   const long long n = 9LL * a.Cin * a.Cout;
-  reduce_partials_kernel<<<nb(n, 256), 256, 0, s>>>(a.part, splits, n, dw, accumulate);
+  reduce_partials(a.part, splits, n, dw, accumulate, s);
   return clv_host::check_cuda("reduce_partials_kernel");
 }
 
@@ -274,7 +277,7 @@ int clv_unet_wgrad3x3(const void* x, int x_cs, int x_co, const void* g, int N, i
   dim3 grid((9 * Cin + WG_BM - 1) / WG_BM, (Cout + WG_BN - 1) / WG_BN, s);
   wgrad3x3_kernel<<<grid, 256, 0, S(stream)>>>(a);
   const long long n = 9LL * Cin * Cout;
-  reduce_partials_kernel<<<nb(n, 256), 256, 0, S(stream)>>>(a.part, s, n, dw, accumulate);
+  reduce_partials(a.part, s, n, dw, accumulate, S(stream));
   return clv_host::check_cuda("wgrad3x3_kernel");
 }
 
@@ -285,8 +288,11 @@ int clv_unet_bias_grad(const void* g, int g_cs, long long P, int C, float* db, v
   if (!g || !db || !scratch || scratch_bytes < clv_unet_rows_scratch_bytes(C))
     return clv_host::set_error(CLV_ERR_INVALID, "unet_bias_grad: bad argument");
   const long long rows = (P + kRowBlocks - 1) / kRowBlocks;
-  colsum_kernel<<<kRowBlocks, 128, 0, S(stream)>>>((const bf16*)g, g_cs, P, C, rows, (float*)scratch);
-  reduce_partials_kernel<<<nb(C, 256), 256, 0, S(stream)>>>((const float*)scratch, kRowBlocks, C, db, 0);
+  if (vec8_ok(g, g_cs, 0) && group8(C))
+    colsum8_kernel<<<kRowBlocks, 512, 0, S(stream)>>>((const bf16*)g, g_cs, P, C, rows, (float*)scratch);
+  else
+    colsum_kernel<<<kRowBlocks, 128, 0, S(stream)>>>((const bf16*)g, g_cs, P, C, rows, (float*)scratch);
+  reduce_partials((const float*)scratch, kRowBlocks, C, db, 0, S(stream));
   return clv_host::check_cuda("colsum_kernel");
 }
 
@@ -294,7 +300,11 @@ int clv_unet_first_fwd(const float* x, const float* w, const float* bias, int N,
                        void* out, int out_cs, int out_co, void* stream) {
   if (!x || !w || !bias || !pre || !out) return clv_host::set_error(CLV_ERR_INVALID, "unet_first_fwd: null");
   const long long n = (long long)N * H * W * C;
-  conv_first_kernel<<<nb(n, 256), 256, 0, S(stream)>>>(x, w, bias, N, H, W, C, (bf16*)pre, (bf16*)out, out_cs, out_co);
+  if (vec8_ok(pre, C, 0) && vec8_ok(out, out_cs, out_co) && n < kIndex32)
+    conv_first8_kernel<<<nb(n / 8, 256), 256, 0, S(stream)>>>(x, w, bias, N, H, W, C, (bf16*)pre, (bf16*)out, out_cs,
+                                                              out_co);
+  else
+    conv_first_kernel<<<nb(n, 256), 256, 0, S(stream)>>>(x, w, bias, N, H, W, C, (bf16*)pre, (bf16*)out, out_cs, out_co);
   return clv_host::check_cuda("conv_first_kernel");
 }
 
@@ -304,8 +314,11 @@ int clv_unet_first_wgrad(const float* x, const void* g, int N, int H, int W, int
     return clv_host::set_error(CLV_ERR_INVALID, "unet_first_wgrad: bad argument");
   const long long P = (long long)N * H * W;
   const long long rows = (P + kRowBlocks - 1) / kRowBlocks;
-  wgrad_first_kernel<<<kRowBlocks, 288, 0, S(stream)>>>(x, (const bf16*)g, N, H, W, C, rows, (float*)scratch);
-  reduce_partials_kernel<<<nb(9 * C, 256), 256, 0, S(stream)>>>((const float*)scratch, kRowBlocks, 9LL * C, dw, 0);
+  if (vec8_ok(g, C, 0) && group8(C) && 3 * C <= 256)
+    wgrad_first8_kernel<<<kRowBlocks, 512, 0, S(stream)>>>(x, (const bf16*)g, N, H, W, C, rows, (float*)scratch);
+  else
+    wgrad_first_kernel<<<kRowBlocks, 288, 0, S(stream)>>>(x, (const bf16*)g, N, H, W, C, rows, (float*)scratch);
+  reduce_partials((const float*)scratch, kRowBlocks, 9LL * C, dw, 0, S(stream));
   return clv_host::check_cuda("wgrad_first_kernel");
 }
 
@@ -320,25 +333,40 @@ int clv_unet_head_bwd(const void* y, int y_cs, int y_co, const void* z, const fl
                       int C, int K, void* gz, float* dwb, void* scratch, size_t scratch_bytes, void* stream) {
   if (!y || !z || !g || !w || !gz || !dwb || !scratch || scratch_bytes < clv_unet_rows_scratch_bytes((C + 1) * K))
     return clv_host::set_error(CLV_ERR_INVALID, "unet_head_bwd: bad argument");
-  head_dgrad_kernel<<<nb(P * C, 256), 256, 0, S(stream)>>>(g, w, (const bf16*)z, P, C, K, (bf16*)gz);
+  const bool v8 = C % 8 == 0 && K <= 8;
+  if (v8 && vec8_ok(z, C, 0) && vec8_ok(gz, C, 0) && P * C < kIndex32)
+    head_dgrad8_kernel<<<nb(P * C / 8, 256), 256, 0, S(stream)>>>(g, w, (const bf16*)z, P, C, K, (bf16*)gz);
+  else
+    head_dgrad_kernel<<<nb(P * C, 256), 256, 0, S(stream)>>>(g, w, (const bf16*)z, P, C, K, (bf16*)gz);
   const long long rows = (P + kRowBlocks - 1) / kRowBlocks;
-  head_wgrad_kernel<<<kRowBlocks, 224, 0, S(stream)>>>((const bf16*)y, y_cs, y_co, g, P, C, K, rows,
-                                                       (float*)scratch);
-  reduce_partials_kernel<<<nb((C + 1) * K, 256), 256, 0, S(stream)>>>((const float*)scratch, kRowBlocks,
-                                                                       (long long)(C + 1) * K, dwb, 0);
+  if (v8 && group8(C) && vec8_ok(y, y_cs, y_co) && C * ((K + 2) / 3) + K <= 256)
+    head_wgrad8_kernel<<<kRowBlocks, 512, 0, S(stream)>>>((const bf16*)y, y_cs, y_co, g, P, C, K, rows,
+                                                           (float*)scratch);
+  else
+    head_wgrad_kernel<<<kRowBlocks, 224, 0, S(stream)>>>((const bf16*)y, y_cs, y_co, g, P, C, K, rows,
+                                                         (float*)scratch);
+  reduce_partials((const float*)scratch, kRowBlocks, (long long)(C + 1) * K, dwb, 0, S(stream));
   return clv_host::check_cuda("head_bwd");
 }
 
 int clv_unet_pool(const void* x, int x_cs, int x_co, int N, int H, int W, int C, void* out, void* stream) {
   if (!x || !out || H % 2 || W % 2) return clv_host::set_error(CLV_ERR_INVALID, "unet_pool: bad argument");
-  pool_kernel<<<nb((long long)N * (H / 2) * (W / 2) * C, 256), 256, 0, S(stream)>>>((const bf16*)x, x_cs, x_co, N, H,
+  const long long n8 = (long long)N * H * W * C;
+  if (vec8_ok(x, x_cs, x_co) && vec8_ok(out, C, 0) && n8 < kIndex32)
+    pool8_kernel<<<nb(n8 / 32, 256), 256, 0, S(stream)>>>((const bf16*)x, x_cs, x_co, N, H, W, C, (bf16*)out);
+  else
+    pool_kernel<<<nb((long long)N * (H / 2) * (W / 2) * C, 256), 256, 0, S(stream)>>>((const bf16*)x, x_cs, x_co, N, H,
                                                                                       W, C, (bf16*)out);
   return clv_host::check_cuda("pool_kernel");
 }
 
 int clv_unet_up(const void* x, int N, int H, int W, int C, void* out, int out_cs, int out_co, void* stream) {
   if (!x || !out) return clv_host::set_error(CLV_ERR_INVALID, "unet_up: null");
-  up_kernel<<<nb((long long)N * 4 * H * W * C, 256), 256, 0, S(stream)>>>((const bf16*)x, N, H, W, C, (bf16*)out,
+  const long long n8 = (long long)N * H * W * C;
+  if (vec8_ok(x, C, 0) && vec8_ok(out, out_cs, out_co) && n8 < kIndex32)
+    up8_kernel<<<nb(n8 / 8, 256), 256, 0, S(stream)>>>((const bf16*)x, N, H, W, C, (bf16*)out, out_cs, out_co);
+  else
+    up_kernel<<<nb((long long)N * 4 * H * W * C, 256), 256, 0, S(stream)>>>((const bf16*)x, N, H, W, C, (bf16*)out,
                                                                           out_cs, out_co);
   return clv_host::check_cuda("up_kernel");
 }
@@ -346,7 +374,12 @@ int clv_unet_up(const void* x, int N, int H, int W, int C, void* out, int out_cs
 int clv_unet_skip_grad(const void* gcat, int gcat_cs, int gcat_co, const void* gpool, const void* z, int N, int H,
                        int W, int C, void* gz, void* stream) {
   if (!gcat || !z || !gz) return clv_host::set_error(CLV_ERR_INVALID, "unet_skip_grad: null");
-  skip_grad_kernel<<<nb((long long)N * H * W * C, 256), 256, 0, S(stream)>>>(
+  const long long n8 = (long long)N * H * W * C;
+  if (vec8_ok(gcat, gcat_cs, gcat_co) && vec8_ok(gpool, C, 0) && vec8_ok(z, C, 0) && vec8_ok(gz, C, 0) && n8 < kIndex32)
+    skip_grad8_kernel<<<nb(n8 / 8, 256), 256, 0, S(stream)>>>((const bf16*)gcat, gcat_cs, gcat_co, (const bf16*)gpool,
+                                                              (const bf16*)z, N, H, W, C, (bf16*)gz);
+  else
+    skip_grad_kernel<<<nb((long long)N * H * W * C, 256), 256, 0, S(stream)>>>(
       (const bf16*)gcat, gcat_cs, gcat_co, (const bf16*)gpool, (const bf16*)z, N, H, W, C, (bf16*)gz);
   return clv_host::check_cuda("skip_grad_kernel");
 }
@@ -354,7 +387,12 @@ int clv_unet_skip_grad(const void* gcat, int gcat_cs, int gcat_co, const void* g
 int clv_unet_up_grad(const void* gcat, int gcat_cs, int gcat_co, const void* z, int N, int H, int W, int C, void* gz,
                      void* stream) {
   if (!gcat || !z || !gz) return clv_host::set_error(CLV_ERR_INVALID, "unet_up_grad: null");
-  up_grad_kernel<<<nb((long long)N * H * W * C, 256), 256, 0, S(stream)>>>((const bf16*)gcat, gcat_cs, gcat_co,
+  const long long n8 = (long long)N * H * W * C;
+  if (vec8_ok(gcat, gcat_cs, gcat_co) && vec8_ok(z, C, 0) && vec8_ok(gz, C, 0) && n8 < kIndex32)
+    up_grad8_kernel<<<nb(n8 / 8, 256), 256, 0, S(stream)>>>((const bf16*)gcat, gcat_cs, gcat_co, (const bf16*)z, N, H,
+                                                            W, C, (bf16*)gz);
+  else
+    up_grad_kernel<<<nb((long long)N * H * W * C, 256), 256, 0, S(stream)>>>((const bf16*)gcat, gcat_cs, gcat_co,
                                                                            (const bf16*)z, N, H, W, C, (bf16*)gz);
   return clv_host::check_cuda("up_grad_kernel");
 }

@@ -911,12 +911,82 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-__global__ void reduce_partials_kernel(const float* part, int S, long long n, float* out, int accumulate) {
+// out[i] (+)= the sum over S partials of part[k][i], in order, a thread an output
+__global__ void __launch_bounds__(256) reduce_partials_kernel(const float* part, int S, long long n, float* out,
+                                                              int accumulate) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float s = 0.0f;
+#pragma unroll 8
   for (int k = 0; k < S; k++) s += part[(long long)k * n + i];
   out[i] = accumulate ? out[i] + s : s;
+}
+// The same sums (the same order) for few outputs: the weight gradients of the
+// small layers and every bias have 32 to a few thousand, and a thread an output
+// was one chain of S dependent reads on a nearly empty chip (20 us a launch, 29
+// launches a training step). A block takes 32 outputs: its 32 warps bring
+// the partials to shared memory, one adds them.
+constexpr int RED_ROWS = 320;
+__global__ void __launch_bounds__(1024) reduce_few_kernel(const float* part, int S, long long n, float* out,
+                                                          int accumulate) {
+  __shared__ float sh[RED_ROWS][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long i = (long long)blockIdx.x * 32 + lane;
+  float s = 0.0f;
+  for (int k0 = 0; k0 < S; k0 += RED_ROWS) {
+    const int m = min(RED_ROWS, S - k0);
+    float v[RED_ROWS / 32];
+#pragma unroll
+    for (int q = 0; q < RED_ROWS / 32; q++)
+      v[q] = i < n && w + 32 * q < m ? part[(long long)(k0 + w + 32 * q) * n + i] : 0.0f;
+    if (k0) __syncthreads();
+#pragma unroll
+    for (int q = 0; q < RED_ROWS / 32; q++) sh[w + 32 * q][lane] = v[q];
+    __syncthreads();
+    if (w == 0 && i < n)
+#pragma unroll 16
+      for (int k = 0; k < m; k++) s += sh[k][lane];
+  }
+  if (w == 0 && i < n) out[i] = accumulate ? out[i] + s : s;
+}
+inline void reduce_partials(const float* part, int S, long long n, float* out, int accumulate, cudaStream_t s) {
+  if (n < 65536) reduce_few_kernel<<<(unsigned int)((n + 31) / 32), 1024, 0, s>>>(part, S, n, out, accumulate);
+  else reduce_partials_kernel<<<(unsigned int)((n + 255) / 256), 256, 0, s>>>(part, S, n, out, accumulate);
+}
+
+// Eight neighbouring channels (16 bytes) a thread for the layers below where
+// C, the strides and the offsets are multiples of 8 and the pointers 16-byte
+// aligned (vec8_ok); else one channel a thread. They move 30 to 100 MB a launch
+// at the first level, and with one 2-byte element and two 64-bit divisions a
+// thread they ran at a tenth of the memory's rate (32 images of 128 x 128, a
+// training step's upsampling 323 us, now 27; skip gradients 240, now 73; first
+// layer 216, now 53).
+struct Vec8 {
+  float v[8];
+};
+__device__ __forceinline__ Vec8 load8(const bf16* p) {
+  const uint4 u = *reinterpret_cast<const uint4*>(p);
+  const unsigned int w[4] = {u.x, u.y, u.z, u.w};
+  Vec8 r;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(&w[i]);
+    r.v[2 * i] = __low2float(h);
+    r.v[2 * i + 1] = __high2float(h);
+  }
+  return r;
+}
+__device__ __forceinline__ void store8(bf16* p, const Vec8& r) {
+  unsigned int w[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const __nv_bfloat162 h = __halves2bfloat162(__float2bfloat16_rn(r.v[2 * i]), __float2bfloat16_rn(r.v[2 * i + 1]));
+    w[i] = *reinterpret_cast<const unsigned int*>(&h);
+  }
+  *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+inline bool vec8_ok(const void* p, int cs, int co) {
+  return (reinterpret_cast<uintptr_t>(p) % 16) == 0 && cs % 8 == 0 && co % 8 == 0;
 }
 
 // column sums of g[P][C] (bias gradient): block b sums rows [b*rows, ...) into part[b][C]
@@ -928,6 +998,57 @@ __global__ void colsum_kernel(const bf16* g, int g_cs, long long P, int C, long 
     for (long long p = p0; p < p1; p++) s += __bfloat162float(g[p * g_cs + c]);
     part[(long long)blockIdx.x * C + c] = s;
   }
+}
+// Sums over the pixels of a block, each output by one thread in pixel order
+// (the order of colsum_kernel, wgrad_first_kernel and head_wgrad_kernel: the
+// same bits). The chain of one output is short work (a few cycles a pixel);
+// what those kernels waited for was a global load in every link of it. Here
+// threads 256 .. 511 of a block bring the next tile of rows to shared memory
+// (16 bytes a load, NV a thread) while the first 256 add up the present one.
+// 32 images of 128 x 128, 32 channels: the first layer's weight gradient 1015 to
+// 89 us, the head's 408 to 44, a bias gradient 110 to 18.
+template <int NV> struct RowTile {
+  static constexpr int NE = 256 * NV * 8;       // elements
+  static constexpr int RMAX = 64 * NV;          // rows at most
+  static __device__ __forceinline__ int rows(int C) { return min(NE / C, RMAX); }
+  // rows p .. of g (up to p1) to dst[row][C]; q: the thread's number, 0 .. 255
+  static __device__ __forceinline__ void load(const bf16* g, long long g_cs, long long p, long long p1, int C, int q,
+                                              bf16* dst) {
+    const int tx = C / 8, n = (int)min((long long)rows(C), p1 - p) * tx;
+    uint4 v[NV];
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+      const int k = q + 256 * i;
+      if (k < n) v[i] = *reinterpret_cast<const uint4*>(g + (p + k / tx) * g_cs + 8 * (k % tx));
+    }
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+      const int k = q + 256 * i;
+      if (k < n) *reinterpret_cast<uint4*>(dst + 8 * k) = v[i];
+    }
+  }
+};
+__global__ void __launch_bounds__(512) colsum8_kernel(const bf16* g, int g_cs, long long P, int C, long long rows,
+                                                      float* part) {
+  typedef RowTile<4> T;
+  __shared__ __align__(16) bf16 sh[2][T::NE];
+  const int t = threadIdx.x, R = T::rows(C);
+  const long long p0 = (long long)blockIdx.x * rows, p1 = p0 + rows < P ? p0 + rows : P;
+  float s = 0.0f;
+  if (t >= 256 && p0 < p1) T::load(g, g_cs, p0, p1, C, t - 256, sh[0]);
+  int b = 0;
+  for (long long p = p0; p < p1; p += R, b ^= 1) {
+    __syncthreads();  // tile b is here, and the one before it has been read
+    if (t >= 256) {
+      if (p + R < p1) T::load(g, g_cs, p + R, p1, C, t - 256, sh[b ^ 1]);
+    } else if (t < C) {
+      const int n = (int)min((long long)R, p1 - p);
+      const bf16* v = sh[b] + t;
+#pragma unroll 16
+      for (int r = 0; r < n; r++) s += __bfloat162float(v[r * C]);
+    }
+  }
+  if (t < C) part[(long long)blockIdx.x * C + t] = s;
 }
 
 // --------------------------------------------------- small layers (CUDA cores)
@@ -967,6 +1088,95 @@ __global__ void wgrad_first_kernel(const float* x, const bf16* g, int N, int H, 
   }
 }
 
+// both with 8 channels a thread: the nine inputs of a pixel are read once for
+// eight outputs; per output the same products in the same order
+__global__ void __launch_bounds__(256) conv_first8_kernel(const float* x, const float* w, const float* bias, int N,
+                                                          int H, int W, int C, bf16* pre, bf16* out, int out_cs,
+                                                          int out_co) {
+  const unsigned int t = blockIdx.x * 256u + threadIdx.x, cg = (unsigned int)C / 8u;
+  const unsigned int p = t / cg, c = 8u * (t % cg);
+  if (p >= (unsigned int)(N * H * W)) return;
+  const int wq = (int)(p % (unsigned int)W), hn = (int)(p / (unsigned int)W), h = hn % H;
+  Vec8 s;
+#pragma unroll
+  for (int i = 0; i < 8; i++) s.v[i] = bias[c + i];
+#pragma unroll
+  for (int tap = 0; tap < 9; tap++) {
+    const int hh = h + tap / 3 - 1, ww = wq + tap % 3 - 1;
+    if (hh < 0 || hh >= H || ww < 0 || ww >= W) continue;
+    const float xv = x[(long long)(hn - h + hh) * W + ww];
+#pragma unroll
+    for (int i = 0; i < 8; i++) s.v[i] += xv * __ldg(w + tap * C + c + i);
+  }
+  store8(pre + (long long)p * C + c, s);
+#pragma unroll
+  for (int i = 0; i < 8; i++) s.v[i] = gelu_f(s.v[i]);
+  store8(out + (long long)p * out_cs + out_co + c, s);
+}
+// wgrad_first_kernel's sums with the tiles of RowTile: a thread has one channel
+// and one row of taps (3 C <= 256). The pixels are consecutive, so a tap's
+// inputs are too: x[p + dr W + ds].
+__global__ void __launch_bounds__(512) wgrad_first8_kernel(const float* x, const bf16* g, int N, int H, int W, int C,
+                                                           long long rows, float* part) {
+  typedef RowTile<2> T;
+  __shared__ __align__(16) bf16 sh[2][T::NE];
+  __shared__ __align__(16) float xs[2][3][T::RMAX + 4];  // x[p - 1 + dr W + i]
+  const int t = threadIdx.x, R = T::rows(C);
+  const long long P = (long long)N * H * W;
+  const long long p0 = (long long)blockIdx.x * rows, p1 = p0 + rows < P ? p0 + rows : P;
+  auto load = [&](long long p, int b) {
+    T::load(g, C, p, p1, C, t - 256, sh[b]);
+    for (int q = t - 256; q < 3 * (T::RMAX + 2); q += 256) {
+      const int d = q / (T::RMAX + 2), i = q - d * (T::RMAX + 2);
+      const long long k = p - 1 + (long long)(d - 1) * W + i;
+      xs[b][d][i] = k >= 0 && k < P ? x[k] : 0.0f;
+    }
+  };
+  float s[3] = {};
+  const int tr = t / C, c = t - tr * C;  // the thread's row of taps and channel (t < 3 C)
+  if (t >= 256 && p0 < p1) load(p0, 0);
+  int h = (int)(p0 / W % H), w = (int)(p0 % W), b = 0;
+  for (long long p = p0; p < p1; p += R, b ^= 1) {
+    __syncthreads();
+    if (t >= 256) {
+      if (p + R < p1) load(p + R, b ^ 1);
+    } else if (t < 3 * C) {
+      const int n = (int)min((long long)R, p1 - p);
+      const bf16* gv = sh[b] + c;
+      const float* xr = xs[b][tr];
+      for (int r = 0; r < n; r += 4) {
+        if (r + 4 <= n && w >= 1 && w + 4 < W && h + tr >= 1 && h + tr <= H) {  // four pixels with all taps inside
+          const float4 a = *reinterpret_cast<const float4*>(xr + r);
+          const float2 e = *reinterpret_cast<const float2*>(xr + r + 4);
+          const float v[6] = {a.x, a.y, a.z, a.w, e.x, e.y};
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const float gj = __bfloat162float(gv[(r + j) * C]);
+#pragma unroll
+            for (int d = 0; d < 3; d++) s[d] += v[j + d] * gj;
+          }
+          w += 4;
+          continue;
+        }
+        for (int j = 0; j < 4 && r + j < n; j++) {
+          const float gj = __bfloat162float(gv[(r + j) * C]);
+          if (h + tr >= 1 && h + tr <= H)
+#pragma unroll
+            for (int d = 0; d < 3; d++)
+              if (w + d >= 1 && w + d <= W) s[d] += xr[r + j + d] * gj;
+          if (++w == W) {
+            w = 0;
+            if (++h == H) h = 0;
+          }
+        }
+      }
+    }
+  }
+  if (t < 3 * C)
+#pragma unroll
+    for (int d = 0; d < 3; d++) part[((long long)blockIdx.x * 9 + tr * 3 + d) * C + c] = s[d];
+}
+
 // head: 1x1 convolution C -> K (FP32 out)
 __global__ void head_fwd_kernel(const bf16* y, int y_cs, int y_co, const float* w /*[C][K]*/, const float* b,
                                 long long P, int C, int K, float* out) {
@@ -998,6 +1208,88 @@ __global__ void head_wgrad_kernel(const bf16* y, int y_cs, int y_co, const float
     for (long long p = p0; p < p1; p++)
       s += (c < C ? __bfloat162float(y[p * y_cs + y_co + c]) : 1.0f) * g[p * K + k];
     part[(long long)blockIdx.x * (C + 1) * K + q] = s;
+  }
+}
+
+// head backward with 8 channels a thread (K <= 8); per output the same order
+__global__ void __launch_bounds__(256) head_dgrad8_kernel(const float* g, const float* w, const bf16* z, long long P,
+                                                          int C, int K, bf16* gz) {
+  const unsigned int t = blockIdx.x * 256u + threadIdx.x, cg = (unsigned int)C / 8u;
+  const unsigned int p = t / cg, c = 8u * (t % cg);
+  if (p >= (unsigned int)P) return;
+  Vec8 s = {};
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    if (k >= K) break;
+    const float gk = g[(long long)p * K + k];
+#pragma unroll
+    for (int i = 0; i < 8; i++) s.v[i] += gk * __ldg(w + (c + i) * K + k);
+  }
+  const Vec8 zv = load8(z + (long long)p * C + c);
+#pragma unroll
+  for (int i = 0; i < 8; i++) s.v[i] = s.v[i] * gelu_grad(zv.v[i]);
+  store8(gz + (long long)p * C + c, s);
+}
+// head_wgrad_kernel's sums with the tiles of RowTile: a thread has one channel
+// and three outputs, the next K threads one bias each (C ceil(K/3) + K <= 256,
+// K <= 8)
+__global__ void __launch_bounds__(512) head_wgrad8_kernel(const bf16* y, int y_cs, int y_co, const float* g,
+                                                          long long P, int C, int K, long long rows, float* part) {
+  typedef RowTile<2> T;
+  __shared__ __align__(16) bf16 sh[2][T::NE];
+  __shared__ __align__(16) float gs[2][9][T::RMAX];  // g[p + r][k] at [k][r]
+  const int t = threadIdx.x, R = T::rows(C), ng = (K + 2) / 3;
+  const long long p0 = (long long)blockIdx.x * rows, p1 = p0 + rows < P ? p0 + rows : P;
+  auto load = [&](long long p, int b) {
+    T::load(y + y_co, y_cs, p, p1, C, t - 256, sh[b]);
+    const int n = (int)min((long long)R, p1 - p) * K;
+    for (int q = t - 256; q < n; q += 256) gs[b][q % K][q / K] = g[p * K + q];
+  };
+  float s[3] = {};
+  const int kg = t / C, c = t - kg * C;
+  const int kb = t - C * ng;  // the bias of threads C ng .. C ng + K - 1
+  if (t >= 256 && p0 < p1) load(p0, 0);
+  int b = 0;
+  for (long long p = p0; p < p1; p += R, b ^= 1) {
+    __syncthreads();
+    const int n = (int)min((long long)R, p1 - p);
+    if (t >= 256) {
+      if (p + R < p1) load(p + R, b ^ 1);
+    } else if (kb < 0) {
+      const bf16* yv = sh[b] + c;
+      const float* gk = gs[b][3 * kg];  // rows K .. 8 are not read for an output that counts
+      int r = 0;
+      for (; r + 4 <= n; r += 4) {
+        float v[3][4];
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          const float4 a = *reinterpret_cast<const float4*>(gk + d * T::RMAX + r);
+          v[d][0] = a.x, v[d][1] = a.y, v[d][2] = a.z, v[d][3] = a.w;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const float yj = __bfloat162float(yv[(r + j) * C]);
+#pragma unroll
+          for (int d = 0; d < 3; d++) s[d] += yj * v[d][j];
+        }
+      }
+      for (; r < n; r++) {
+        const float yj = __bfloat162float(yv[r * C]);
+#pragma unroll
+        for (int d = 0; d < 3; d++) s[d] += yj * gk[d * T::RMAX + r];
+      }
+    } else if (kb < K) {
+#pragma unroll 16
+      for (int r = 0; r < n; r++) s[0] += gs[b][kb][r];
+    }
+  }
+  float* out = part + (long long)blockIdx.x * (C + 1) * K;
+  if (kb < 0) {
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+      if (3 * kg + d < K) out[c * K + 3 * kg + d] = s[d];
+  } else if (kb < K) {
+    out[C * K + kb] = s[0];
   }
 }
 
@@ -1053,6 +1345,76 @@ __global__ void up_grad_kernel(const bf16* gcat, int gcat_cs, int gcat_co, const
     s += __bfloat162float(gcat[p * gcat_cs + gcat_co + c]);
   }
   gz[t] = __float2bfloat16_rn(s * gelu_grad(__bfloat162float(z[t])));
+}
+
+// pooling, upsampling and their gradients with 8 channels a thread; each output
+// is the one-channel kernels' expression
+__global__ void __launch_bounds__(256) pool8_kernel(const bf16* x, int x_cs, int x_co, int N, int H, int W, int C,
+                                                    bf16* out) {
+  const unsigned int t = blockIdx.x * 256u + threadIdx.x, cg = (unsigned int)C / 8u, Ho = H / 2, Wo = W / 2;
+  const unsigned int q = t / cg, c = 8u * (t % cg);
+  if (q >= N * Ho * Wo) return;
+  const unsigned int w = q % Wo, hn = q / Wo, h = hn % Ho, n = hn / Ho;
+  Vec8 s = {};
+#pragma unroll
+  for (int d = 0; d < 4; d++) {
+    const long long p = ((long long)n * H + 2 * h + d / 2) * W + 2 * w + d % 2;
+    const Vec8 v = load8(x + p * x_cs + x_co + c);
+#pragma unroll
+    for (int i = 0; i < 8; i++) s.v[i] += v.v[i];
+  }
+#pragma unroll
+  for (int i = 0; i < 8; i++) s.v[i] = 0.25f * s.v[i];
+  store8(out + (long long)q * C + c, s);
+}
+__global__ void __launch_bounds__(256) up8_kernel(const bf16* x, int N, int H, int W, int C, bf16* out, int out_cs,
+                                                  int out_co) {
+  const unsigned int t = blockIdx.x * 256u + threadIdx.x, cg = (unsigned int)C / 8u;
+  const unsigned int q = t / cg, c = 8u * (t % cg);
+  if (q >= (unsigned int)(N * H * W)) return;  // an input pixel: read once, written four times
+  const unsigned int w = q % (unsigned int)W, hn = q / (unsigned int)W, h = hn % (unsigned int)H, n = hn / (unsigned int)H;
+  const uint4 v = *reinterpret_cast<const uint4*>(x + (long long)q * C + c);
+#pragma unroll
+  for (int d = 0; d < 4; d++) {
+    const long long p = ((long long)n * 2 * H + 2 * h + d / 2) * (2 * W) + 2 * w + d % 2;
+    *reinterpret_cast<uint4*>(out + p * out_cs + out_co + c) = v;
+  }
+}
+__global__ void __launch_bounds__(256) skip_grad8_kernel(const bf16* gcat, int gcat_cs, int gcat_co, const bf16* gpool,
+                                                         const bf16* z, int N, int H, int W, int C, bf16* gz) {
+  const unsigned int t = blockIdx.x * 256u + threadIdx.x, cg = (unsigned int)C / 8u;
+  const unsigned int p = t / cg, c = 8u * (t % cg);
+  if (p >= (unsigned int)(N * H * W)) return;
+  const unsigned int w = p % (unsigned int)W, hn = p / (unsigned int)W, h = hn % (unsigned int)H, n = hn / (unsigned int)H;
+  Vec8 s = load8(gcat + (long long)p * gcat_cs + gcat_co + c);
+  if (gpool) {
+    const Vec8 v = load8(gpool + (((long long)n * (H / 2) + h / 2) * (W / 2) + w / 2) * C + c);
+#pragma unroll
+    for (int i = 0; i < 8; i++) s.v[i] += 0.25f * v.v[i];
+  }
+  const Vec8 zv = load8(z + (long long)p * C + c);
+#pragma unroll
+  for (int i = 0; i < 8; i++) s.v[i] = s.v[i] * gelu_grad(zv.v[i]);
+  store8(gz + (long long)p * C + c, s);
+}
+__global__ void __launch_bounds__(256) up_grad8_kernel(const bf16* gcat, int gcat_cs, int gcat_co, const bf16* z, int N,
+                                                       int H, int W, int C, bf16* gz) {
+  const unsigned int t = blockIdx.x * 256u + threadIdx.x, cg = (unsigned int)C / 8u;
+  const unsigned int q = t / cg, c = 8u * (t % cg);
+  if (q >= (unsigned int)(N * H * W)) return;
+  const unsigned int w = q % (unsigned int)W, hn = q / (unsigned int)W, h = hn % (unsigned int)H, n = hn / (unsigned int)H;
+  Vec8 s = {};
+#pragma unroll
+  for (int d = 0; d < 4; d++) {
+    const long long p = ((long long)n * 2 * H + 2 * h + d / 2) * (2 * W) + 2 * w + d % 2;
+    const Vec8 v = load8(gcat + p * gcat_cs + gcat_co + c);
+#pragma unroll
+    for (int i = 0; i < 8; i++) s.v[i] += v.v[i];
+  }
+  const Vec8 zv = load8(z + (long long)q * C + c);
+#pragma unroll
+  for (int i = 0; i < 8; i++) s.v[i] = s.v[i] * gelu_grad(zv.v[i]);
+  store8(gz + (long long)q * C + c, s);
 }
 
 // weighted squared error: loss partials per block, gradient dL/dout

@@ -67,3 +67,78 @@ def test_diagnostics_slice_edges(cuda_lib, use_float32, grid):
     w2 = 1.0 / (1.0 - vx ** 2 - vy ** 2)[:, :, NZ // 2]
     got = b.plane_sums[-1]
     np.testing.assert_allclose(got[4], (np.sqrt(w2) * e[:, :, NZ // 2]).sum(), rtol=1e-12)
+
+
+def _unet_call(lib, name, *args):
+    import ctypes
+    import torch
+    a = [ctypes.c_void_p(t.data_ptr()) if isinstance(t, torch.Tensor) else t for t in args]
+    assert getattr(lib, name)(*a, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0, name
+
+
+@pytest.mark.parametrize('C,cs,co', [(8, 8, 0), (24, 24, 0), (32, 96, 64), (32, 96, 60), (36, 36, 0), (256, 256, 0)])
+@pytest.mark.parametrize('H', [2, 6])
+def test_unet_small_layers(cuda_lib, C, cs, co, H):
+    """Pooling, upsampling, their gradients, the first layer, the head and the
+    bias sums at channel counts, strides and offsets on either side of the
+    16-byte path, against torch in FP32. BF16 outputs to their rounding (2^-8
+    of the value; one of the scale where terms cancel), FP32 sums over P
+    pixels of products of unit size to P 2^-23."""
+    import ctypes
+    import torch
+    import torch.nn.functional as F
+    lib, N, W, K = cuda_lib, 3, 10, 6
+    g = torch.Generator().manual_seed(C + H)
+    rnd = lambda *s: torch.randn(*s, generator=g).cuda()
+    bf = lambda t: t.to(torch.bfloat16)
+    wide = lambda h, w: bf(rnd(N, h, w, cs))
+    f = lambda t: t[..., co:co + C].float().permute(0, 3, 1, 2)
+    near = lambda got, want: np.testing.assert_allclose(got.float().cpu().numpy(), want.cpu().numpy(), rtol=2.0 ** -8,
+                                                        atol=2.0 ** -8 * 0.01)
+    nhwc = lambda t: t.permute(0, 2, 3, 1)
+    x = wide(H, W)
+    out = torch.zeros(N, H // 2, W // 2, C, dtype=torch.bfloat16, device='cuda')
+    _unet_call(lib, 'clv_unet_pool', x, cs, co, N, H, W, C, out)
+    near(out, nhwc(F.avg_pool2d(f(x), 2)))
+    src, dst = bf(rnd(N, H, W, C)), torch.zeros(N, 2 * H, 2 * W, cs, dtype=torch.bfloat16, device='cuda')
+    _unet_call(lib, 'clv_unet_up', src, N, H, W, C, dst, cs, co)
+    want = torch.zeros_like(dst)
+    want[..., co:co + C] = src.repeat_interleave(2, 1).repeat_interleave(2, 2)
+    assert torch.equal(dst, want)
+    dgelu = lambda z: torch.autograd.functional.jvp(F.gelu, z, torch.ones_like(z))[1]
+    z, gp = bf(rnd(N, H, W, C)), bf(rnd(N, H // 2, W // 2, C))
+    gz = torch.zeros_like(z)
+    _unet_call(lib, 'clv_unet_skip_grad', x, cs, co, gp, z, N, H, W, C, gz)
+    up = gp.float().repeat_interleave(2, 1).repeat_interleave(2, 2)
+    near(gz, (x[..., co:co + C].float() + 0.25 * up) * dgelu(z.float()))
+    big = wide(2 * H, 2 * W)
+    _unet_call(lib, 'clv_unet_up_grad', big, cs, co, z, N, H, W, C, gz)
+    near(gz, nhwc(4.0 * F.avg_pool2d(f(big), 2)) * dgelu(z.float()))
+    # first layer and its weight gradient
+    img, w9, b = rnd(N, H, W), rnd(9, C), rnd(C)
+    pre, y = torch.zeros_like(z), torch.zeros(N, H, W, cs, dtype=torch.bfloat16, device='cuda')
+    _unet_call(lib, 'clv_unet_first_fwd', img, w9, b, N, H, W, C, pre, y, cs, co)
+    k = w9.reshape(3, 3, 1, C).permute(3, 2, 0, 1)
+    zz = nhwc(F.conv2d(img[:, None].double(), k.double(), b.double(), padding=1)).float()
+    near(pre, zz)
+    near(y[..., co:co + C], F.gelu(zz))
+    P = N * H * W
+    tol = dict(rtol=0, atol=16 * P * 2.0 ** -23)
+    nb = int(lib.clv_unet_rows_scratch_bytes(max(9 * C, (C + 1) * K)))
+    scratch = torch.zeros(nb // 4 + 4, device='cuda')
+    dw = torch.zeros(9, C, device='cuda')
+    _unet_call(lib, 'clv_unet_first_wgrad', img, z, N, H, W, C, dw, scratch, ctypes.c_size_t(nb))
+    cols = F.unfold(img[:, None].double(), 3, padding=1)  # (N, 9, HW)
+    want = torch.einsum('ntp,npc->tc', cols, z.double().reshape(N, H * W, C))
+    np.testing.assert_allclose(dw.cpu().numpy(), want.cpu().numpy(), **tol)
+    # head gradients and a bias sum
+    go, wh = rnd(P, K), rnd(C, K)
+    dwb = torch.zeros(C + 1, K, device='cuda')
+    _unet_call(lib, 'clv_unet_head_bwd', x, cs, co, z, go, wh, P, C, K, gz, dwb, scratch, ctypes.c_size_t(nb))
+    near(gz.reshape(P, C), (go.double() @ wh.double().T).float() * dgelu(z.float()).reshape(P, C))
+    xs = x[..., co:co + C].double().reshape(P, C)
+    np.testing.assert_allclose(dwb[:C].cpu().numpy(), (xs.T @ go.double()).cpu().numpy(), **tol)
+    np.testing.assert_allclose(dwb[C].cpu().numpy(), go.double().sum(0).cpu().numpy(), **tol)
+    db = torch.zeros(C, device='cuda')
+    _unet_call(lib, 'clv_unet_bias_grad', z, C, ctypes.c_longlong(P), C, db, scratch, ctypes.c_size_t(nb))
+    np.testing.assert_allclose(db.cpu().numpy(), z.double().reshape(P, C).sum(0).cpu().numpy(), **tol)
