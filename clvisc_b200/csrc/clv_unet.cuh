@@ -558,35 +558,40 @@ __global__ void __launch_bounds__(TMA_THREADS)
 
   if (warp == 0) {
     if (lane == 0) {  // TMA producer
+      // counters in place of divisions: this one thread's instructions, one
+      // after the other, are the pace of a tile with few of them in flight
       long long it = 0;
+      int st = 0;
+      uint32_t round = 0;  // it / TC_STAGES
       bool ok = true;
       for (long long q = blockIdx.x; q < ntiles && ok; q += gridDim.x) {
         int img, h0, w0, n0;
         tile(q, img, h0, w0, n0);
-        for (int ch = 0; ch < kchunks; ch++, it++) {
-          const int st = (int)(it % TC_STAGES);
-          const long long j = it / TC_STAGES;
-          if (j >= 1 && !tc_wait(smem_u32(&s.empty[st]), (uint32_t)((j - 1) & 1))) {
-            ok = false;
-            atomicAdd(&g_tc_timeouts, 1);
-            break;
-          }
-          const int tap = ch / cpt, c0 = (ch % cpt) * TC_BK;
-          const uint32_t fb = smem_u32(&s.full[st]);
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fb), "r"(A_BYTES + B_BYTES)
-                       : "memory");
-          const uint32_t sa = smem_u32(s.A[st]), sb = smem_u32(s.B[st]);
-          if (SW) {
-            tma_load4(sa, &ta, a.in_co + c0, w0 + tap % 3 - 1, h0 + tap / 3 - 1, img, fb);
+        int row = 0;  // tap Cin + c0 of the weights
+        for (int tap = 0; tap < 9 && ok; tap++) {
+          const int wt = w0 + tap % 3 - 1, ht = h0 + tap / 3 - 1;
+          for (int c0 = 0; c0 < a.Cin; c0 += TC_BK, row += TC_BK, it++) {
+            if (round && !tc_wait(smem_u32(&s.empty[st]), (round - 1) & 1)) {
+              ok = false;
+              atomicAdd(&g_tc_timeouts, 1);
+              break;
+            }
+            const uint32_t fb = smem_u32(&s.full[st]);
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fb), "r"(A_BYTES + B_BYTES)
+                         : "memory");
+            const uint32_t sa = smem_u32(s.A[st]), sb = smem_u32(s.B[st]);
+            if (SW) {
+              tma_load4(sa, &ta, a.in_co + c0, wt, ht, img, fb);
 #pragma unroll
-            for (int ng = 0; ng < BN / 32; ng++) tma_load2(sb + ng * 2048, &tb, n0 + 32 * ng, tap * a.Cin + c0, fb);
-          } else {
+              for (int ng = 0; ng < BN / 32; ng++) tma_load2(sb + ng * 2048, &tb, n0 + 32 * ng, row, fb);
+            } else {
 #pragma unroll
-            for (int g = 0; g < TC_BK / 8; g++)
-              tma_load4(sa + g * TC_BM * 16, &ta, a.in_co + c0 + 8 * g, w0 + tap % 3 - 1, h0 + tap / 3 - 1, img, fb);
+              for (int g = 0; g < TC_BK / 8; g++)
+                tma_load4(sa + g * TC_BM * 16, &ta, a.in_co + c0 + 8 * g, wt, ht, img, fb);
 #pragma unroll
-            for (int ng = 0; ng < BN / 8; ng++)
-              tma_load2(sb + ng * TC_BK * 16, &tb, n0 + 8 * ng, tap * a.Cin + c0, fb);
+              for (int ng = 0; ng < BN / 8; ng++) tma_load2(sb + ng * TC_BK * 16, &tb, n0 + 8 * ng, row, fb);
+            }
+            if (++st == TC_STAGES) st = 0, round++;
           }
         }
       }
@@ -596,8 +601,8 @@ __global__ void __launch_bounds__(TMA_THREADS)
     }
   } else if (warp == 1) {
     if (lane == 0) {  // MMA issuer
-      long long it = 0;
-      int t = 0;
+      int t = 0, st = 0;
+      uint32_t round = 0;
       bool ok = true;
       for (long long q = blockIdx.x; q < ntiles && ok; q += gridDim.x, t++) {
         const int acc = t & 1;
@@ -608,9 +613,8 @@ __global__ void __launch_bounds__(TMA_THREADS)
         }
         tc_fence_after();
         const uint32_t dtm = tmem + acc * BN;
-        for (int ch = 0; ch < kchunks; ch++, it++) {
-          const int st = (int)(it % TC_STAGES);
-          if (!tc_wait(smem_u32(&s.full[st]), (uint32_t)((it / TC_STAGES) & 1))) {
+        for (int ch = 0; ch < kchunks; ch++) {
+          if (!tc_wait(smem_u32(&s.full[st]), round & 1)) {
             ok = false;
             atomicAdd(&g_tc_timeouts, 1);
             break;
@@ -622,6 +626,7 @@ __global__ void __launch_bounds__(TMA_THREADS)
             tc_mma(dtm, tc_smem_desc(sa + kh * KSTEP_A, LBO_A, SBO_A, LAYOUT),
                    tc_smem_desc(sb + kh * KSTEP_B, LBO_B, SBO_B, LAYOUT), IDESC, (ch > 0 || kh > 0) ? 1u : 0u);
           tc_commit(smem_u32(&s.empty[st]));
+          if (++st == TC_STAGES) st = 0, round++;
         }
         if (ok) tc_commit(smem_u32(&s.acc_full[acc]));
       }
@@ -831,36 +836,49 @@ __global__ void __launch_bounds__(128)
   const uint32_t tmem = s.tmem;
 
   if (tid == 0) {  // TMA producer
+    int gc[4], gw[4], gh[4];  // rows m0 + 32 i ..: one tap, 32 input channels
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int r0 = m0 + 32 * i, tap = r0 / a.Cin;
+      gc[i] = a.x_co + r0 % a.Cin;
+      gw[i] = tap % 3 - 1;
+      gh[i] = tap / 3 - 1;
+    }
+    int img = (int)(c0 / per_img), q = (int)(c0 % per_img), h0 = (q / per_row) * bh, w0 = (q % per_row) * bw;
     long long it = 0;
+    int st = 0;
+    uint32_t round = 0;  // it / WGT_STAGES
     for (long long c = c0; c < c1; c++, it++) {
-      const int st = (int)(it % WGT_STAGES);
-      const long long j = it / WGT_STAGES;
-      if (j >= 1 && !tc_wait(smem_u32(&s.empty[st]), (uint32_t)((j - 1) & 1))) {
+      if (round && !tc_wait(smem_u32(&s.empty[st]), (round - 1) & 1)) {
         atomicAdd(&g_tc_timeouts, 1);
         break;
       }
-      const int img = (int)(c / per_img), q = (int)(c % per_img);
-      const int h0 = (q / per_row) * bh, w0 = (q % per_row) * bw;
       const uint32_t fb = smem_u32(&s.full[st]);
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fb),
                    "r"((uint32_t)(groups * 32 + nn) * WGT_BK * 2)
                    : "memory");
       const uint32_t sa = smem_u32(s.A[st]), sb = smem_u32(s.B[st]);
-      for (int gi = 0; gi < groups; gi++) {  // rows m0 + 32 gi ..: one tap, 32 input channels
-        const int r0 = m0 + 32 * gi, tap = r0 / a.Cin, ci = r0 % a.Cin;
-        tma_load4(sa + gi * LBO, &tx, a.x_co + ci, w0 + tap % 3 - 1, h0 + tap / 3 - 1, img, fb);
-      }
+#pragma unroll
+      for (int gi = 0; gi < 4; gi++)
+        if (gi < groups) tma_load4(sa + gi * LBO, &tx, gc[gi], w0 + gw[gi], h0 + gh[gi], img, fb);
       for (int ng = 0; ng < nn / 32; ng++) tma_load4(sb + ng * LBO, &tg, co0 + 32 * ng, w0, h0, img, fb);
+      w0 += bw;  // the next pixel block
+      if (w0 == a.W) {
+        w0 = 0;
+        h0 += bh;
+        if (h0 == a.H) h0 = 0, img++;
+      }
+      if (++st == WGT_STAGES) st = 0, round++;
     }
     // the loads in flight land before the CTA can exit
     for (long long c = it - 1; c >= 0 && c >= it - WGT_STAGES; c--)
       tc_wait(smem_u32(&s.full[c % WGT_STAGES]), (uint32_t)((c / WGT_STAGES) & 1));
   } else if (tid == 32) {  // MMA issuer
-    long long it = 0;
+    int st = 0;
+    uint32_t round = 0;
     bool ok = true;
-    for (long long c = c0; c < c1; c++, it++) {
-      const int st = (int)(it % WGT_STAGES);
-      if (!tc_wait(smem_u32(&s.full[st]), (uint32_t)((it / WGT_STAGES) & 1))) {
+    for (long long c = c0; c < c1; c++) {
+      if (!tc_wait(smem_u32(&s.full[st]), round & 1)) {
         ok = false;
         atomicAdd(&g_tc_timeouts, 1);
         break;
@@ -870,11 +888,16 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
       for (int kh = 0; kh < WGT_BK / 16; kh++)
         tc_mma(tmem, tc_smem_desc(sa + kh * KSTEP, LBO, SBO, LAYOUT), tc_smem_desc(sb + kh * KSTEP, LBO, SBO, LAYOUT),
-               idesc, (it > 0 || kh > 0) ? 1u : 0u);
+               idesc, (c > c0 || kh > 0) ? 1u : 0u);
       tc_commit(smem_u32(&s.empty[st]));
+      if (++st == WGT_STAGES) st = 0, round++;
     }
     if (ok && c1 > c0) tc_commit(smem_u32(&s.done));
   }
+  // The other lanes of warps 0 and 1 wait here, not on the barrier: a try_wait
+  // suspends the whole warp for a time, the producer's or the issuer's lane with
+  // it (2.3 us a pixel block, whatever its size, in place of 0.6).
+  __syncwarp();
   bool ready = c1 > c0 ? tc_wait(smem_u32(&s.done), 0) : true;
   tc_fence_after();
   ready = __syncthreads_and(ready);
