@@ -23,7 +23,8 @@ namespace {
 int g_stage_kernel = 0;  // CLV_OPT_STAGE_KERNEL: 0 automatic, 1 per-cell, 2 tiled (3+1)D, 3 tiled (2+1)D
 constexpr int kTiledMinNz = 24;  // fewer cells along eta: per-cell kernel
 constexpr int kTiled2dMin = 4;   // (2+1)D tiles: at least this many cells along x and y
-int g_chunk = 32;        // CLV_OPT_CHUNK: x planes per tiled CTA
+constexpr int kChunkDefault = 32;  // CLV_OPT_CHUNK's default: the split is chosen from the grid (clv::march_chunk)
+int g_chunk = kChunkDefault;  // CLV_OPT_CHUNK: x planes per tiled CTA
 int g_minb = 2;          // CLV_OPT_TILED_BLOCKS: resident tiled CTAs per SM (FP32)
 int g_tile = 0;          // CLV_OPT_TILE: 0 = 8 x 32, 1 = 16 x 16, 2 = 8 x 16 (y, eta) tile of the fused stage
 int g_rows2d = 64;       // CLV_OPT_TILE2D_ROWS: threads of a (2+1)D tile block (64 or 128)
@@ -124,7 +125,7 @@ inline unsigned int nblk(long long n, int bs) { return (unsigned int)((n + bs - 
 clv::StageOpts stage_opts(const clv::Params& p) {
   clv::StageOpts o;
   o.stage_kernel = p.opt[0] ? p.opt[0] - 1 : g_stage_kernel;
-  o.chunk = p.opt[1] ? p.opt[1] : g_chunk;
+  o.chunk = p.opt[1] ? p.opt[1] : (g_chunk == kChunkDefault ? 0 : g_chunk);
   o.minb = p.opt[2] ? p.opt[2] : g_minb;
   o.tile = p.opt[3] ? p.opt[3] - 1 : g_tile;
   o.rows2d = g_rows2d;
@@ -145,8 +146,9 @@ int launch_tiled_b(const clv::Params& p, const clv::ViscBuffers<real>& v, int st
       return cuda_check("cudaFuncSetAttribute(visc_stage_tiled_kernel)");
     configured[dev] = true;
   }
-  const int chunk = o.chunk;
-  dim3 grid((p.nz + TK - 1) / TK, (p.ny + TJ - 1) / TJ, (p.nx + chunk - 1) / chunk);
+  const int gz = (p.nz + TK - 1) / TK, gy = (p.ny + TJ - 1) / TJ;
+  const int chunk = o.chunk ? o.chunk : clv::march_chunk(p.nx, (long long)gz * gy, clv::sm_count() * MINB);
+  dim3 grid(gz, gy, (p.nx + chunk - 1) / chunk);
   kern<<<grid, TJ * TK, sizeof(SM), s>>>(p, v, step, tau_const<real>(p, tau), chunk);
   return cuda_check("visc_stage_tiled_kernel");
 }

@@ -36,7 +36,9 @@ int launch_tiled(const clv::Params& p, const clv::ViscBuffers<real>& v, int step
       return clv_host::check_cuda("cudaFuncSetAttribute(fast visc_stage_tiled_kernel)");
     configured[dev] = true;
   }
-  dim3 grid((p.nz + TK - 1) / TK, (p.ny + TJ - 1) / TJ, (p.nx + chunk - 1) / chunk);
+  const int gz = (p.nz + TK - 1) / TK, gy = (p.ny + TJ - 1) / TJ;
+  if (!chunk) chunk = clv::march_chunk(p.nx, (long long)gz * gy, clv::sm_count() * MINB);
+  dim3 grid(gz, gy, (p.nx + chunk - 1) / chunk);
   kern<<<grid, TJ * TK, sizeof(SM), s>>>(p, v, step, tc, chunk);
   return clv_host::check_cuda("fast visc_stage_tiled_kernel");
 }
@@ -66,7 +68,7 @@ int visc_stage(const clv::Params& p, const clv::ViscBuffers<real>& v, int step, 
                const clv::StageOpts& o, cudaStream_t s) {
   const bool bulk = p.flags & clv::FLAG_BULK;
   const bool cpl = p.flags & (clv::FLAG_GUBSER_VISC | clv::FLAG_PIMN_OMEGA | clv::FLAG_OMEGA_OMEGA);
-  if (o.chunk < 1) return clv_host::set_error(CLV_ERR_INVALID, "fast visc stage: chunk must be >= 1");
+  if (o.chunk < 0) return clv_host::set_error(CLV_ERR_INVALID, "fast visc stage: chunk must be >= 1");
   if (!bulk && (o.stage_kernel == 2 || (o.stage_kernel != 1 && p.nz >= kTiledMinNz))) {
     if (cpl) return launch_tiled<real, true, 1, 8, 32>(p, v, step, tc, o.chunk, s);
     // 16 x 16 and 8 x 16 (y, eta) tiles as in the exact build (CLV_OPT_TILE 1, 2)
