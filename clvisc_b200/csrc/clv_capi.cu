@@ -1,4 +1,5 @@
 // extern "C" entry points of libclvisc_b200.so (declared in include/clvisc_b200.h).
+#include <algorithm>
 #include <cfloat>
 #include <cstdio>
 #include <cstring>
@@ -71,6 +72,9 @@ int to_params(const clv_params* in, clv::Params* out) {
   p.nxskip = in->nxskip; p.nyskip = in->nyskip; p.nzskip = in->nzskip;
   p.eos_start = in->eos_ed_start; p.eos_step = in->eos_ed_step;
   p.eos_num = in->eos_num_ed; p.eos_nrow = in->eos_nrow; p.eos_ncol = in->eos_ncol;
+  p.eos_last = (int)std::min((long long)in->eos_nrow * in->eos_ncol, 1ll << 30) - 1;
+  p.eos_top = in->eos_ed_start + in->eos_num_ed * in->eos_ed_step;
+  p.eos_inner = std::min(p.eos_top, in->eos_ed_start + (float)p.eos_last * in->eos_ed_step);
   p.eos = in->eos_table;
   p.eos_p2 = reinterpret_cast<const float2*>(in->eos_p2);
   if (in->eos_p2 && (reinterpret_cast<uintptr_t>(in->eos_p2) % 8))
@@ -133,11 +137,11 @@ clv::StageOpts stage_opts(const clv::Params& p) {
   return o;
 }
 
-template <class real, bool IS, bool KT, bool CPL, int MINB, int TJ = 8, int TK = 32>
-int launch_tiled_b(const clv::Params& p, const clv::ViscBuffers<real>& v, int step, double tau, cudaStream_t s,
+template <class real, bool IS, bool KT, bool CPL, int MINB, int TJ, int TK, int STAGE>
+int launch_tiled_s(const clv::Params& p, const clv::ViscBuffers<real>& v, int step, double tau, cudaStream_t s,
                    const clv::StageOpts& o) {
   typedef clv::TileSmem<real, TJ, TK> SM;
-  auto kern = clv::visc_stage_tiled_kernel<real, IS, KT, CPL, TJ, TK, MINB>;
+  auto kern = clv::visc_stage_tiled_kernel<real, IS, KT, CPL, TJ, TK, MINB, false, STAGE>;
   static bool configured[kMaxDev] = {};  // the attribute is per device
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return cuda_check("cudaGetDevice");
@@ -151,6 +155,18 @@ int launch_tiled_b(const clv::Params& p, const clv::ViscBuffers<real>& v, int st
   dim3 grid(gz, gy, (p.nx + chunk - 1) / chunk);
   kern<<<grid, TJ * TK, sizeof(SM), s>>>(p, v, step, tau_const<real>(p, tau), chunk);
   return cuda_check("visc_stage_tiled_kernel");
+}
+
+// the fused default shape (8 x 32) comes per stage
+template <class real, bool IS, bool KT, bool CPL, int MINB, int TJ = 8, int TK = 32>
+int launch_tiled_b(const clv::Params& p, const clv::ViscBuffers<real>& v, int step, double tau, cudaStream_t s,
+                   const clv::StageOpts& o) {
+  if constexpr (IS && KT && !CPL && TJ == 8 && TK == 32 && (sizeof(real) == 8 || MINB == 2)) {
+    const int kind = clv::stage_kind(v, step);
+    if (kind == 1) return launch_tiled_s<real, IS, KT, CPL, MINB, TJ, TK, 1>(p, v, step, tau, s, o);
+    if (kind == 2) return launch_tiled_s<real, IS, KT, CPL, MINB, TJ, TK, 2>(p, v, step, tau, s, o);
+  }
+  return launch_tiled_s<real, IS, KT, CPL, MINB, TJ, TK, 0>(p, v, step, tau, s, o);
 }
 
 template <class real, bool BULK, int TB>
@@ -223,22 +239,24 @@ int visc_stage_t(const clv::Params& p, int step, double tau, int parts, const cl
   const bool cpl0 = p.flags & (clv::FLAG_GUBSER_VISC | clv::FLAG_PIMN_OMEGA | clv::FLAG_OMEGA_OMEGA);
   // tolerance arithmetic (CLV_FLAG_FAST) for the fused stage
   if ((p.flags & clv::FLAG_FAST) && is && kt) return clv_fastpath::visc_stage<real>(p, v, step, tau_const<real>(p, tau), o, s);
-  // the tiled (2+1)D kernel (bulk sector, no coupling terms) when asked for:
-  // on B200 the per-cell kernel is faster on the (2+1)D grids of this code
+  // the marching (2+1)D kernel (bulk sector, no coupling terms) when asked
+  // for: the per-cell kernel is faster on the (2+1)D grids of this code
   const bool fit2d = p.nz == 1 && p.nx >= kTiled2dMin && p.ny >= kTiled2dMin && is && kt && !cpl0;
   if (fit2d && o.stage_kernel == 3)
     return bulk ? launch_tiled2d<real, true>(p, v, step, tau, s) : launch_tiled2d<real, false>(p, v, step, tau, s);
-  // The tiled kernel has no bulk sector, and its 8 x 32 (y, eta) tile leaves
-  // most threads idle on grids with few cells along eta ((2+1)D runs have
-  // one): those runs take the per-cell kernel, which gives the same bits.
-  if (!bulk && (o.stage_kernel == 2 || (o.stage_kernel == 0 && p.nz >= kTiledMinNz))) {
+  // The exact tiled kernel has no bulk sector, and its 8 x 32 (y, eta) tile
+  // leaves most threads idle on grids with few cells along eta, and it counts
+  // offsets in 32 bits: other runs take the per-cell kernel, which gives the
+  // same bits.  97 x 93 x 65 FP64, one step:
+  // 2.11 ms tiled (3.79 ms before the update shared its loads).
+  if (!bulk && clv::fits_idx32<real>(p) && (o.stage_kernel == 2 || (o.stage_kernel == 0 && p.nz >= kTiledMinNz))) {
     if (is && kt) return launch_tiled<real, true, true>(p, v, step, tau, s, o);
     if (is) return launch_tiled<real, true, false>(p, v, step, tau, s, o);
     return launch_tiled<real, false, true>(p, v, step, tau, s, o);
   }
+  const clv::TauConst<real> t = tau_const<real>(p, tau);
   const int bs = 128;
   dim3 grid(nblk(ncell(p), bs));
-  const clv::TauConst<real> t = tau_const<real>(p, tau);
   const bool cpl = p.flags & (clv::FLAG_GUBSER_VISC | clv::FLAG_PIMN_OMEGA | clv::FLAG_OMEGA_OMEGA);
   if (bulk) {
     if (is && kt && cpl) clv::visc_stage_kernel<real, true, true, true, true><<<grid, bs, 0, s>>>(p, v, step, t);

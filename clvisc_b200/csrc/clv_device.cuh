@@ -48,6 +48,9 @@ struct Params {
   int nxskip, nyskip, nzskip;
   float eos_start, eos_step;
   int eos_num, eos_nrow, eos_ncol;
+  int eos_last;    // nrow*ncol - 1, the last texel
+  float eos_top;   // start + num*step as the kernels form it: the table's end
+  float eos_inner; // start + (last texel)*step: below it a lookup's two texels are neighbours
   const float* eos;  // nrow*ncol texels of (cs2, p, T, s)
   const float2* eos_p2;  // optional: pairs (p[t], p[t+1]) of the pressure column (tolerance build)
   int flags;
@@ -188,6 +191,44 @@ template <class real> __device__ __forceinline__ real div_step(real x, int step)
   return step == 2 ? x * (real)0.5f : x;
 }
 
+#if CLV_FAST
+// FP64 quotient, reciprocal square root and square root of the tolerance
+// build: the hardware's approximation (20 bits or more) and two Newton-Raphson
+// steps, x <- x + x (1 - b x) and x <- x + x (1 - a x^2) / 2, each doubling the
+// correct bits (about 1e-16 of the result; the tolerance is 1e-11), without
+// the branches of the library's correctly rounded forms. Arguments are
+// normal numbers away from the range's ends: energy densities, velocities and
+// their sums, floored where they can vanish.
+__device__ __forceinline__ double fast_rcp(double b) {
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(b));
+  x = fma(x, fma(-b, x, 1.0), x);
+  return fma(x, fma(-b, x, 1.0), x);
+}
+__device__ __forceinline__ double fast_rsqrt(double a) {
+  double x;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
+  x = fma(0.5 * x, fma(-a * x, x, 1.0), x);
+  return fma(0.5 * x, fma(-a * x, x, 1.0), x);
+}
+__device__ __forceinline__ float fast_rsqrt(float a) { return rsqrt(a); }
+// the integer below x (as an int and as a double) for |x| < 2^31, by adding
+// 3 * 2^51 to x - 1/2: no conversion instructions. At an integer x either
+// neighbour may come out, where a piecewise linear function has one value.
+__device__ __forceinline__ double fast_floor(double x, int& i) {
+  const double t = (x - 0.5) + 6755399441055744.0;
+  i = __double2loint(t);
+  return t - 6755399441055744.0;
+}
+#endif
+// quotient and reciprocal of per-cell values
+template <class real> __device__ __forceinline__ real quot(real a, real b) {
+#if CLV_FAST
+  if constexpr (sizeof(real) == 8) return a * fast_rcp(b);
+#endif
+  return a / b;
+}
+
 // ------------------------------------------------------------------ EOS
 // Table lookup of eos_table.h:39-62: row/col from the energy density, two
 // nearest texels (the second wraps to the next row), clamp-to-edge, lerp.
@@ -204,6 +245,27 @@ template <class real> __device__ __forceinline__ real div_step(real x, int step)
 template <class real> __device__ __forceinline__ EosSpot<real> eos_spot(const Params& p, real eps) {
   const Recips<real>& rc = recips<real>(p);
   real ed_per_row = p.eos_step * p.eos_ncol;
+#if CLV_FAST
+  if constexpr (sizeof(real) == 8) {
+    // the same row, column and weight, the reference's float roundings of the
+    // row width and of col * step included, from two additions each in place of
+    // the double conversions; inside the table t1 is the texel after t0 (the
+    // last column's next is the next row's first), except where the rounded row
+    // width leaves a column beyond the last, which reads the last twice
+    if (eps < p.eos_inner) {
+      int row, col;
+      const double rowd = fast_floor(eps * rc.eos_epr, row);
+      const double x = eps - p.eos_start - rowd * ed_per_row;
+      fast_floor(x * rc.eos_step, col);
+      const int t = row * p.eos_ncol + min(col, p.eos_ncol - 1);
+      EosSpot<real> s;
+      s.t0 = min(max(t, 0), p.eos_last);
+      s.t1 = min(max(t + (col < p.eos_ncol ? 1 : 0), 0), p.eos_last);
+      s.r = (x - (double)((float)col * p.eos_step)) * rc.eos_step;
+      return s;
+    }
+  }
+#endif
   int row = (int)div_by<real>(eps, ed_per_row, rc.eos_epr);
   int col = (int)div_by<real>(eps - p.eos_start - row * ed_per_row, (real)p.eos_step, rc.eos_step);
   real eps_low = p.eos_start + row * ed_per_row + col * p.eos_step;
@@ -223,8 +285,72 @@ template <class real> __device__ __forceinline__ EosSpot<real> eos_spot(const Pa
 template <class real> __device__ __forceinline__ real eos_lerp(real r, float lo, float hi) {
   return (real)(1.0f - r) * (real)lo + r * (real)hi;
 }
+#if CLV_FAST
+// Tolerance build, FP32: the texel straight from x = (eps - start) / step, no
+// row and column. The reference's row/col arithmetic (above) rounds at the
+// same places to the same 2^-24 of x (the two differ by less than x ulps of
+// the weight, 6e-8 of the pressure at the table's end); in FP64 its
+// float-rounded row width moves the result by 1e-9, so FP64 keeps it. About
+// 10 instructions and one conversion on the dependent chain of a lookup
+// against 35 and two: the chain sits inside the root finder's loop. Below
+// eos_inner only: the last texel and beyond (where the row/col clamps decide
+// what is read) take the reference's way.
+struct EosAt {
+  int t;    // texel, clamped to the table
+  float r;  // weight of the next one
+};
+__device__ __forceinline__ EosAt eos_at(const Params& p, float eps) {
+  const float x = (eps - p.eos_start) * p.rf.eos_step;
+  const int i = (int)x;
+  return EosAt{min(max(i, 0), p.eos_last), x - (float)i};
+}
+#endif
+#if CLV_FAST
+// The reference's lookup and its formula beyond the table, out of line (one
+// copy a kernel of the power and exponential): the last texel and beyond. The
+// constants go by value: a reference would put the kernel's parameters in
+// local memory.
+struct EosEdge {
+  const float* eos;
+  float start, step, rstep, repr, top;
+  int ncol, nrow;
+};
+__device__ __forceinline__ EosEdge eos_edge(const Params& p) {
+  return EosEdge{p.eos, p.eos_start, p.eos_step, p.rf.eos_step, p.rf.eos_epr, p.eos_top, p.eos_ncol, p.eos_nrow};
+}
+static __device__ __noinline__ float eos_comp_edge(EosEdge g, float eps, int c) {
+  Params p;
+  p.eos_start = g.start;
+  p.eos_step = g.step;
+  p.eos_ncol = g.ncol;
+  p.eos_nrow = g.nrow;
+  p.rf.eos_step = g.rstep;
+  p.rf.eos_epr = g.repr;
+  const EosSpot<float> s = eos_spot<float>(p, eps);
+  return eos_lerp<float>(s.r, __ldg(g.eos + 4 * s.t0 + c), __ldg(g.eos + 4 * s.t1 + c));
+}
+static __device__ __noinline__ float eosP_edge(EosEdge g, float eps) {
+  if (eps < g.top) return eos_comp_edge(g, eps, 1);
+  return 0.3327f * eps - 0.3223f * pow(eps, 0.4585f) - 0.003906f * eps * exp(-0.05697f * eps);
+}
+#endif
 template <class real>
 __device__ CLV_EOS_ATTR real eos_comp(const Params& p, real eps, int c) {
+#if CLV_FAST
+  if constexpr (sizeof(real) == 4) {
+    if (eps < p.eos_inner) {
+      const EosAt a = eos_at(p, eps);
+      if (c == 1 && p.eos_p2) {
+        const float2 q = __ldg(p.eos_p2 + a.t);
+        return q.x + a.r * (q.y - q.x);
+      }
+      const float lo = __ldg(p.eos + 4 * (long long)a.t + c);
+      const float hi = __ldg(p.eos + 4 * (long long)min(a.t + 1, p.eos_last) + c);
+      return lo + a.r * (hi - lo);
+    }
+    return eos_comp_edge(eos_edge(p), eps, c);
+  }
+#endif
   const EosSpot<real> s = eos_spot<real>(p, eps);
 #if CLV_FAST
   // tolerance build: the pressure from one 8-byte read of the pair table
@@ -242,6 +368,22 @@ __device__ CLV_EOS_ATTR real eos_comp(const Params& p, real eps, int c) {
 // 16-byte texel reads; component c equals eos_comp(p, eps, c) bit for bit
 // (the table is 16-byte aligned: the library checks it)
 template <class real> __device__ __forceinline__ void eos_texel4(const Params& p, real eps, real out[4]) {
+#if CLV_FAST
+  if constexpr (sizeof(real) == 4) {
+    if (eps < p.eos_inner) {
+      const EosAt a = eos_at(p, eps);
+      const float4 l = __ldg(reinterpret_cast<const float4*>(p.eos) + a.t);
+      const float4 h = __ldg(reinterpret_cast<const float4*>(p.eos) + min(a.t + 1, p.eos_last));
+      out[0] = l.x + a.r * (h.x - l.x);
+      out[1] = l.y + a.r * (h.y - l.y);
+      out[2] = l.z + a.r * (h.z - l.z);
+      out[3] = l.w + a.r * (h.w - l.w);
+      return;
+    }
+    for (int c = 0; c < 4; c++) out[c] = eos_comp_edge(eos_edge(p), eps, c);
+    return;
+  }
+#endif
   const EosSpot<real> s = eos_spot<real>(p, eps);
   const float4 lo = __ldg(reinterpret_cast<const float4*>(p.eos) + s.t0);
   const float4 hi = __ldg(reinterpret_cast<const float4*>(p.eos) + s.t1);
@@ -251,13 +393,35 @@ template <class real> __device__ __forceinline__ void eos_texel4(const Params& p
   out[3] = eos_lerp<real>(s.r, lo.w, hi.w);
 }
 template <class real> __device__ __forceinline__ bool eos_in_table(const Params& p, real eps) {
-  return eps < p.eos_start + p.eos_num * p.eos_step;
+  return eps < p.eos_top;
 }
 // P(e): eos_table.h:65-71
 template <class real> __device__ __forceinline__ real eosP(const Params& p, real eps) {
+#if CLV_FAST
+  if constexpr (sizeof(real) == 4) return eps < p.eos_inner ? eos_comp<real>(p, eps, 1) : eosP_edge(eos_edge(p), eps);
+#endif
   if (eos_in_table(p, eps)) return eos_comp(p, eps, 1);
   return 0.3327f * eps - 0.3223f * pow(eps, (real)0.4585f) - 0.003906f * eps * exp(-0.05697f * eps);
 }
+#if CLV_FAST
+// pressure and its table slope dP/de (1/3 beyond the table, as the root
+// finder's derivative takes it there)
+__device__ __forceinline__ float eos_p_slope(const Params& p, float eps, float& dpe) {
+  dpe = 1.0f / 3.0f;
+  if (!(eps < p.eos_inner)) return eosP_edge(eos_edge(p), eps);
+  const EosAt a = eos_at(p, eps);
+  float2 q;
+  if (p.eos_p2) {
+    q = __ldg(p.eos_p2 + a.t);
+  } else {
+    q.x = __ldg(p.eos + 4 * (long long)a.t + 1);
+    q.y = __ldg(p.eos + 4 * (long long)min(a.t + 1, p.eos_last) + 1);
+  }
+  const float d = q.y - q.x;
+  dpe = d * p.rf.eos_step;
+  return q.x + a.r * d;
+}
+#endif
 // CS2(e): eos_table.h:94-100
 template <class real> __device__ __forceinline__ real eosCS2(const Params& p, real eps) {
   if (eos_in_table(p, eps)) return eos_comp(p, eps, 0);
@@ -267,7 +431,7 @@ template <class real> __device__ __forceinline__ real eosCS2(const Params& p, re
 // ---------------------------------------------------------------- helper.h
 template <class real> __device__ __forceinline__ real gamma3(real vx, real vy, real vz) {  // helper.h:46-48
 #if CLV_FAST
-  return rsqrt(cmax<real>(1.0f - vx * vx - vy * vy - vz * vz, Acu<real>::v));
+  return fast_rsqrt(cmax<real>(1.0f - vx * vx - vy * vy - vz * vz, Acu<real>::v));
 #else
   return 1.0f / sqrt(cmax<real>(1.0f - vx * vx - vy * vy - vz * vz, Acu<real>::v));
 #endif
@@ -283,6 +447,16 @@ template <class real> __device__ __forceinline__ real minmod(real x, real y) {  
 // below, in a few instructions
 template <class real> __device__ __forceinline__ real gminmod(real a, real b) {
   const real TH = CLV_THETA;
+  if constexpr (sizeof(real) == 8) {
+    // FP64 has no min instruction: with one sign all three candidates carry
+    // it, so the smaller magnitudes are picked by compare and select (the
+    // same value; the library fmin, fabs and copysign take twice the
+    // instructions)
+    const real m = TH * (fabs(b) < fabs(a) ? b : a);
+    const real h = (real)0.5f * (a + b);
+    const real r = fabs(h) < fabs(m) ? h : m;
+    return (a * b > (real)0) ? r : (real)0;
+  }
   const real m = fmin(TH * fmin(fabs(a), fabs(b)), (real)0.5f * fabs(a + b));
   return (a * b > (real)0) ? copysign(m, a) : (real)0;
 }
@@ -325,15 +499,11 @@ __device__ __forceinline__ real max_speed(const Params& p, real e, real vx, real
 // helper.h:128-167; returns the energy density. With BULK the pressure is
 // P(e) + bulk, the bulk viscous pressure of the cell.
 template <class real, bool BULK = false>
-__device__ __forceinline__ real root_newton(const Params& p, real T00, real M, real bulk = (real)0.0f,
-                                            real v_start = (real)-1.0f) {
+__device__ __forceinline__ real root_newton(const Params& p, real T00, real M, real bulk = (real)0.0f) {
   real vl = 0.0f;
   real vh = 1.0f;
   real dpe = 1.0f / 3.0f;
-  // the reference starts at the middle of the bracket; a start in [0, 1)
-  // (the tolerance build passes the cell's speed at the start of the step)
-  // leaves the bracket and the safeguards as they are
-  real v = v_start >= (real)0.0f ? v_start : 0.5f * (vl + vh);
+  real v = 0.5f * (vl + vh);
   real ed = T00 - M * v;
   real pr = eosP<real>(p, ed);
   if (BULK) pr = pr + bulk;
@@ -349,7 +519,7 @@ __device__ __forceinline__ real root_newton(const Params& p, real T00, real M, r
       v = vl + dv;
     } else {
       dvold = dv;
-      dv = f / df;
+      dv = quot<real>(f, df);
       v -= dv;
     }
     i++;
@@ -367,6 +537,54 @@ __device__ __forceinline__ real root_newton(const Params& p, real T00, real M, r
   }
   return T00 - M * v;
 }
+#if CLV_FAST
+// The FP32 tolerance build's root finder: the same equation, bracket,
+// safeguards and stopping rule (a step below 1e-5). Every evaluation of the
+// reference's finder is a dependent table read out of L2, four to five of them
+// a cell at the end of the cell's longest chain. This one starts from the root
+// of the equation with P(e) linear about (er, pr, cs2), an energy density near
+// the new one that the pi update has looked up (a quadratic: no table read), takes the
+// table's own dP/de from the texels of each evaluation, and returns the
+// pressure at the root from the last evaluation's segment: most cells read the
+// table once. (FP64, with its tolerance of 1e-11, keeps the reference's
+// iterates: where the finder stops within 1e-5 depends on them.)
+template <bool BULK>
+__device__ __forceinline__ float root_near(const Params& p, float T00, float M, float bulk, float er, float pr0,
+                                           float cs2, float& pr_out) {
+  // cs2 M v^2 - b v + M = 0, b = T00 + P + cs2 (T00 - er): the smaller root
+  const float b = T00 + pr0 + (BULK ? bulk : 0.0f) + cs2 * (T00 - er);
+  const float disc = b * b - 4.0f * cs2 * M * M;
+  float v = 2.0f * M / (b + sqrtf(fmaxf(disc, 0.0f)));
+  if (!(v >= 0.0f && v <= 1.0f)) v = 0.5f;
+  float vl = 0.0f, vh = 1.0f, dv = 1.0f, dvold = 1.0f, ed, pt, dpe;
+  int i = 0;
+  while (true) {
+    ed = T00 - M * v;
+    pt = eos_p_slope(p, ed, dpe);
+    const float pr = BULK ? pt + bulk : pt;
+    const float f = (T00 + pr) * v - M;
+    const float df = (T00 + pr) - M * v * dpe;
+    if (i > 0) {
+      if (f > 0.0f) vh = v;
+      else vl = v;
+    }
+    if ((f + df * (vh - v)) * (f + df * (vl - v)) > 0.0f || fabsf(2.f * f) > fabsf(dvold * df)) {
+      dvold = dv;
+      dv = 0.5f * (vh - vl);
+      v = vl + dv;
+    } else {
+      dvold = dv;
+      dv = f / df;
+      v -= dv;
+    }
+    i++;
+    if (fabsf(dv) < 0.00001f || i > 100) break;
+  }
+  const float e = T00 - M * v;
+  pr_out = (fabsf(dv) < 0.00001f && ed < p.eos_inner) ? pt + dpe * (e - ed) : eosP<float>(p, e);
+  return e;
+}
+#endif
 
 // Bulk sector (no counterpart in the reference): zeta/s(T) as a skewed Cauchy
 // peak, ZETAOS_MAX w^2 / (w^2 + (T - T0)^2), w = WIDTH (1 + SKEW sign(T - T0))
@@ -499,29 +717,27 @@ __device__ __forceinline__ unsigned long long fkey(double f) {
   unsigned long long b = (unsigned long long)__double_as_longlong(f);
   return (b & 0x8000000000000000ull) ? ~b : (b | 0x8000000000000000ull);
 }
-// atomicMax of the ordered key of f into *key; the tolerance build first takes
-// the maximum over the active lanes of the warp that update the same key (a
-// warp of the batched kernel can span several events), by hardware warp
-// reductions over the lanes __match_any_sync groups (64-bit keys as the high
-// word, then the low word among the lanes holding the largest high word), so
-// that one lane of each group issues the atomic
+// atomicMax of the ordered key of f into *key, NaN left out. The active lanes
+// of the warp that update the same key (a warp of the batched kernel can span
+// several events) first take their maximum by hardware warp reductions over
+// the lanes __match_any_sync groups (64-bit keys as the high word, then the low
+// word among the lanes holding the largest high word), so that one lane of
+// each group issues the atomic
 __device__ __forceinline__ unsigned int warp_max_key(unsigned int m, unsigned int k) { return __reduce_max_sync(m, k); }
 __device__ __forceinline__ unsigned long long warp_max_key(unsigned int m, unsigned long long k) {
   const unsigned int hi = __reduce_max_sync(m, (unsigned int)(k >> 32));
   const unsigned int lo = __reduce_max_sync(m, (unsigned int)(k >> 32) == hi ? (unsigned int)k : 0u);
   return ((unsigned long long)hi << 32) | lo;
 }
-template <class real> __device__ __forceinline__ void key_max(typename KeyT<real>::type* key, real f) {
+template <class real>
+__device__ __forceinline__ void key_commit(typename KeyT<real>::type* key, typename KeyT<real>::type k) {
   typedef typename KeyT<real>::type K;
-  const bool ok = (f == f);
-  K k = ok ? fkey(f) : (K)0;
-#if CLV_FAST
   const unsigned int m = __match_any_sync(__activemask(), (unsigned long long)key);
   k = warp_max_key(m, k);
   if ((threadIdx.x & 31) == (unsigned int)(__ffs(m) - 1) && k != (K)0) atomicMax(key, k);
-#else
-  if (ok) atomicMax(key, k);
-#endif
+}
+template <class real> __device__ __forceinline__ void key_max(typename KeyT<real>::type* key, real f) {
+  key_commit<real>(key, f == f ? fkey(f) : (typename KeyT<real>::type)0);
 }
 }  // namespace CLV_ARITH
 }  // namespace clv

@@ -23,11 +23,11 @@ constexpr int kTiledMinNz = 24;  // fewer cells along eta: per-cell kernel
 // per-device "dynamic shared memory raised" flags of each tiled instantiation
 constexpr int kMaxDev = 64;
 
-template <class real, bool CPL, int MINB, int TJ, int TK>
-int launch_tiled(const clv::Params& p, const clv::ViscBuffers<real>& v, int step, const clv::TauConst<real>& tc,
+template <class real, bool CPL, int MINB, int TJ, int TK, bool BULK, int STAGE>
+int launch_tiled_stage(const clv::Params& p, const clv::ViscBuffers<real>& v, int step, const clv::TauConst<real>& tc,
                  int chunk, cudaStream_t s) {
-  typedef clv::TileSmem<real, TJ, TK> SM;
-  auto kern = clv::visc_stage_tiled_kernel<real, true, true, CPL, TJ, TK, MINB>;
+  typedef clv::TileSmem<real, TJ, TK, BULK> SM;
+  auto kern = clv::visc_stage_tiled_kernel<real, true, true, CPL, TJ, TK, MINB, BULK, STAGE>;
   static bool configured[kMaxDev] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return clv_host::check_cuda("cudaGetDevice");
@@ -41,6 +41,18 @@ int launch_tiled(const clv::Params& p, const clv::ViscBuffers<real>& v, int step
   dim3 grid(gz, gy, (p.nx + chunk - 1) / chunk);
   kern<<<grid, TJ * TK, sizeof(SM), s>>>(p, v, step, tc, chunk);
   return clv_host::check_cuda("fast visc_stage_tiled_kernel");
+}
+
+// SPLIT: the default shapes come per stage
+template <class real, bool CPL, int MINB, int TJ, int TK, bool BULK = false, bool SPLIT = false>
+int launch_tiled(const clv::Params& p, const clv::ViscBuffers<real>& v, int step, const clv::TauConst<real>& tc,
+                 int chunk, cudaStream_t s) {
+  if constexpr (SPLIT) {
+    const int kind = clv::stage_kind(v, step);
+    if (kind == 1) return launch_tiled_stage<real, CPL, MINB, TJ, TK, BULK, 1>(p, v, step, tc, chunk, s);
+    if (kind == 2) return launch_tiled_stage<real, CPL, MINB, TJ, TK, BULK, 2>(p, v, step, tc, chunk, s);
+  }
+  return launch_tiled_stage<real, CPL, MINB, TJ, TK, BULK, 0>(p, v, step, tc, chunk, s);
 }
 
 template <class real, bool BULK, int TB>
@@ -69,7 +81,8 @@ int visc_stage(const clv::Params& p, const clv::ViscBuffers<real>& v, int step, 
   const bool bulk = p.flags & clv::FLAG_BULK;
   const bool cpl = p.flags & (clv::FLAG_GUBSER_VISC | clv::FLAG_PIMN_OMEGA | clv::FLAG_OMEGA_OMEGA);
   if (o.chunk < 0) return clv_host::set_error(CLV_ERR_INVALID, "fast visc stage: chunk must be >= 1");
-  if (!bulk && (o.stage_kernel == 2 || (o.stage_kernel != 1 && p.nz >= kTiledMinNz))) {
+  const bool idx32 = clv::fits_idx32<real>(p);
+  if (!bulk && idx32 && (o.stage_kernel == 2 || (o.stage_kernel != 1 && p.nz >= kTiledMinNz))) {
     if (cpl) return launch_tiled<real, true, 1, 8, 32>(p, v, step, tc, o.chunk, s);
     // 16 x 16 and 8 x 16 (y, eta) tiles as in the exact build (CLV_OPT_TILE 1, 2)
     if (o.tile == 1) {
@@ -80,13 +93,20 @@ int visc_stage(const clv::Params& p, const clv::ViscBuffers<real>& v, int step, 
       if (sizeof(real) == 8 || o.minb == 1) return launch_tiled<real, false, 2, 8, 16>(p, v, step, tc, o.chunk, s);
       if constexpr (sizeof(real) == 4) return launch_tiled<real, false, 4, 8, 16>(p, v, step, tc, o.chunk, s);
     }
-    if constexpr (sizeof(real) == 8) return launch_tiled<real, false, 1, 8, 32>(p, v, step, tc, o.chunk, s);
+    if constexpr (sizeof(real) == 8) return launch_tiled<real, false, 1, 8, 32, false, true>(p, v, step, tc, o.chunk, s);
     else {
       // 16 x 32 (y, eta) tiles, one 512-thread CTA an SM: less halo than two 8 x 32 CTAs
       if (o.tile == 3) return launch_tiled<real, false, 1, 16, 32>(p, v, step, tc, o.chunk, s);
       if (o.minb == 1) return launch_tiled<real, false, 1, 8, 32>(p, v, step, tc, o.chunk, s);
-      return launch_tiled<real, false, 2, 8, 32>(p, v, step, tc, o.chunk, s);
+      return launch_tiled<real, false, 2, 8, 32, false, true>(p, v, step, tc, o.chunk, s);
     }
+  }
+  // the bulk sector's larger record (24 values) takes 8 x 16 tiles, three
+  // 128-thread CTAs an SM, in FP32; in FP64 one such CTA fills the shared
+  // memory and the per-cell kernel is the better one
+  if constexpr (sizeof(real) == 4) {
+    if (bulk && idx32 && !cpl && o.stage_kernel != 1 && p.nz >= kTiledMinNz)
+      return launch_tiled<real, false, 3, 8, 16, true, true>(p, v, step, tc, o.chunk, s);
   }
   // (2+1)D grids: the tiled (2+1)D kernel (CLV_OPT_STAGE_KERNEL 3), with
   // or without the bulk sector; not the coupling terms
@@ -98,7 +118,7 @@ int visc_stage(const clv::Params& p, const clv::ViscBuffers<real>& v, int step, 
     return bulk ? launch_tiled2d<real, true, 64>(p, v, step, tc, o.chunk2d, s)
                 : launch_tiled2d<real, false, 64>(p, v, step, tc, o.chunk2d, s);
   }
-  // one thread per cell: (2+1)D grids, short eta axes, the bulk sector
+  // one thread per cell: (2+1)D grids, short eta axes, coupling terms, the FP64 bulk sector
   const int bs = 128;
   const long long n = (long long)p.nx * p.ny * p.nz;
   dim3 grid((unsigned int)((n + bs - 1) / bs));

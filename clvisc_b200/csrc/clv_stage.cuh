@@ -14,6 +14,8 @@
 // the two cells that share the face, so the value at face i+1/2 is the same
 // for cells i and i+1, as in the reference.
 #pragma once
+#include <type_traits>
+
 #include "clv_device.cuh"
 
 namespace clv {
@@ -45,6 +47,15 @@ template <class real> struct IdealBuffers {
   int write_src;
 };
 
+// Kinds of a fused stage launch, compiled apart: 1 and 2 are the step's first
+// and second stage, whose buffers are known to coincide (stage 1: the stage
+// input is the step's start, d_ev[1] and d_pi[1]) or not, so that neither
+// carries the other's loads or tests for them; 0: any buffers.
+template <class real> inline int stage_kind(const ViscBuffers<real>& b, int step) {
+  if (step == 1 && b.pi1 == b.pi_st && b.ev1 == b.ev_st && b.pin == b.pi1) return 1;
+  if (step == 2 && b.pi1 != b.pi_st && b.ev1 != b.ev_st && b.pin == b.pi1) return 2;
+  return 0;
+}
 // neighbour offsets along one axis, clamped at the edges: the reference's
 // two ghost cells repeat the edge cell (kernel_ideal.cl:166-172)
 struct Stencil {
@@ -62,6 +73,7 @@ struct GridDims {
 template <class real> struct CellIn {
   real e0[4], g0, p0;
   real e1[4], g1, p1;
+  real er, pr, cr;  // tolerance build, FP32: an energy density near the new one with its P(e) and c_s^2 (pi_update's lookup)
 };
 
 inline namespace CLV_ARITH {
@@ -75,10 +87,26 @@ __device__ __forceinline__ Stencil make_stencil(int q, int L, long long stride) 
   return s;
 }
 
+// Element I of the plane that starts `po` elements into a field. With I an
+// Idx32 (every byte offset of a plane below 2^32: the tiled kernels, whose
+// launch checks it) the plane's start is the same for the whole block and the
+// cell's part one 32-bit offset, which a load takes as a base and an offset
+// register; a 64-bit index costs an add with carry for each of the ~110
+// accesses of a cell.
+struct Idx32 {
+  unsigned int i;
+};
+template <class real> inline bool fits_idx32(const Params& p) { return p.ld < (1ll << 32) / (long long)sizeof(real); }
+template <class T> __device__ __forceinline__ T& plane_at(T* b, long long po, long long I) { return b[po + I]; }
+template <class T> __device__ __forceinline__ T& plane_at(T* b, long long po, Idx32 I) {
+  typedef typename std::conditional<std::is_const<T>::value, const char, char>::type byte;
+  return *reinterpret_cast<T*>(reinterpret_cast<byte*>(b + po) + (size_t)(I.i * (unsigned int)sizeof(T)));
+}
+
 // e0, g0 and p0 set: fills e1, g1, p1. At stage 1 the stencil input is d_ev[1]
 // itself (same buffer), so its values are e0's; otherwise they are read.
-template <class real>
-__device__ __forceinline__ void cell_in_ev1(const Params& p, const ViscBuffers<real>& b, long long I, long long ld,
+template <class real, class Idx>
+__device__ __forceinline__ void cell_in_ev1(const Params& p, const ViscBuffers<real>& b, Idx I, long long ld,
                                             CellIn<real>& c) {
   if (b.ev1 == b.ev_st) {
 #pragma unroll
@@ -87,7 +115,20 @@ __device__ __forceinline__ void cell_in_ev1(const Params& p, const ViscBuffers<r
     c.p1 = c.p0;
   } else {
 #pragma unroll
-    for (int q = 0; q < 4; q++) c.e1[q] = b.ev1[q * ld + I];
+    for (int q = 0; q < 4; q++) c.e1[q] = plane_at(b.ev1, q * ld, I);
+    c.g1 = gamma3<real>(c.e1[1], c.e1[2], c.e1[3]);
+    c.p1 = eosP<real>(p, c.e1[0]);
+  }
+}
+
+// the same with d_ev[1] at the cell already in c.e1 unless it is the stage input (same)
+template <class real> __device__ __forceinline__ void cell_in_ev1_of(const Params& p, bool same, CellIn<real>& c) {
+  if (same) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) c.e1[q] = c.e0[q];
+    c.g1 = c.g0;
+    c.p1 = c.p0;
+  } else {
     c.g1 = gamma3<real>(c.e1[1], c.e1[2], c.e1[3]);
     c.p1 = eosP<real>(p, c.e1[0]);
   }
@@ -98,10 +139,12 @@ __device__ __forceinline__ void cell_in_ev1(const Params& p, const ViscBuffers<r
 // S10 the IS sources (updated in place); writes pi_new and goodcell, returns
 // the new pi in pinew. With BULK, component 10 of pc, S10 and pinew is the
 // bulk pressure Pi.
-template <class real, bool COUPLED, bool BULK>
+// pi_old(m, u0): u0 times component m of pi at the start of the step (d_pi[1]).
+template <class real, bool COUPLED, bool BULK, class Idx, class PiOld>
 __device__ __forceinline__ void pi_update(const Params& p, const ViscBuffers<real>& b, int step,
-                                          const TauConst<real>& tc, long long I, long long ld, const CellIn<real>& cin,
-                                          const real pc[11], const real grad[3][4], real S10[11], real pinew[11]) {
+                                          const TauConst<real>& tc, Idx I, long long ld, CellIn<real>& cin,
+                                          const real pc[11], const real grad[3][4], real S10[11], real pinew[11],
+                                          PiOld&& pi_start) {
   const real acu = Acu<real>::v;
   const real tau = tc.tau;
   const Recips<real>& rc = recips<real>(p);
@@ -114,11 +157,11 @@ __device__ __forceinline__ void pi_update(const Params& p, const ViscBuffers<rea
   if (step == 1) {
 #pragma unroll
     for (int c = 0; c < 4; c++) {
-      real ud = b.udiff[c * ld + I];
+      real ud = plane_at(b.udiff, c * ld, I);
       udt[c] = div_by<real>(ud, (real)p.DT, rc.DT);
       u_new[c] = u_old[c] + ud;
     }
-    e2s0 = b.ev2e[I];
+    e2s0 = plane_at(b.ev2e, 0, I);
   } else {
     real g2 = cin.g0;
     u_new[0] = g2 * 1.0f;
@@ -146,6 +189,11 @@ __device__ __forceinline__ void pi_update(const Params& p, const ViscBuffers<rea
   real theta = udt[0] + grad[0][1] + grad[1][2] + grad[2][3];
   real tex[4];  // cs2, P, T, s at ed_step
   eos_texel4<real>(p, ed_step, tex);
+#if CLV_FAST
+  cin.er = ed_step;
+  cin.pr = tex[1];
+  cin.cr = tex[0];
+#endif
   real temperature = tex[2];
   real sdens = tex[3];
   real local_etaos = etaos<real>(p, temperature);
@@ -165,7 +213,7 @@ __device__ __forceinline__ void pi_update(const Params& p, const ViscBuffers<rea
 
   // the implicit update's denominator, shared by the ten components
   const real den = u_new[0] + p.DT * one_over_taupi;
-  const real rden = (real)1.0f / den;
+  const real rden = quot<real>((real)1.0f, den);
   real max_pimn_abs = 0.0f;
 #if CLV_FAST
   // tolerance build: the transversality terms of every component,
@@ -188,7 +236,7 @@ __device__ __forceinline__ void pi_update(const Params& p, const ViscBuffers<rea
       const int mn = pidx(mu, nu);
       if (u[0] > 10000.0f) sigma = 0.0f;
       real piNS = etav * sigma;
-      real pi_old = b.pi1[mn * ld + I] * u_old[0];
+      real pi_old = pi_start(mn, u_old[0]);
 #if CLV_FAST
       real src = -pc[mn] * (theta * r3 + u[0] * tc.rtau) - (u[mu] * Wv[nu] + u[nu] * Wv[mu]);
 #else
@@ -233,7 +281,7 @@ __device__ __forceinline__ void pi_update(const Params& p, const ViscBuffers<rea
     real bc = pc[10];
     real srcB = div_by<real>(bc * theta, (real)3.0f, rc.three) - div_by<real>(bc * u[0], tau, tc.rtau);
     S10[10] += srcB;
-    real b_old = b.pi1[10 * ld + I] * u_old[0];
+    real b_old = pi_start(10, u_old[0]);
     b_old = (b_old + div_step(S10[10] * p.DT, step) + p.DT * one_over_taubulk * bulkNS) /
             (u_new[0] + p.DT * one_over_taubulk);
     const real pb = (step == 1) ? eosP<real>(p, e2s0) : cin.p0;
@@ -252,8 +300,8 @@ __device__ __forceinline__ void pi_update(const Params& p, const ViscBuffers<rea
     good = 0;
   }
 #pragma unroll
-  for (int m = 0; m < NPI; m++) b.pinew[m * ld + I] = pinew[m];
-  b.goodcell[I] = good;
+  for (int m = 0; m < NPI; m++) plane_at(b.pinew, m * ld, I) = pinew[m];
+  plane_at(b.goodcell, 0, I) = good;
 }
 
 // update_ev (kernel_visc.cl:322-393) for cell I: cin holds d_ev[1] at the
@@ -261,9 +309,9 @@ __device__ __forceinline__ void pi_update(const Params& p, const ViscBuffers<rea
 // pi^{tau mu} comes from pinew (fused pi update) or from pi_new_in. Also
 // get_udiff and the edmax key. With BULK, pin[4] is Pi at the start of the
 // step and the pressure of the old and the new state is P(e) + Pi.
-template <class real, bool FUSED_PI, bool BULK>
+template <class real, bool FUSED_PI, bool BULK, class Idx>
 __device__ __forceinline__ void ev_update(const Params& p, const ViscBuffers<real>& b, int step,
-                                          const TauConst<real>& tc, long long I, long long ld, const CellIn<real>& cin,
+                                          const TauConst<real>& tc, Idx I, long long ld, const CellIn<real>& cin,
                                           const real pin[5], const real S4[4], const real pinew[11]) {
   const real acu = Acu<real>::v;
   const real tau = tc.tau;
@@ -281,10 +329,10 @@ __device__ __forceinline__ void ev_update(const Params& p, const ViscBuffers<rea
     T0m[c] = ((ed + pressure) * u0 * umu[c] - pressure * g0 + pin[c]) * old_time;
   }
   real bnew = 0.0f;
-  if (BULK) bnew = FUSED_PI ? pinew[10] : b.pi2in[10 * ld + I];
+  if (BULK) bnew = FUSED_PI ? pinew[10] : plane_at(b.pi2in, 10 * ld, I);
 #pragma unroll
   for (int c = 0; c < 4; c++) {
-    real pim2 = FUSED_PI ? pinew[c] : b.pi2in[c * ld + I];
+    real pim2 = FUSED_PI ? pinew[c] : plane_at(b.pi2in, c * ld, I);
     T0m[c] = T0m[c] + div_step(S4[c] * p.DT, step) - pim2 * tau;
   }
   real T00 = div_by<real>(cmax<real>(acu, T0m[0]), tau, tc.rtau);
@@ -299,36 +347,44 @@ __device__ __forceinline__ void ev_update(const Params& p, const ViscBuffers<rea
     T03 *= SCALE_COEF * T00 / M;
     M = SCALE_COEF * T00;
   }
-  // tolerance build, FP32: Newton from the cell's speed at the start of the
-  // step, which is near the root, instead of from 1/2 (fewer EOS lookups).
-  // The finder stops at a step below 1e-5, so where it ends depends on where
-  // it starts: about 1e-9 of the energy density, inside the FP32 tolerance
-  // but not the FP64 one, which keeps the reference's start.
-  real v_start = -1.0f;
+  real pr, ed_find;
 #if CLV_FAST
-  if constexpr (sizeof(real) == 4) v_start = fmin(sqrt(vx * vx + vy * vy + vz * vz), (real)0.999f);
+  if constexpr (sizeof(real) == 4 && FUSED_PI) {
+    ed_find = root_near<BULK>(p, T00, M, bnew, cin.er, cin.pr, cin.cr, pr);
+    if (ed_find < acu) {
+      T01 = 0.0f;
+      T02 = 0.0f;
+      T03 = 0.0f;
+    }
+    if (ed_find < 0.0f) {
+      ed_find = 0.0f;
+      pr = eosP<real>(p, ed_find);
+    }
+  } else
 #endif
-  real ed_find = root_newton<real, BULK>(p, T00, M, bnew, v_start);
-  if (ed_find < acu) {
-    T01 = 0.0f;
-    T02 = 0.0f;
-    T03 = 0.0f;
+  {
+    ed_find = root_newton<real, BULK>(p, T00, M, bnew);
+    if (ed_find < acu) {
+      T01 = 0.0f;
+      T02 = 0.0f;
+      T03 = 0.0f;
+    }
+    ed_find = cmax<real>(0.0f, ed_find);
+    pr = eosP<real>(p, ed_find);
   }
-  ed_find = cmax<real>(0.0f, ed_find);
-  real pr = eosP<real>(p, ed_find);
   if (BULK) pr = pr + bnew;
   real epv = cmax<real>(acu, T00 + pr);
-  const real repv = (real)1.0f / epv;
+  const real repv = quot<real>((real)1.0f, epv);
   real en[4] = {ed_find, div_by<real>(T01, epv, repv), div_by<real>(T02, epv, repv), div_by<real>(T03, epv, repv)};
 #pragma unroll
-  for (int c = 0; c < 4; c++) b.evnew[c * ld + I] = en[c];
+  for (int c = 0; c < 4; c++) plane_at(b.evnew, c * ld, I) = en[c];
   if (b.write_udiff) {  // get_udiff, kernel_IS.cl:714-724
     real gn = gamma3<real>(en[1], en[2], en[3]);
     real go = cin.g1;
-    b.udiff[0 * ld + I] = gn * 1.0f - go * 1.0f;
-    b.udiff[1 * ld + I] = gn * en[1] - go * e1[1];
-    b.udiff[2 * ld + I] = gn * en[2] - go * e1[2];
-    b.udiff[3 * ld + I] = gn * en[3] - go * e1[3];
+    plane_at(b.udiff, 0 * ld, I) = gn * 1.0f - go * 1.0f;
+    plane_at(b.udiff, 1 * ld, I) = gn * en[1] - go * e1[1];
+    plane_at(b.udiff, 2 * ld, I) = gn * en[2] - go * e1[2];
+    plane_at(b.udiff, 3 * ld, I) = gn * en[3] - go * e1[3];
   }
   if (b.edmax_key) key_max<real>(b.edmax_key, en[0]);
 }
@@ -573,7 +629,9 @@ __device__ __forceinline__ void visc_stage_cell(const Params& p, const GridDims 
 
   real pinew[11];
   cell_in_ev1<real>(p, b, I, ld, cin);
-  if (DO_IS) pi_update<real, COUPLED, BULK>(p, b, step, tc, I, ld, cin, pc, grad, S10, pinew);
+  if (DO_IS)
+    pi_update<real, COUPLED, BULK>(p, b, step, tc, I, ld, cin, pc, grad, S10, pinew,
+                                   [&](int m, real u) { return b.pi1[m * ld + I] * u; });
   if (DO_KT) ev_update<real, DO_IS, BULK>(p, b, step, tc, I, ld, cin, pin, S4, pinew);
 
   if (b.write_src) {
@@ -595,6 +653,67 @@ __global__ void __launch_bounds__(128) visc_stage_kernel(Params p, ViscBuffers<r
 }
 
 // ----------------------------------------------------------------- ideal
+// update_ev of the ideal step (kernel_ideal.cl:283-339) for cell I with the
+// sources S: writes e, v and the sources, returns e (for the edmax key). rec:
+// (e, v, P(e)) of d_ev[1] at the cell where the caller holds them, else null.
+template <class real>
+__device__ __forceinline__ real ideal_update_ev(const Params& p, const IdealBuffers<real>& b, int step,
+                                                const TauConst<real>& tc, long long I, const real S[4],
+                                                const real* rec) {
+  const real tau = tc.tau;
+  const long long ld = p.ld;
+  const real acu = Acu<real>::v;
+  const bool riemann = (p.flags & FLAG_RIEMANN) != 0;
+  real e1[4];
+#pragma unroll
+  for (int c = 0; c < 4; c++) e1[c] = rec ? rec[c] : b.ev1[c * ld + I];
+  real ed = e1[0], vx = e1[1], vy = e1[2], vz = e1[3];
+  real pressure = rec ? rec[4] : eosP<real>(p, ed);
+  real u0 = gamma3<real>(vx, vy, vz);
+  real umu[4] = {u0 * 1.0f, u0 * vx, u0 * vy, u0 * vz};
+  real old_time = tau - (step - 1) * p.DT;
+  real T0m[4];
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    real g0 = c == 0 ? (real)1.0f : (real)0.0f;
+    T0m[c] = (ed + pressure) * u0 * umu[c] - pressure * g0;
+    if (!riemann) T0m[c] = T0m[c] * old_time;
+    T0m[c] = T0m[c] + div_step(S[c] * p.DT, step);
+  }
+  real T00, T01, T02, T03;
+  if (riemann) {
+    T00 = cmax<real>(acu, T0m[0]);
+    T01 = (fabs(T0m[1]) < acu) ? (real)0.0f : T0m[1];
+    T02 = (fabs(T0m[2]) < acu) ? (real)0.0f : T0m[2];
+    T03 = (fabs(T0m[3]) < acu) ? (real)0.0f : T0m[3];
+  } else {
+    T00 = div_by<real>(cmax<real>(acu, T0m[0]), tau, tc.rtau);
+    T01 = (fabs(T0m[1]) < acu) ? (real)0.0f : div_by<real>(T0m[1], tau, tc.rtau);
+    T02 = (fabs(T0m[2]) < acu) ? (real)0.0f : div_by<real>(T0m[2], tau, tc.rtau);
+    T03 = (fabs(T0m[3]) < acu) ? (real)0.0f : div_by<real>(T0m[3], tau, tc.rtau);
+  }
+  real M = sqrt(T01 * T01 + T02 * T02 + T03 * T03);
+  real SCALE_COEF = 0.999f;
+  if (M > T00) {
+    T01 *= SCALE_COEF * T00 / M;
+    T02 *= SCALE_COEF * T00 / M;
+    T03 *= SCALE_COEF * T00 / M;
+    M = SCALE_COEF * T00;
+  }
+  real ed_find = root_newton<real>(p, T00, M);
+  ed_find = cmax<real>(0.0f, ed_find);
+  real pr = eosP<real>(p, ed_find);
+  real epv = cmax<real>(acu, T00 + pr);
+  const real repv = (real)1.0f / epv;
+  real en[4] = {ed_find, div_by<real>(T01, epv, repv), div_by<real>(T02, epv, repv), div_by<real>(T03, epv, repv)};
+#pragma unroll
+  for (int c = 0; c < 4; c++) b.evnew[c * ld + I] = en[c];
+  if (b.write_src)
+#pragma unroll
+    for (int c = 0; c < 4; c++) b.src[c * ld + I] = S[c];
+  return en[0];
+}
+
 template <class real>
 __global__ void __launch_bounds__(128) ideal_stage_kernel(Params p, IdealBuffers<real> b, int step, TauConst<real> tc) {
   const real tau = tc.tau;
@@ -607,7 +726,6 @@ __global__ void __launch_bounds__(128) ideal_stage_kernel(Params p, IdealBuffers
   const long long t = I / p.nz;
   const int j = (int)(t % p.ny);
   const int i = (int)(t / p.ny);
-  const real acu = Acu<real>::v;
   const bool riemann = (p.flags & FLAG_RIEMANN) != 0;
 
   real e0[4];
@@ -690,55 +808,8 @@ __global__ void __launch_bounds__(128) ideal_stage_kernel(Params p, IdealBuffers
     }
   }
 
-  // update_ev, kernel_ideal.cl:283-339
-  real e1[4];
-#pragma unroll
-  for (int c = 0; c < 4; c++) e1[c] = b.ev1[c * ld + I];
-  real ed = e1[0], vx = e1[1], vy = e1[2], vz = e1[3];
-  real pressure = eosP<real>(p, ed);
-  real u0 = gamma3<real>(vx, vy, vz);
-  real umu[4] = {u0 * 1.0f, u0 * vx, u0 * vy, u0 * vz};
-  real old_time = tau - (step - 1) * p.DT;
-  real T0m[4];
-#pragma unroll
-  for (int c = 0; c < 4; c++) {
-    real g0 = c == 0 ? (real)1.0f : (real)0.0f;
-    T0m[c] = (ed + pressure) * u0 * umu[c] - pressure * g0;
-    if (!riemann) T0m[c] = T0m[c] * old_time;
-    T0m[c] = T0m[c] + div_step(S[c] * p.DT, step);
-  }
-  real T00, T01, T02, T03;
-  if (riemann) {
-    T00 = cmax<real>(acu, T0m[0]);
-    T01 = (fabs(T0m[1]) < acu) ? (real)0.0f : T0m[1];
-    T02 = (fabs(T0m[2]) < acu) ? (real)0.0f : T0m[2];
-    T03 = (fabs(T0m[3]) < acu) ? (real)0.0f : T0m[3];
-  } else {
-    T00 = div_by<real>(cmax<real>(acu, T0m[0]), tau, tc.rtau);
-    T01 = (fabs(T0m[1]) < acu) ? (real)0.0f : div_by<real>(T0m[1], tau, tc.rtau);
-    T02 = (fabs(T0m[2]) < acu) ? (real)0.0f : div_by<real>(T0m[2], tau, tc.rtau);
-    T03 = (fabs(T0m[3]) < acu) ? (real)0.0f : div_by<real>(T0m[3], tau, tc.rtau);
-  }
-  real M = sqrt(T01 * T01 + T02 * T02 + T03 * T03);
-  real SCALE_COEF = 0.999f;
-  if (M > T00) {
-    T01 *= SCALE_COEF * T00 / M;
-    T02 *= SCALE_COEF * T00 / M;
-    T03 *= SCALE_COEF * T00 / M;
-    M = SCALE_COEF * T00;
-  }
-  real ed_find = root_newton<real>(p, T00, M);
-  ed_find = cmax<real>(0.0f, ed_find);
-  real pr = eosP<real>(p, ed_find);
-  real epv = cmax<real>(acu, T00 + pr);
-  const real repv = (real)1.0f / epv;
-  real en[4] = {ed_find, div_by<real>(T01, epv, repv), div_by<real>(T02, epv, repv), div_by<real>(T03, epv, repv)};
-#pragma unroll
-  for (int c = 0; c < 4; c++) b.evnew[c * ld + I] = en[c];
-  if (b.write_src)
-#pragma unroll
-    for (int c = 0; c < 4; c++) b.src[c * ld + I] = S[c];
-  if (b.edmax_key) key_max<real>(b.edmax_key, en[0]);
+  const real e = ideal_update_ev<real>(p, b, step, tc, I, S, nullptr);
+  if (b.edmax_key) key_max<real>(b.edmax_key, e);
 }
 
 }  // namespace CLV_ARITH

@@ -23,6 +23,7 @@
 // Each record, slope and face flux is the per-cell kernel's expression, so the
 // results are identical bit for bit.
 #pragma once
+#include "clv_pairs.cuh"
 #include "clv_smem16.cuh"
 #include "clv_stage.cuh"
 
@@ -83,6 +84,13 @@ __device__ __forceinline__ void rec2_make(const Params& p, const GridDims& gd, c
   real p0 = eosP<real>(p, e);
   real pr = p0;
   if (BULK) pr = pr + pv[R::NPI - 1];
+#if CLV_FAST
+  if constexpr (Pairs<real>::on) {
+    pair_record<R::NPI>(tau, e, vx, vy, vz, pr, pv, dst);
+    if (BULK) dst[R::P0] = p0;
+    return;
+  }
+#endif
   real u0 = gamma3<real>(vx, vy, vz);
   real A = (e + pr) * u0;
   real u4[4] = {(real)1.0f * u0, vx * u0, vy * u0, vz * u0};
@@ -108,6 +116,19 @@ template <class real, bool BULK>
 __device__ __forceinline__ void rec2_slopes(const real* L, const real* M, const real* R_, real* out) {
   typedef Rec2<BULK> R;
   constexpr int sl = 1, sm = 1, sr = 1, so = 1;
+#if CLV_FAST
+  if constexpr (Pairs<real>::on) {
+    // with the bulk sector the last pair is (u0 Pi, P(e)); its second slope is
+    // never used
+    constexpr int NC = (R::NCOMP + 1) / 2 * 2;
+#pragma unroll
+    for (int q = 0; q < NC; q += 2)
+      pair_limit(pair_at(L + PK_Q + q), pair_at(M + PK_Q + q), pair_at(R_ + PK_Q + q), out + q);
+#pragma unroll
+    for (int c = NC; c < Rec2L<real, BULK>::CP; c++) out[c] = 0.0f;  // padding
+    return;
+  }
+#endif
 #pragma unroll
   for (int c = R::NCOMP; c < Rec2L<real, BULK>::CP; c++) out[c] = 0.0f;  // padding
 #pragma unroll
@@ -125,23 +146,32 @@ __device__ __forceinline__ void rec2_face(const Params& p, real tau, int a, cons
                                           const real* R_, const real* sR, real F[Rec2L<real, BULK>::CP]) {
   typedef Rec2<BULK> R;
   constexpr int sl = 1, ssl = 1, sr = 1, ssr = 1;
+#if CLV_FAST
+  if constexpr (Pairs<real>::on) {
+    constexpr int NC = (R::NCOMP + 1) / 2 * 2;
+    pair_face<NC>(tau, a, L, sL, R_, sR, F);
+#pragma unroll
+    for (int c = NC; c < Rec2L<real, BULK>::CP; c++) F[c] = 0.0f;  // padding
+    return;
+  }
+#endif
 #pragma unroll
   for (int c = R::NCOMP; c < Rec2L<real, BULK>::CP; c++) F[c] = 0.0f;  // padding
 #if CLV_FAST
   // tolerance build, KT speed 1: the weighted form of the (3+1)D kernel's
   // face_flux (cp = (v+1)/2 on the left state, cm = (v-1)/2 on the right)
   {
-    const int va = R::VX + a;
-    const real vh = 0.5f * (L[va * sl] + R_[va * sr]);
+    const real vh = 0.5f * ((a == 0 ? L[R::VX * sl] : L[R::VY * sl]) + (a == 0 ? R_[R::VX * sr] : R_[R::VY * sr]));
     const real cp = 0.5f * (vh + (real)1.0f), cm = 0.5f * (vh - (real)1.0f);
     const real hp = 0.5f * cp, hm = 0.5f * cm;
     const real pt = 0.5f * (L[R::PR * sl] + R_[R::PR * sr]) * tau;
     const real th = 0.5f * tau;
 #pragma unroll
     for (int c = 0; c < 4; c++) {
-      const int mi = a == 0 ? pidx(1, c) : pidx(2, c);
+      const int m1 = pidx(1, c), m2 = pidx(2, c);
       const real p0s = L[(R::PI + c) * sl] + R_[(R::PI + c) * sr];
-      const real pis = L[(R::PI + mi) * sl] + R_[(R::PI + mi) * sr];
+      const real pis = (a == 0 ? L[(R::PI + m1) * sl] : L[(R::PI + m2) * sl]) +
+                       (a == 0 ? R_[(R::PI + m1) * sr] : R_[(R::PI + m2) * sr]);
       real k = (c == 0 ? pt - th * p0s : -th * p0s) * vh + th * pis;
       if (c == a + 1) k += pt;
       real f = cm * R_[(R::Q0 + c) * sr] + k;
@@ -170,9 +200,10 @@ __device__ __forceinline__ void rec2_face(const Params& p, real tau, int a, cons
   for (int c = 0; c < 4; c++) {
     real AL = L[(R::Q0 + c) * sl] + 0.5f * sL[c * ssl];
     real AR = R_[(R::Q0 + c) * sr] - 0.5f * sR[c * ssr];
-    const int mi = a == 0 ? pidx(1, c) : pidx(2, c);
+    const int m1 = pidx(1, c), m2 = pidx(2, c);
     real pim0_half = 0.5f * (L[(R::PI + c) * sl] + R_[(R::PI + c) * sr]);
-    real pimi_half = 0.5f * (L[(R::PI + mi) * sl] + R_[(R::PI + mi) * sr]);
+    real pimi_half = 0.5f * ((a == 0 ? L[(R::PI + m1) * sl] : L[(R::PI + m2) * sl]) +
+                             (a == 0 ? R_[(R::PI + m1) * sr] : R_[(R::PI + m2) * sr]));
     real g0 = c == 0 ? (real)1.0f : (real)0.0f;
     real ga = c == a + 1 ? (real)-1.0f : (real)0.0f;
     real Jp = (AR + pt * g0 - tau * pim0_half) * vh - pt * ga + tau * pimi_half;
@@ -191,14 +222,196 @@ __device__ __forceinline__ void rec2_face(const Params& p, real tau, int a, cons
 #endif
 }
 
+// u^mu of a record: u^0..u^3 (in pairs: u^1, u^2, u^3, u^0, the record's order)
+template <class real, bool BULK> __device__ __forceinline__ void rec2_umu(const real* r, real u[4]) {
+  typedef Rec2<BULK> R;
+  if constexpr (Pairs<real>::on) {
+#pragma unroll
+    for (int c = 0; c < 4; c++) u[c] = r[PK_UX + c];
+  } else {
+    const real u0 = r[R::U0];
+    u[0] = u0 * 1.0f;
+    u[1] = u0 * r[R::VX];
+    u[2] = u0 * r[R::VY];
+    u[3] = u0 * r[R::VZ];
+  }
+}
+
+// The update's inputs at cell I, whose record is slot c of the region C of n
+// slots: the stage input (cin), its pi and Pi (pc), pi^{tau mu} and Pi at the
+// start of the step (pin), and the sources with the Christoffel terms added
+template <class real, bool BULK>
+__device__ __forceinline__ void rec2_cell(const Params& p, const GridDims& gd, const ViscBuffers<real>& b, int step,
+                                          const TauConst<real>& tc, long long I, const real* C, int n, int c0,
+                                          CellIn<real>& cin, real pc[11], real pin[5], real S4[4], real S10[11]) {
+  typedef Rec2<BULK> R;
+  const real tau = tc.tau;
+  const long long ld = gd.ld;
+  real Cs[Rec2L<real, BULK>::NP];
+  grp_load<real, Rec2L<real, BULK>::RG>(C, n, c0, Cs);
+  real* e0 = cin.e0;
+  if constexpr (Pairs<real>::on) {
+    const real ru = Cs[PK_RU];
+    e0[0] = b.ev_st[I];
+    e0[1] = Cs[PK_UX] * ru;
+    e0[2] = Cs[PK_UY] * ru;
+    e0[3] = Cs[PK_UZ] * ru;
+    cin.g0 = Cs[PK_U0];
+    cin.p0 = BULK ? Cs[R::P0] : Cs[PK_PR];
+#pragma unroll
+    for (int m = 0; m < R::NPI; m++) pc[m] = Cs[PK_U + m] * ru;
+  } else {
+    e0[0] = Cs[R::E];
+    e0[1] = Cs[R::VX];
+    e0[2] = Cs[R::VY];
+    e0[3] = Cs[R::VZ];
+    cin.g0 = Cs[R::U0];
+    cin.p0 = Cs[R::P0];
+#pragma unroll
+    for (int m = 0; m < R::NPI; m++) pc[m] = Cs[R::PI + m];
+  }
+  if (!BULK) pc[10] = 0.0f;
+#pragma unroll
+  for (int c = 0; c < 4; c++) pin[c] = b.pin[c * ld + I];
+  pin[4] = BULK ? b.pin[10 * ld + I] : (real)0.0f;
+  if (step == 1) {
+#pragma unroll
+    for (int c = 0; c < 4; c++) S4[c] = 0.0f;
+#pragma unroll
+    for (int m = 0; m < 11; m++) S10[m] = 0.0f;
+  } else {
+#pragma unroll
+    for (int c = 0; c < 4; c++) S4[c] = b.src[c * ld + I];
+#pragma unroll
+    for (int m = 0; m < R::NPI; m++) S10[m] = b.src[(4 + m) * ld + I];
+    if (!BULK) S10[10] = 0.0f;
+  }
+  {  // Christoffel terms, kernel_IS.cl:56-65
+    real uz = e0[3] * cin.g0;
+    S10[0] -= div_by<real>(2.0f * uz * pc[pidx(0, 3)], tau, tc.rtau);
+    S10[1] -= div_by<real>(uz * pc[pidx(1, 3)], tau, tc.rtau);
+    S10[2] -= div_by<real>(uz * pc[pidx(2, 3)], tau, tc.rtau);
+    S10[3] -= div_by<real>(uz * (pc[pidx(0, 0)] + pc[pidx(3, 3)]), tau, tc.rtau);
+    S10[6] -= div_by<real>(uz * pc[pidx(0, 1)], tau, tc.rtau);
+    S10[8] -= div_by<real>(uz * pc[pidx(0, 2)], tau, tc.rtau);
+    S10[9] -= div_by<real>(2.0f * uz * pc[pidx(0, 3)], tau, tc.rtau);
+  }
+  {  // kernel_visc.cl:24-50
+    real ed = e0[0], vx = e0[1], vy = e0[2], vz = e0[3];
+    real u0 = cin.g0;
+    real bulkpi = BULK ? pc[10] : (real)0.0f;
+    real pressure = cin.p0 + bulkpi;
+    real Tzz_tilde = (ed + pressure) * u0 * u0 * vz * vz + pressure + pc[pidx(3, 3)];
+    real Ttz_tilde = (ed + pressure) * u0 * u0 * vz + pc[pidx(0, 3)];
+    S4[0] = S4[0] - Tzz_tilde;
+    S4[1] = S4[1] - (real)0.0f;
+    S4[2] = S4[2] - (real)0.0f;
+    S4[3] = S4[3] - Ttz_tilde;
+    if (p.flags & FLAG_RIEMANN) {
+      real Ttt_tilde = (ed + pressure) * u0 * u0 - pressure;
+      real Ttx_tilde = (ed + pressure) * u0 * u0 * vx;
+      real Tty_tilde = (ed + pressure) * u0 * u0 * vy;
+      S4[0] = S4[0] + (Tzz_tilde + Ttt_tilde);
+      S4[1] = S4[1] + Ttx_tilde;
+      S4[2] = S4[2] + Tty_tilde;
+      S4[3] = S4[3] + 3.0f * Ttz_tilde;
+    }
+  }
+}
+// flux difference of one direction into the sources
+template <class real, bool BULK>
+__device__ __forceinline__ void rec2_flux(const real* Fp, const real* Fm, real D, real rD, real S4[4], real S10[11]) {
+  constexpr int NC = Rec2<BULK>::NCOMP;
+#if CLV_FAST
+  if constexpr (Pairs<real>::on) {
+    const float2 rd2 = make_float2(-rD, -rD);
+#pragma unroll
+    for (int c = 0; c < NC; c += 2) {
+      const float2 d = pair_sub(pair_at(Fp + c), pair_at(Fm + c));
+      real* const s2 = c < 4 ? S4 + c : S10 + (c - 4);
+      if (c + 1 < NC) {
+        const float2 t = __ffma2_rn(d, rd2, pair_at(s2));
+        s2[0] = t.x;
+        s2[1] = t.y;
+      } else {
+        s2[0] = s2[0] - d.x * rD;
+      }
+    }
+    return;
+  }
+#endif
+#pragma unroll
+  for (int c = 0; c < NC; c++) {
+    real src = Fp[c];
+    src -= Fm[c];
+    if (c < 4) S4[c] = S4[c] - div_by<real>(src, D, rD);
+    else S10[c - 4] = S10[c - 4] - div_by<real>(src, D, rD);
+  }
+}
+// velocity gradients, kernel_IS.cl:134-137 / 217-220 / 299-304, from u of the
+// cell and its neighbours in x and y (rec2_umu's order)
+template <class real, bool BULK>
+__device__ __forceinline__ void rec2_grad(const Params& p, const TauConst<real>& tc, const CellIn<real>& cin,
+                                          const real um[4], const real ux0[4], const real ux1[4], const real uy0[4],
+                                          const real uy1[4], real grad[3][4]) {
+  const Recips<real>& rc = recips<real>(p);
+  const real tau = tc.tau;
+  const real* e0 = cin.e0;
+  const real u0c = cin.g0;
+#if CLV_FAST
+  if constexpr (Pairs<real>::on) {
+#pragma unroll
+    for (int a = 0; a < 2; a++) {
+      const real sc = CLV_THETA * (a == 0 ? rc.DX : rc.DY);
+      const real* lo = a == 0 ? ux0 : uy0;
+      const real* hi = a == 0 ? ux1 : uy1;
+      real o[4];
+      pair_limit(pair_at(lo), pair_at(um), pair_at(hi), o);
+      pair_limit(pair_at(lo + 2), pair_at(um + 2), pair_at(hi + 2), o + 2);
+#pragma unroll
+      for (int c = 0; c < 4; c++) grad[a][c] = sc * o[(c + 3) & 3];
+    }
+  }
+#endif
+  if constexpr (!Pairs<real>::on) {
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      grad[0][c] = div_by<real>(grad_limit<real>(ux0[c], um[c], ux1[c]), (real)p.DX, rc.DX);
+      grad[1][c] = div_by<real>(grad_limit<real>(uy0[c], um[c], uy1[c]), (real)p.DY, rc.DY);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 4; c++) grad[2][c] = 0.0f;
+  grad[2][0] = grad[2][0] + div_by<real>(e0[3] * u0c, tau, tc.rtau);
+  grad[2][1] = grad[2][1] + div_by<real>((real)0.0f * u0c, tau, tc.rtau);
+  grad[2][2] = grad[2][2] + div_by<real>((real)0.0f * u0c, tau, tc.rtau);
+  grad[2][3] = grad[2][3] + div_by<real>((real)1.0f * u0c, tau, tc.rtau);
+}
+
+// pi (and Pi) at the start of the step, d_pi[1]. STAGE 1: it is the stage
+// input (the same buffer), whose values pc holds; 2: another buffer; 0: unknown.
+template <class real, bool BULK, int STAGE>
+__device__ __forceinline__ void rec2_start(const ViscBuffers<real>& b, long long I, long long ld, const real pc[11],
+                                           real* out) {
+  constexpr int NPI = Rec2<BULK>::NPI;
+  if (STAGE == 1 || (STAGE == 0 && b.pi1 == b.pi_st)) {
+#pragma unroll
+    for (int m = 0; m < NPI; m++) out[m] = pc[m];
+  } else {
+#pragma unroll
+    for (int m = 0; m < NPI; m++) out[m] = b.pi1[m * ld + I];
+  }
+}
+
 // One tile: rows j0 .. j0+TB-5 of planes i0 .. i1-1 of the event (gd, b).
 // Every thread of the block calls it (it holds barriers).
-template <class real, bool BULK, int TB>
-__device__ __forceinline__ void tile2d(const Params& p, const GridDims& gd, const ViscBuffers<real>& b, int step,
+template <class real, bool BULK, int TB, int STAGE = 0>
+__device__ __forceinline__ void tile2d(const Params& p, const GridDims& gd, const ViscBuffers<real>& b, int step_,
                                        const TauConst<real>& tc, int j0, int i0, int i1, Tile2Smem<real, BULK, TB>& s) {
   typedef Rec2<BULK> R;
   typedef Rec2L<real, BULK> L;
   constexpr int NC = R::NCOMP, NP = L::NP, CP = L::CP, RG = L::RG, CG = L::CG;
+  const int step = STAGE ? STAGE : step_;
   const real tau = tc.tau;
   const Recips<real>& rc = recips<real>(p);
   const long long ld = gd.ld;
@@ -225,11 +438,7 @@ __device__ __forceinline__ void tile2d(const Params& p, const GridDims& gd, cons
     grp_store<real, RG>(A, TB, t, r0);
     rec2_slopes<real, BULK>(r1, r2, r0, s_cur);  // x slope at i0
     rec2_face<real, BULK>(p, tau, 0, r1, s_prev, r2, s_cur, F_prev);
-    real u0 = r1[R::U0];
-    umu_prev[0] = u0 * 1.0f;
-    umu_prev[1] = u0 * r1[R::VX];
-    umu_prev[2] = u0 * r1[R::VY];
-    umu_prev[3] = u0 * r1[R::VZ];
+    rec2_umu<real, BULK>(r1, umu_prev);
     rec2_make<real, BULK>(p, gd, b, tau, i0 + 2, jj, r0);
     grp_store<real, RG>(B, TB, t, r0);
   } else {
@@ -280,116 +489,35 @@ __device__ __forceinline__ void tile2d(const Params& p, const GridDims& gd, cons
     // ------------------------------------------------------ cell update
     if (inside && i < gd.nx) {
       const long long I = (long long)i * gd.ny + jj;
-      real Cs[NP];
-      grp_load<real, RG>(Cp, TB, t, Cs);
       CellIn<real> cin;
-      real* e0 = cin.e0;
-      e0[0] = Cs[R::E];
-      e0[1] = Cs[R::VX];
-      e0[2] = Cs[R::VY];
-      e0[3] = Cs[R::VZ];
-      cin.g0 = Cs[R::U0];
-      cin.p0 = Cs[R::P0];
-      real pc[11];
-#pragma unroll
-      for (int m = 0; m < R::NPI; m++) pc[m] = Cs[R::PI + m];
-      if (!BULK) pc[10] = 0.0f;
-      real pin[5];
-#pragma unroll
-      for (int c = 0; c < 4; c++) pin[c] = b.pin[c * ld + I];
-      pin[4] = BULK ? b.pin[10 * ld + I] : (real)0.0f;
-      real S4[4], S10[11];
-      if (step == 1) {
-#pragma unroll
-        for (int c = 0; c < 4; c++) S4[c] = 0.0f;
-#pragma unroll
-        for (int m = 0; m < 11; m++) S10[m] = 0.0f;
-      } else {
-#pragma unroll
-        for (int c = 0; c < 4; c++) S4[c] = b.src[c * ld + I];
-#pragma unroll
-        for (int m = 0; m < R::NPI; m++) S10[m] = b.src[(4 + m) * ld + I];
-        if (!BULK) S10[10] = 0.0f;
-      }
-      {  // Christoffel terms, kernel_IS.cl:56-65
-        real uz = e0[3] * cin.g0;
-        S10[0] -= div_by<real>(2.0f * uz * pc[pidx(0, 3)], tau, tc.rtau);
-        S10[1] -= div_by<real>(uz * pc[pidx(1, 3)], tau, tc.rtau);
-        S10[2] -= div_by<real>(uz * pc[pidx(2, 3)], tau, tc.rtau);
-        S10[3] -= div_by<real>(uz * (pc[pidx(0, 0)] + pc[pidx(3, 3)]), tau, tc.rtau);
-        S10[6] -= div_by<real>(uz * pc[pidx(0, 1)], tau, tc.rtau);
-        S10[8] -= div_by<real>(uz * pc[pidx(0, 2)], tau, tc.rtau);
-        S10[9] -= div_by<real>(2.0f * uz * pc[pidx(0, 3)], tau, tc.rtau);
-      }
-      {  // kernel_visc.cl:24-50
-        real ed = e0[0], vx = e0[1], vy = e0[2], vz = e0[3];
-        real u0 = cin.g0;
-        real bulkpi = BULK ? pc[10] : (real)0.0f;
-        real pressure = cin.p0 + bulkpi;
-        real Tzz_tilde = (ed + pressure) * u0 * u0 * vz * vz + pressure + pc[pidx(3, 3)];
-        real Ttz_tilde = (ed + pressure) * u0 * u0 * vz + pc[pidx(0, 3)];
-        S4[0] = S4[0] - Tzz_tilde;
-        S4[1] = S4[1] - (real)0.0f;
-        S4[2] = S4[2] - (real)0.0f;
-        S4[3] = S4[3] - Ttz_tilde;
-        if (p.flags & FLAG_RIEMANN) {
-          real Ttt_tilde = (ed + pressure) * u0 * u0 - pressure;
-          real Ttx_tilde = (ed + pressure) * u0 * u0 * vx;
-          real Tty_tilde = (ed + pressure) * u0 * u0 * vy;
-          S4[0] = S4[0] + (Tzz_tilde + Ttt_tilde);
-          S4[1] = S4[1] + Ttx_tilde;
-          S4[2] = S4[2] + Tty_tilde;
-          S4[3] = S4[3] + 3.0f * Ttz_tilde;
-        }
-      }
+      real pc[11], pin[5], S4[4], S10[11], grad[3][4];
+      rec2_cell<real, BULK>(p, gd, b, step, tc, I, Cp, TB, t, cin, pc, pin, S4, S10);
       // flux differences in the reference's order x, y (eta: one cell, none)
       real Fyp[CP], Fym[CP];
       grp_load<real, CG>(FYp, TB, t, Fyp);
       grp_load<real, CG>(FYp, TB, t - 1, Fym);
-#pragma unroll
-      for (int a = 0; a < 2; a++) {
-        const real D = a == 0 ? (real)p.DX : (real)p.DY;
-        const real rD = a == 0 ? rc.DX : rc.DY;
-#pragma unroll
-        for (int c = 0; c < NC; c++) {
-          real fp = a == 0 ? Fx[c] : Fyp[c];
-          real fm = a == 0 ? F_prev[c] : Fym[c];
-          real src = fp;
-          src -= fm;
-          if (c < 4) S4[c] = S4[c] - div_by<real>(src, D, rD);
-          else S10[c - 4] = S10[c - 4] - div_by<real>(src, D, rD);
-        }
-      }
-      // velocity gradients, kernel_IS.cl:134-137 / 217-220 / 299-304
-      real grad[3][4];
+      rec2_flux<real, BULK>(Fx, F_prev, (real)p.DX, rc.DX, S4, S10);
+      rec2_flux<real, BULK>(Fyp, Fym, (real)p.DY, rc.DY, S4, S10);
       {
-        real Ax[NP], Cy0[NP], Cy1[NP];
-        grp_load<real, RG>(A, TB, t, Ax);
-        grp_load<real, RG>(Cp, TB, t - 1, Cy0);
-        grp_load<real, RG>(Cp, TB, t + 1, Cy1);
-        real u0c = cin.g0;
-        real umc[4] = {u0c * 1.0f, u0c * e0[1], u0c * e0[2], u0c * e0[3]};
-        real ua = Ax[R::U0];
-        real umx1[4] = {ua * 1.0f, ua * Ax[R::VX], ua * Ax[R::VY], ua * Ax[R::VZ]};
-        real uy0 = Cy0[R::U0], uy1 = Cy1[R::U0];
-        real umy0[4] = {uy0 * 1.0f, uy0 * Cy0[R::VX], uy0 * Cy0[R::VY], uy0 * Cy0[R::VZ]};
-        real umy1[4] = {uy1 * 1.0f, uy1 * Cy1[R::VX], uy1 * Cy1[R::VY], uy1 * Cy1[R::VZ]};
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-          grad[0][c] = div_by<real>(grad_limit<real>(umu_prev[c], umc[c], umx1[c]), (real)p.DX, rc.DX);
-          grad[1][c] = div_by<real>(grad_limit<real>(umy0[c], umc[c], umy1[c]), (real)p.DY, rc.DY);
-          grad[2][c] = 0.0f;
-        }
-        grad[2][0] = grad[2][0] + div_by<real>(e0[3] * u0c, tau, tc.rtau);
-        grad[2][1] = grad[2][1] + div_by<real>((real)0.0f * u0c, tau, tc.rtau);
-        grad[2][2] = grad[2][2] + div_by<real>((real)0.0f * u0c, tau, tc.rtau);
-        grad[2][3] = grad[2][3] + div_by<real>((real)1.0f * u0c, tau, tc.rtau);
+        real n[NP], umc[4], umx1[4], umy0[4], umy1[4];
+        grp_load<real, RG>(Cp, TB, t, n);
+        rec2_umu<real, BULK>(n, umc);
+        grp_load<real, RG>(A, TB, t, n);
+        rec2_umu<real, BULK>(n, umx1);
+        grp_load<real, RG>(Cp, TB, t - 1, n);
+        rec2_umu<real, BULK>(n, umy0);
+        grp_load<real, RG>(Cp, TB, t + 1, n);
+        rec2_umu<real, BULK>(n, umy1);
+        rec2_grad<real, BULK>(p, tc, cin, umc, umu_prev, umx1, umy0, umy1, grad);
 #pragma unroll
         for (int c = 0; c < 4; c++) umu_prev[c] = umc[c];
       }
       real pinew[11];
       cell_in_ev1<real>(p, b, I, ld, cin);
-      pi_update<real, false, BULK>(p, b, step, tc, I, ld, cin, pc, grad, S10, pinew);
+      real pstart[R::NPI];  // pi at the start of the step: at stage 1 the stage input's
+      rec2_start<real, BULK, STAGE>(b, I, ld, pc, pstart);
+      pi_update<real, false, BULK>(p, b, step, tc, I, ld, cin, pc, grad, S10, pinew,
+                                   [&](int m, real u) { return pstart[m] * u; });
       ev_update<real, true, BULK>(p, b, step, tc, I, ld, cin, pin, S4, pinew);
       if (b.write_src) {
 #pragma unroll
@@ -400,11 +528,7 @@ __device__ __forceinline__ void tile2d(const Params& p, const GridDims& gd, cons
     } else if (mid) {
       real Cs[NP];
       grp_load<real, RG>(Cp, TB, t, Cs);
-      real u0c = Cs[R::U0];
-      umu_prev[0] = u0c * 1.0f;
-      umu_prev[1] = u0c * Cs[R::VX];
-      umu_prev[2] = u0c * Cs[R::VY];
-      umu_prev[3] = u0c * Cs[R::VZ];
+      rec2_umu<real, BULK>(Cs, umu_prev);
     }
     if (mid) {
 #pragma unroll

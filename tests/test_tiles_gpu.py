@@ -15,6 +15,56 @@ BULK = dict(ZETAOS_MAX=0.12, ZETAOS_T0=0.2, ZETAOS_WIDTH=0.05, ZETAOS_SKEW=0.3)
 
 
 @pytest.mark.parametrize('use_float32', [True, False])
+@pytest.mark.parametrize('arithmetic', ['exact', 'fast'])
+@pytest.mark.parametrize('extra', [{}, BULK], ids=['shear', 'bulk'])
+@pytest.mark.parametrize('grid', [(1, 9, 1), (7, 1, 1), (8, 8, 1), (9, 17, 1), (41, 33, 1), (3, 8, 24), (9, 17, 33),
+                                  (37, 7, 25)])
+def test_viscous_edges(cuda_lib, oracle_mod, use_float32, arithmetic, extra, grid):
+    """(2+1)D patches and (3+1)D tiles with and without the bulk sector."""
+    from clvisc_b200.visc import CLVisc
+    cfg = make_cfg(*grid, use_float32=use_float32, arithmetic=arithmetic, **extra)
+    v, o = CLVisc(cfg), oracle_mod.OracleVisc(cfg)
+    ic = seeded_ic(cfg, seed=17, flow=0.2)
+    for h in (v, o):
+        h.load_ini(ic)
+        h.IS_initialize()
+    for n in range(6):
+        v.step(n, edmax=(n == 5))
+        o.step(n)
+    if arithmetic == 'fast':
+        compare_fields(v, o, use_float32, 'edges %s' % (grid,))
+    else:
+        assert_same('ev', v.ideal.field_to_host(v.ideal.d_ev[1]), o.ideal.d_ev[1])
+        assert_same('pi', v.pi_to_host(1), o.d_pi[1])
+        if v.bulk:
+            assert_same('Pi', v.bulk_to_host(1), o.d_bulk[1])
+    want = o.ideal.max_energy_density()
+    assert abs(v.read_edmax_key() - want) <= (TOL[use_float32] if arithmetic == 'fast' else 0.0) * abs(want)
+
+
+@pytest.mark.parametrize('use_float32', [True, False])
+def test_fast_stage_beyond_the_eos_table(cuda_lib, oracle_mod, use_float32):
+    """Energy densities from the table's first texel over its last
+    (310.998 GeV/fm^3) into the formula beyond it, no flow: the tolerance
+    build's lookup takes the reference's way from the last texel on. The
+    formula's power and exponential differ between CUDA and the host library
+    by 2 ulp, far inside the tolerance."""
+    from clvisc_b200.visc import CLVisc
+    cfg = make_cfg(9, 8, 40, use_float32=use_float32, arithmetic='fast')
+    v, o = CLVisc(cfg), oracle_mod.OracleVisc(cfg)
+    n = 9 * 8 * 40
+    ic = np.zeros((n, 4), cfg.real)
+    ic[:, 0] = np.linspace(0.0, 400.0, n)
+    for h in (v, o):
+        h.load_ini(ic)
+        h.IS_initialize()
+        h.step(0)
+    errs = field_errors(v.ideal.field_to_host(v.ideal.d_ev[1]), o.ideal.d_ev[1], v.pi_to_host(1), o.d_pi[1],
+                        Eos(cfg.eos_type), float(v.ideal.tau))
+    assert max(e for k, e in errs.items() if k != 'components') <= TOL[use_float32], errs
+
+
+@pytest.mark.parametrize('use_float32', [True, False])
 @pytest.mark.parametrize('viscous', [False, True])
 @pytest.mark.parametrize('n', [1, 127, 128, 129, 1800])
 def test_spectra_element_counts(cuda_lib, oracle_mod, use_float32, viscous, n):
