@@ -21,7 +21,7 @@ replays it until every event has stopped.
 
 The stage kernel is either one thread per cell for any grids
 (clv_batch_stage) or, for batches of (2+1)D events, the tiled kernel
-(clv_batch_stage_tiled: y strips of rows-4 cells marching along x); both give
+(clv_batch_stage_tiled: patches of cells, of the kernel's own size); both give
 the same bits. autotune() times both families over their launch shapes.
 
 Only the viscous path is batched (no Gubser, coupling or Riemann test flags);
@@ -409,7 +409,8 @@ class CLViscBatch(object):
         size with persistent grids of 1..occupancy blocks per SM and the
         one-cell-per-thread grid, without and (FP32) with a 128-register cap
         (and a 168-register cap below 256 threads). Tiled ((2+1)D batches only): rows x chunks, each with the grid
-        that fills the GPU once and the one-tile-per-block grid."""
+        that fills the GPU once and the one-tile-per-block grid (the kernel chooses its patch itself, and a grid
+        above one resident wave counts as one)."""
         sms = torch.cuda.get_device_properties(self.device).multi_processor_count
         out = []
         total = sum(self.sizes)

@@ -90,8 +90,8 @@ int batch_stage_tiled_t(const clv_params* pp, int step, const clv_batch* b, int 
     return clv_host::set_error(CLV_ERR_INVALID, "batch: test flags (Gubser, couplings, Riemann) are not batched");
   if (chunk < 1 || chunk > 4096) return clv_host::set_error(CLV_ERR_INVALID, "batch: chunk must be in 1..4096");
   if (rows != 64 && rows != 128) return clv_host::set_error(CLV_ERR_INVALID, "batch: rows must be 64 or 128");
-  if (p.flags & clv::FLAG_FAST) return clv_fastpath::batch_stage_tiled<real>(p, a, step, rows, chunk, grid, s);
-  return clv::batch_launch::stage_tiled<real>(p, a, step, rows, chunk, grid, s);
+  if (p.flags & clv::FLAG_FAST) return clv_fastpath::batch_stage_tiled<real>(p, a, step, grid, s);
+  return clv::batch_launch::stage_tiled<real>(p, a, step, grid, s);
 }
 
 template <class real> int batch_advance_t(const clv_params* pp, const clv_batch* b, int first, cudaStream_t s) {
@@ -134,18 +134,11 @@ int clv_batch_occupancy_tiled(const clv_params* p, int rows, int* blocks_per_sm)
   const bool bulk = p->flags & CLV_FLAG_BULK;
   int n = 0, rc;
   if (p->flags & CLV_FLAG_FAST)
-    rc = p->precision == 4 ? clv_fastpath::batch_occupancy_tiled<float>(bulk, rows, &n)
-                           : clv_fastpath::batch_occupancy_tiled<double>(bulk, rows, &n);
-  else if (p->precision == 4)
-    rc = rows == 64 ? (bulk ? clv::batch_launch::occupancy_tiled<float, true, 64>(&n)
-                            : clv::batch_launch::occupancy_tiled<float, false, 64>(&n))
-                    : (bulk ? clv::batch_launch::occupancy_tiled<float, true, 128>(&n)
-                            : clv::batch_launch::occupancy_tiled<float, false, 128>(&n));
+    rc = p->precision == 4 ? clv_fastpath::batch_occupancy_tiled<float>(bulk, &n)
+                           : clv_fastpath::batch_occupancy_tiled<double>(bulk, &n);
   else
-    rc = rows == 64 ? (bulk ? clv::batch_launch::occupancy_tiled<double, true, 64>(&n)
-                            : clv::batch_launch::occupancy_tiled<double, false, 64>(&n))
-                    : (bulk ? clv::batch_launch::occupancy_tiled<double, true, 128>(&n)
-                            : clv::batch_launch::occupancy_tiled<double, false, 128>(&n));
+    rc = p->precision == 4 ? clv::batch_launch::occupancy_tiled<float>(bulk, &n)
+                           : clv::batch_launch::occupancy_tiled<double>(bulk, &n);
   if (rc) return rc;
   *blocks_per_sm = n;
   return CLV_OK;

@@ -19,6 +19,7 @@
 // the event stops when it is below the freeze-out energy density.
 #pragma once
 #include "clv_stage.cuh"
+#include "clv_stage_patch.cuh"
 #include "clv_stage_tiled2d.cuh"
 
 namespace clv {
@@ -142,49 +143,58 @@ __global__ void __launch_bounds__(BS, MINB) batch_stage_kernel(Params p, BatchAr
   }
 }
 
-// The same stage for batches of (2+1)D events (every event NZ = 1) with the
-// tiled kernel of clv_stage_tiled2d.cuh: the work items are tiles of TB-4 rows
-// by `chunk` x planes; a persistent block takes tiles g = blockIdx.x,
-// blockIdx.x + gridDim.x, ... of the running events in order.
-template <class real, bool BULK, int TB, int MINB>
-__global__ void __launch_bounds__(TB, MINB) batch_tiled2d_kernel(Params p, BatchArgs<real> a, int step, int chunk) {
-  __shared__ int s_tprefix[BATCH_MAX_EVENTS + 1];  // the only static shared memory: 4 KB
+// The same stage for batches of (2+1)D events by patches (clv_stage_patch.cuh):
+// the work items are the TX x TY patches of the running events in order; a
+// persistent block takes patches blockIdx.x, blockIdx.x + gridDim.x, ...
+template <class real, bool BULK, int TX, int TY, int NT, int MINB, int STAGE>
+__global__ void __launch_bounds__(NT, MINB) batch_patch_kernel(Params p, BatchArgs<real> a) {
+  constexpr int step = STAGE;
+  __shared__ int s_prefix[BATCH_MAX_EVENTS + 1];
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Tile2Smem<real, BULK, TB>& sm = *reinterpret_cast<Tile2Smem<real, BULK, TB>*>(smem_raw);
+  PatchSmem<real, BULK, TX, TY>& sm = *reinterpret_cast<PatchSmem<real, BULK, TX, TY>*>(smem_raw);
   const BatchCtl ctl = *a.ctl;
   if (ctl.done) return;
   const int n = ctl.n_active;
-  constexpr int TI = TB - 4;  // rows of a tile
-  for (int q = threadIdx.x; q < n; q += TB) {
-    const BatchEvent E = a.events[a.active[q]];
-    s_tprefix[q + 1] = E.nz == 1 ? ((E.ny + TI - 1) / TI) * ((E.nx + chunk - 1) / chunk) : 0;  // its tiles
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {  // prefix of the tile counts (n <= 1024)
-    s_tprefix[0] = 0;
-    for (int q = 0; q < n; q++) s_tprefix[q + 1] += s_tprefix[q];
+  // inclusive prefix of the events' patch counts: each warp scans 32 events
+  // and adds the total so far (n <= 1024; warp 0 alone)
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    int base = 0;
+    if (lane == 0) s_prefix[0] = 0;
+    for (int q0 = 0; q0 < n; q0 += 32) {
+      int x = 0;
+      if (q0 + lane < n) {
+        const BatchEvent& E = a.events[a.active[q0 + lane]];
+        x = E.nz == 1 ? ((E.ny + TY - 1) / TY) * ((E.nx + TX - 1) / TX) : 0;
+      }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (q0 + lane < n) s_prefix[q0 + lane + 1] = base + x;
+      base += __shfl_sync(0xffffffffu, x, 31);
+    }
   }
   __syncthreads();
   const int loop = ctl.loop;
   const TauConst<real> tc = batch_tau_const<real>(p, a, loop, step);
   const bool fold = (step == 2) && ((loop + 1) % a.ntskip == 0);
-  const int total = s_tprefix[n];
+  const int total = s_prefix[n];
   for (int g = blockIdx.x; g < total; g += gridDim.x) {  // block-uniform
     int lo = 0, hi = n;  // largest slot with prefix <= g
     while (hi - lo > 1) {
-      int mid = (lo + hi) >> 1;
-      if (s_tprefix[mid] <= g) lo = mid;
+      const int mid = (lo + hi) >> 1;
+      if (s_prefix[mid] <= g) lo = mid;
       else hi = mid;
     }
     const int e = a.active[lo];
     const BatchEvent E = a.events[e];
     const GridDims gd{E.nx, E.ny, E.nz, E.ld};
     const ViscBuffers<real> b = batch_buffers<real>(a, E, e, step, fold);
-    const int local = g - s_tprefix[lo];
-    const int nty = (E.ny + TI - 1) / TI;
-    const int ty = local % nty, tx = local / nty;
-    const int i0 = tx * chunk;
-    tile2d<real, BULK, TB>(p, gd, b, step, tc, ty * TI, i0, min(i0 + chunk, E.nx), sm);
+    const int local = g - s_prefix[lo];
+    const int nty = (E.ny + TY - 1) / TY;
+    patch2d<real, BULK, TX, TY, NT, STAGE>(p, gd, b, step, tc, local / nty * TX, local % nty * TY, sm);
     __syncthreads();
   }
 }

@@ -10,6 +10,7 @@
 #include "clv_hypersf.cuh"
 #include "clv_misc.cuh"
 #include "clv_stage.cuh"
+#include "clv_stage_patch.cuh"
 #include "clv_stage_tiled.cuh"
 #include "clv_stage_tiled2d.cuh"
 #include "clv_fast.h"
@@ -240,14 +241,14 @@ int visc_stage_t(const clv::Params& p, int step, double tau, int parts, const cl
   // tolerance arithmetic (CLV_FLAG_FAST) for the fused stage
   if ((p.flags & clv::FLAG_FAST) && is && kt) return clv_fastpath::visc_stage<real>(p, v, step, tau_const<real>(p, tau), o, s);
   // the marching (2+1)D kernel (bulk sector, no coupling terms) when asked
-  // for: the per-cell kernel is faster on the (2+1)D grids of this code
+  // for; the patches below are faster
   const bool fit2d = p.nz == 1 && p.nx >= kTiled2dMin && p.ny >= kTiled2dMin && is && kt && !cpl0;
   if (fit2d && o.stage_kernel == 3)
     return bulk ? launch_tiled2d<real, true>(p, v, step, tau, s) : launch_tiled2d<real, false>(p, v, step, tau, s);
   // The exact tiled kernel has no bulk sector, and its 8 x 32 (y, eta) tile
   // leaves most threads idle on grids with few cells along eta, and it counts
-  // offsets in 32 bits: other runs take the per-cell kernel, which gives the
-  // same bits.  97 x 93 x 65 FP64, one step:
+  // offsets in 32 bits: other runs take the per-cell kernel (or, (2+1)D runs,
+  // the patches), which gives the same bits.  97 x 93 x 65 FP64, one step:
   // 2.11 ms tiled (3.79 ms before the update shared its loads).
   if (!bulk && clv::fits_idx32<real>(p) && (o.stage_kernel == 2 || (o.stage_kernel == 0 && p.nz >= kTiledMinNz))) {
     if (is && kt) return launch_tiled<real, true, true>(p, v, step, tau, s, o);
@@ -255,6 +256,13 @@ int visc_stage_t(const clv::Params& p, int step, double tau, int parts, const cl
     return launch_tiled<real, false, true>(p, v, step, tau, s, o);
   }
   const clv::TauConst<real> t = tau_const<real>(p, tau);
+  // (2+1)D grids: patches (the same bits; clv_stage_patch.cuh has the figures)
+  if (is && kt && !cpl0 && o.stage_kernel == 0 && clv::patch_fits(p)) {
+    if ((bulk ? clv::launch_patch<real, true>(p, v, step, t, s) : clv::launch_patch<real, false>(p, v, step, t, s)) ==
+        cudaSuccess)
+      return CLV_OK;
+    return cuda_check("visc_stage_patch_kernel");
+  }
   const int bs = 128;
   dim3 grid(nblk(ncell(p), bs));
   const bool cpl = p.flags & (clv::FLAG_GUBSER_VISC | clv::FLAG_PIMN_OMEGA | clv::FLAG_OMEGA_OMEGA);

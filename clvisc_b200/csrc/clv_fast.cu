@@ -13,6 +13,7 @@
 #include "../../include/clvisc_b200.h"
 #include "clv_fast.h"
 #include "clv_batch_launch.cuh"
+#include "clv_stage_patch.cuh"
 #include "clv_stage_tiled.cuh"
 
 namespace clv_fastpath {
@@ -118,7 +119,14 @@ int visc_stage(const clv::Params& p, const clv::ViscBuffers<real>& v, int step, 
     return bulk ? launch_tiled2d<real, true, 64>(p, v, step, tc, o.chunk2d, s)
                 : launch_tiled2d<real, false, 64>(p, v, step, tc, o.chunk2d, s);
   }
-  // one thread per cell: (2+1)D grids, short eta axes, coupling terms, the FP64 bulk sector
+  // (2+1)D grids: patches
+  if (!cpl && o.stage_kernel == 0 && clv::patch_fits(p)) {
+    if ((bulk ? clv::launch_patch<real, true>(p, v, step, tc, s) : clv::launch_patch<real, false>(p, v, step, tc, s)) ==
+        cudaSuccess)
+      return CLV_OK;
+    return clv_host::check_cuda("fast visc_stage_patch_kernel");
+  }
+  // one thread per cell: short eta axes, coupling terms, the FP64 bulk sector
   const int bs = 128;
   const long long n = (long long)p.nx * p.ny * p.nz;
   dim3 grid((unsigned int)((n + bs - 1) / bs));
@@ -140,33 +148,26 @@ int batch_stage(const clv::Params& p, const clv::BatchArgs<real>& a, int step, i
 }
 
 template <class real>
-int batch_stage_tiled(const clv::Params& p, const clv::BatchArgs<real>& a, int step, int rows, int chunk, int grid,
-                      cudaStream_t s) {
-  return clv::batch_launch::stage_tiled<real>(p, a, step, rows, chunk, grid, s);
+int batch_stage_tiled(const clv::Params& p, const clv::BatchArgs<real>& a, int step, int grid, cudaStream_t s) {
+  return clv::batch_launch::stage_tiled<real>(p, a, step, grid, s);
 }
 
 template <class real> int batch_occupancy(bool bulk, int bs, int cap, int* n) {
   return bulk ? clv::batch_launch::occupancy<real, true>(bs, cap, n)
               : clv::batch_launch::occupancy<real, false>(bs, cap, n);
 }
-template <class real> int batch_occupancy_tiled(bool bulk, int rows, int* n) {
-  if (rows == 64)
-    return bulk ? clv::batch_launch::occupancy_tiled<real, true, 64>(n)
-                : clv::batch_launch::occupancy_tiled<real, false, 64>(n);
-  return bulk ? clv::batch_launch::occupancy_tiled<real, true, 128>(n)
-              : clv::batch_launch::occupancy_tiled<real, false, 128>(n);
+template <class real> int batch_occupancy_tiled(bool bulk, int* n) {
+  return clv::batch_launch::occupancy_tiled<real>(bulk, n);
 }
 template int batch_occupancy<float>(bool, int, int, int*);
 template int batch_occupancy<double>(bool, int, int, int*);
-template int batch_occupancy_tiled<float>(bool, int, int*);
-template int batch_occupancy_tiled<double>(bool, int, int*);
+template int batch_occupancy_tiled<float>(bool, int*);
+template int batch_occupancy_tiled<double>(bool, int*);
 
 template int batch_stage<float>(const clv::Params&, const clv::BatchArgs<float>&, int, int, int, int, cudaStream_t);
 template int batch_stage<double>(const clv::Params&, const clv::BatchArgs<double>&, int, int, int, int, cudaStream_t);
-template int batch_stage_tiled<float>(const clv::Params&, const clv::BatchArgs<float>&, int, int, int, int,
-                                      cudaStream_t);
-template int batch_stage_tiled<double>(const clv::Params&, const clv::BatchArgs<double>&, int, int, int, int,
-                                       cudaStream_t);
+template int batch_stage_tiled<float>(const clv::Params&, const clv::BatchArgs<float>&, int, int, cudaStream_t);
+template int batch_stage_tiled<double>(const clv::Params&, const clv::BatchArgs<double>&, int, int, cudaStream_t);
 
 template int visc_stage<float>(const clv::Params&, const clv::ViscBuffers<float>&, int, const clv::TauConst<float>&,
                                const clv::StageOpts&, cudaStream_t);

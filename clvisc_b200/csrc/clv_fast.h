@@ -18,14 +18,13 @@ template <class real>
 int visc_stage(const clv::Params& p, const clv::ViscBuffers<real>& v, int step, const clv::TauConst<real>& tc,
                const clv::StageOpts& o, cudaStream_t s);
 // one stage of a batch of events, one thread per cell (block size bs, grid
-// blocks, register cap 0 / 128 / 168) or (2+1)D tiles of rows - 4 rows
+// blocks, register cap 0 / 128 / 168) or (2+1)D patches
 template <class real>
 int batch_stage(const clv::Params& p, const clv::BatchArgs<real>& a, int step, int bs, int grid, int cap,
                 cudaStream_t s);
 template <class real>
-int batch_stage_tiled(const clv::Params& p, const clv::BatchArgs<real>& a, int step, int rows, int chunk, int grid,
-                      cudaStream_t s);
+int batch_stage_tiled(const clv::Params& p, const clv::BatchArgs<real>& a, int step, int grid, cudaStream_t s);
 // resident blocks per SM of the fast batched stage kernels (loads them)
 template <class real> int batch_occupancy(bool bulk, int bs, int cap, int* n);
-template <class real> int batch_occupancy_tiled(bool bulk, int rows, int* n);
+template <class real> int batch_occupancy_tiled(bool bulk, int* n);
 }  // namespace clv_fastpath

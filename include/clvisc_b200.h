@@ -117,11 +117,15 @@ typedef struct clv_visc_buffers {
 /* Tuning options (process-wide defaults; a run's own opt_* fields in
  * clv_params take precedence): the viscous-stage kernel variant
  * (0 = automatic, the default: on grids with at least 24 cells along eta and
- * no bulk sector the tiled (3+1)D kernel, else one thread per cell; 1 = one
- * thread per cell without shared memory; 2 = tiled (3+1)D wherever it
- * applies; 3 = the tiled (2+1)D kernel for the fused stage without coupling
- * terms on (2+1)D grids (NZ = 1, NX and NY >= 4), else as 0), the number of x planes a tiled (3+1)D thread block
- * marches through, and the number of tiled blocks kept resident per SM in
+ * no bulk sector (FP32 tolerance arithmetic: or with it) the tiled (3+1)D
+ * kernel, on (2+1)D grids the patch kernel for the fused stage without
+ * coupling terms, else one thread per cell; 1 = one thread per cell without
+ * shared memory; 2 = tiled (3+1)D wherever it applies; 3 = the marching
+ * (2+1)D kernel for the fused stage without coupling terms on (2+1)D grids
+ * (NZ = 1, NX and NY >= 4), else as 0), the number of x planes a tiled (3+1)D
+ * thread block marches through (the process-wide default, 32, lets the grid
+ * decide; a run's own opt_chunk is taken as it is), and the number of tiled
+ * blocks kept resident per SM in
  * FP32 (1 or 2; FP64 uses 1). Every variant computes the same values bit for
  * bit. */
 #define CLV_OPT_STAGE_KERNEL 1
@@ -291,10 +295,12 @@ int clv_batch_advance(const clv_params *p, const clv_batch *b, int first, void *
 /* Resident blocks per SM of the batch stage kernel at block_size threads. */
 int clv_batch_occupancy(const clv_params *p, int block_size, int max_registers, int *blocks_per_sm);
 /* The same stage for batches of (2+1)D events with the tiled kernel: work
- * items are tiles of (rows - 4) y rows by `chunk` x planes (rows = 64 or 128
- * threads a block), taken in order by grid_blocks persistent blocks
- * (grid_blocks <= 0: fill the GPU once). Every event must have nz = 1: the
- * kernel gives events with nz != 1 no tiles. Same bits as clv_batch_stage. */
+ * items are patches of cells, taken in order by grid_blocks persistent blocks
+ * (grid_blocks <= 0, or above the resident blocks of the GPU: fill it once).
+ * rows must be 64 or 128 and chunk 1 to 4096; the kernel chooses its patch
+ * itself, so neither changes the launch any more. Every event must have
+ * nz = 1: the kernel gives events with nz != 1 no patches. Same bits as
+ * clv_batch_stage. */
 int clv_batch_stage_tiled(const clv_params *p, int step, const clv_batch *b, int rows, int chunk, int grid_blocks,
                           void *stream);
 /* Resident blocks per SM of the tiled batch stage kernel. */
