@@ -8,6 +8,7 @@
 #include "../../include/clvisc_b200.h"
 #include "clv_device.cuh"
 #include "clv_hypersf.cuh"
+#include "clv_ideal_tiled.cuh"
 #include "clv_misc.cuh"
 #include "clv_stage.cuh"
 #include "clv_stage_patch.cuh"
@@ -283,11 +284,40 @@ int visc_stage_t(const clv::Params& p, int step, double tau, int parts, const cl
 }
 
 template <class real>
+int launch_ideal_tiled(const clv::Params& p, const clv::IdealBuffers<real>& b, int step, double tau, cudaStream_t s) {
+  constexpr int TJ = 8, TK = 32, MINB = sizeof(real) == 4 ? 3 : 2;
+  typedef clv::IdealSmem<real, TJ, TK> SM;
+  auto kern = clv::ideal_stage_tiled_kernel<real, TJ, TK, MINB>;
+  static bool configured[kMaxDev] = {};  // the attribute is per device
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return cuda_check("cudaGetDevice");
+  if (!configured[dev]) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SM)) != cudaSuccess)
+      return cuda_check("cudaFuncSetAttribute(ideal_stage_tiled_kernel)");
+    configured[dev] = true;
+  }
+  const int gz = (p.nz + TK - 1) / TK, gy = (p.ny + TJ - 1) / TJ;
+  const int chunk = clv::march_chunk(p.nx, (long long)gz * gy, clv::sm_count() * MINB);
+  kern<<<dim3(gz, gy, (p.nx + chunk - 1) / chunk), TJ * TK, sizeof(SM), s>>>(p, b, step, tau_const<real>(p, tau), chunk);
+  return cuda_check("ideal_stage_tiled_kernel");
+}
+
+template <class real>
 int ideal_stage_t(const clv::Params& p, int step, double tau, const void* ev_st, const void* ev1, void* ev_new,
                   void* src, int write_src, void* key, cudaStream_t s) {
   clv::IdealBuffers<real> b;
   b.ev_st = (const real*)ev_st; b.ev1 = (const real*)ev1; b.evnew = (real*)ev_new; b.src = (real*)src;
   b.edmax_key = (typename clv::KeyT<real>::type*)key; b.write_src = write_src;
+  // The tiled kernel where its 8 x 32 (y, eta) tile is filled (201x201x61
+  // FP32, one stage: 608 us per cell, 390 tiled), patches on (2+1)D grids, the
+  // per-cell kernel on the short eta axes between (2 to 23 cells): the same
+  // bits.
+  if (p.nz >= kTiledMinNz && clv::fits_idx32<real>(p)) return launch_ideal_tiled<real>(p, b, step, tau, s);
+  if (p.nz == 1 && clv::fits_idx32<real>(p) && (p.nx + 7) / 8 <= 65535) {
+    clv::ideal_stage_patch_kernel<real, 8, 8, 64><<<dim3((p.ny + 7) / 8, (p.nx + 7) / 8), 64, 0, s>>>(
+        p, b, step, tau_const<real>(p, tau));
+    return cuda_check("ideal_stage_patch_kernel");
+  }
   const int bs = 128;
   clv::ideal_stage_kernel<real><<<nblk(ncell(p), bs), bs, 0, s>>>(p, b, step, tau_const<real>(p, tau));
   return cuda_check("ideal_stage_kernel");

@@ -15,6 +15,28 @@ BULK = dict(ZETAOS_MAX=0.12, ZETAOS_T0=0.2, ZETAOS_WIDTH=0.05, ZETAOS_SKEW=0.3)
 
 
 @pytest.mark.parametrize('use_float32', [True, False])
+@pytest.mark.parametrize('riemann', [False, True])
+@pytest.mark.parametrize('grid', [(1, 8, 32), (3, 9, 33), (5, 7, 24), (67, 17, 31)])
+def test_ideal_tiled_edges(cuda_lib, oracle_mod, use_float32, riemann, grid):
+    """The tiled ideal stage (eta axes of 24 cells and more), both stages."""
+    from clvisc_b200.ideal import CLIdeal
+    cfg = make_cfg(*grid, use_float32=use_float32, riemann_test=riemann)
+    g, o = CLIdeal(cfg), oracle_mod.OracleIdeal(cfg)
+    ic = seeded_ic(cfg, seed=3, flow=0.3)
+    g.load_ini(ic)
+    o.load_ini(ic)
+    for n in range(3):
+        for step in (1, 2):
+            g.stepUpdate(step)
+            o.stepUpdate(step)
+            assert_same('stage %d src' % step, g.field_to_host(g.d_Src), o.d_Src)
+            assert_same('stage %d ev' % step, g.field_to_host(g.d_ev[3 - step]), o.d_ev[3 - step])
+            if step == 1:
+                g.update_time(n)
+                o.update_time(n)
+
+
+@pytest.mark.parametrize('use_float32', [True, False])
 @pytest.mark.parametrize('arithmetic', ['exact', 'fast'])
 @pytest.mark.parametrize('extra', [{}, BULK], ids=['shear', 'bulk'])
 @pytest.mark.parametrize('grid', [(1, 9, 1), (7, 1, 1), (8, 8, 1), (9, 17, 1), (41, 33, 1), (3, 8, 24), (9, 17, 33),
