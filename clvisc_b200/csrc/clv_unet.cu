@@ -115,11 +115,11 @@ template <int BN, bool SW> int launch_conv_tma(const ConvArgs& a, int bw, cudaSt
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int by_smem = (228 * 1024) / ((int)sizeof(TmaSmem<BN>) + 1024);
-    const int per_sm = std::min(std::min(by_smem, 2048 / TMA_THREADS), 512 / (2 * BN));
+    const int per_sm = std::min(std::min(by_smem, 2048 / tma_threads(BN)), 512 / (2 * BN));
     grid = sms * std::max(per_sm, 1);
   }
   const long long tiles = (long long)a.N * (a.H / (TC_BM / bw)) * (a.W / bw) * (a.Cout / BN);
-  kern<<<(unsigned)std::min<long long>(grid, tiles), TMA_THREADS, sizeof(TmaSmem<BN>), s>>>(ta, tb, a, bw);
+  kern<<<(unsigned)std::min<long long>(grid, tiles), tma_threads(BN), sizeof(TmaSmem<BN>), s>>>(ta, tb, a, bw);
   return clv_host::check_cuda("conv3x3_tma_kernel");
 }
 

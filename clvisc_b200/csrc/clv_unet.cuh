@@ -22,6 +22,7 @@
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <type_traits>
 #include <stdint.h>
 
 namespace clv {
@@ -476,7 +477,10 @@ template <int BN> __global__ void __launch_bounds__(128) conv3x3_tc_kernel(ConvA
 //     one pixel a thread) through the bias / gate / GELU epilogue while the
 //     next tile accumulates in the other one, then free it.
 // Every wait is bounded (g_tc_timeouts); a role whose wait runs out stops.
-constexpr int TMA_THREADS = 192;
+// Threads: a producer warp, an issuer warp, four epilogue warps and, with two or
+// more weight boxes a chunk, a second producer warp for those (one thread issues
+// a load every 150 to 200 cycles, which was the pace of the wide tiles).
+__host__ __device__ constexpr int tma_threads(int BN) { return BN >= 64 ? 224 : 192; }
 
 template <int BN> struct TmaSmem {
   bf16 A[TC_STAGES][TC_BM * TC_BK];
@@ -500,10 +504,11 @@ __device__ __forceinline__ void tma_load2(uint32_t dst, const void* map, int c0,
 }
 
 template <int BN, bool SW>
-__global__ void __launch_bounds__(TMA_THREADS)
+__global__ void __launch_bounds__(tma_threads(BN))
     conv3x3_tma_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, ConvArgs a, int bw) {
   static_assert(BN == 32 || BN == 64 || BN == 128, "BN");
   constexpr int TCOLS = 2 * BN;  // two accumulators
+  constexpr bool WIDE = tma_threads(BN) == 224;
   constexpr uint32_t A_BYTES = TC_BM * TC_BK * 2, B_BYTES = BN * TC_BK * 2;
   // no swizzle: A 8-channel groups (LBO) 2048 B apart, 8-row groups (SBO) 128 B; B 8-row groups (LBO) 128 B,
   // 8-channel groups (SBO) 512 B. 64-byte swizzle: A 8-row atoms (SBO) 512 B apart, K step of 16 channels
@@ -530,7 +535,8 @@ __global__ void __launch_bounds__(TMA_THREADS)
   if (tid == 32) {
 #pragma unroll
     for (int st = 0; st < TC_STAGES; st++) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&s.full[st])) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&s.full[st])), "r"(WIDE ? 2 : 1)
+                   : "memory");
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&s.empty[st])) : "memory");
     }
 #pragma unroll
@@ -556,49 +562,62 @@ __global__ void __launch_bounds__(TMA_THREADS)
     img = (int)(q / tiles_h);
   };
 
-  if (warp == 0) {
-    if (lane == 0) {  // TMA producer
-      // counters in place of divisions: this one thread's instructions, one
-      // after the other, are the pace of a tile with few of them in flight
-      long long it = 0;
-      int st = 0;
-      uint32_t round = 0;  // it / TC_STAGES
-      bool ok = true;
-      for (long long q = blockIdx.x; q < ntiles && ok; q += gridDim.x) {
-        int img, h0, w0, n0;
-        tile(q, img, h0, w0, n0);
-        int row = 0;  // tap Cin + c0 of the weights
-        for (int tap = 0; tap < 9 && ok; tap++) {
-          const int wt = w0 + tap % 3 - 1, ht = h0 + tap / 3 - 1;
-          for (int c0 = 0; c0 < a.Cin; c0 += TC_BK, row += TC_BK, it++) {
-            if (round && !tc_wait(smem_u32(&s.empty[st]), (round - 1) & 1)) {
-              ok = false;
-              atomicAdd(&g_tc_timeouts, 1);
-              break;
-            }
-            const uint32_t fb = smem_u32(&s.full[st]);
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fb), "r"(A_BYTES + B_BYTES)
-                         : "memory");
-            const uint32_t sa = smem_u32(s.A[st]), sb = smem_u32(s.B[st]);
+  // the loads of one thread: the activations (ACT), the weights (WGT) or both
+  auto produce = [&](auto act, auto wgt) {
+    constexpr bool ACT = decltype(act)::value, WGT = decltype(wgt)::value;
+    // counters in place of divisions: this one thread's instructions, one
+    // after the other, are the pace of a tile with few of them in flight
+    long long it = 0;
+    int st = 0;
+    uint32_t round = 0;  // it / TC_STAGES
+    bool ok = true;
+    for (long long q = blockIdx.x; q < ntiles && ok; q += gridDim.x) {
+      int img, h0, w0, n0;
+      tile(q, img, h0, w0, n0);
+      int row = 0;  // tap Cin + c0 of the weights
+      for (int tap = 0; tap < 9 && ok; tap++) {
+        const int wt = w0 + tap % 3 - 1, ht = h0 + tap / 3 - 1;
+        for (int c0 = 0; c0 < a.Cin; c0 += TC_BK, row += TC_BK, it++) {
+          if (round && !tc_wait(smem_u32(&s.empty[st]), (round - 1) & 1)) {
+            ok = false;
+            atomicAdd(&g_tc_timeouts, 1);
+            break;
+          }
+          const uint32_t fb = smem_u32(&s.full[st]);
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fb),
+                       "r"((ACT ? A_BYTES : 0u) + (WGT ? B_BYTES : 0u))
+                       : "memory");
+          const uint32_t sa = smem_u32(s.A[st]), sb = smem_u32(s.B[st]);
+          if constexpr (ACT) {
             if (SW) {
               tma_load4(sa, &ta, a.in_co + c0, wt, ht, img, fb);
-#pragma unroll
-              for (int ng = 0; ng < BN / 32; ng++) tma_load2(sb + ng * 2048, &tb, n0 + 32 * ng, row, fb);
             } else {
 #pragma unroll
               for (int g = 0; g < TC_BK / 8; g++)
                 tma_load4(sa + g * TC_BM * 16, &ta, a.in_co + c0 + 8 * g, wt, ht, img, fb);
+            }
+          }
+          if constexpr (WGT) {
+            if (SW) {
+#pragma unroll
+              for (int ng = 0; ng < BN / 32; ng++) tma_load2(sb + ng * 2048, &tb, n0 + 32 * ng, row, fb);
+            } else {
 #pragma unroll
               for (int ng = 0; ng < BN / 8; ng++) tma_load2(sb + ng * TC_BK * 16, &tb, n0 + 8 * ng, row, fb);
             }
-            if (++st == TC_STAGES) st = 0, round++;
           }
+          if (++st == TC_STAGES) st = 0, round++;
         }
       }
-      // the loads in flight land before the CTA can exit
-      for (long long c = it - 1; c >= 0 && c >= it - TC_STAGES; c--)
-        tc_wait(smem_u32(&s.full[c % TC_STAGES]), (uint32_t)((c / TC_STAGES) & 1));
     }
+    // the loads in flight land before the CTA can exit
+    for (long long c = it - 1; c >= 0 && c >= it - TC_STAGES; c--)
+      tc_wait(smem_u32(&s.full[c % TC_STAGES]), (uint32_t)((c / TC_STAGES) & 1));
+  };
+  if (warp == 0) {
+    if (lane == 0) produce(std::true_type(), std::integral_constant<bool, !WIDE>());
+  } else if (WIDE && warp == 6) {
+    if (lane == 0) produce(std::false_type(), std::true_type());
   } else if (warp == 1) {
     if (lane == 0) {  // MMA issuer
       int t = 0, st = 0;
@@ -780,7 +799,7 @@ __global__ void __launch_bounds__(256) wgrad3x3_kernel(WgradArgs a) {
 // ([32, bw, 64 / bw, 1] boxes of g), K = 64-pixel blocks; both operands are
 // MN-major in the 64-byte swizzled layout. A CTA of 128 threads takes one
 // (row tile, channel tile) and a contiguous range of pixel blocks (split K):
-// thread 0 loads with TMA into WGT_STAGES stages, thread 32 issues the
+// threads 0, 64 and 96 load with TMA into WGT_STAGES stages, thread 32 issues the
 // tcgen05.mma and commits each stage back, and all four warps write the
 // accumulator (one row a thread) as an FP32 partial [split][9 Cin][Cout] that
 // reduce_partials_kernel adds in a fixed order.
@@ -824,7 +843,7 @@ __global__ void __launch_bounds__(128)
   if (tid == 32) {
 #pragma unroll
     for (int st = 0; st < WGT_STAGES; st++) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&s.full[st])) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 3;\n" ::"r"(smem_u32(&s.full[st])) : "memory");
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&s.empty[st])) : "memory");
     }
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&s.done)) : "memory");
@@ -835,11 +854,16 @@ __global__ void __launch_bounds__(128)
   tc_fence_after();
   const uint32_t tmem = s.tmem;
 
-  if (tid == 0) {  // TMA producer
-    int gc[4], gw[4], gh[4];  // rows m0 + 32 i ..: one tap, 32 input channels
+  // Three TMA producers: warp 0 the first two row groups, warp 2 the other two,
+  // warp 3 the gradients. One thread issues a load every 150 to 200 cycles, so
+  // the four to eight boxes of a pixel block from one thread took longer than
+  // its MMAs and loads.
+  if (lane == 0 && warp != 1) {
+    const int b0 = warp == 0 ? 0 : 2, nbox = warp == 3 ? nn / 32 : max(0, min(2, groups - b0));
+    int gc[2], gw[2], gh[2];  // rows m0 + 32 (b0 + i) ..: one tap, 32 input channels
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int r0 = m0 + 32 * i, tap = r0 / a.Cin;
+    for (int i = 0; i < 2; i++) {
+      const int r0 = m0 + 32 * (b0 + i), tap = r0 / a.Cin;
       gc[i] = a.x_co + r0 % a.Cin;
       gw[i] = tap % 3 - 1;
       gh[i] = tap / 3 - 1;
@@ -855,13 +879,16 @@ __global__ void __launch_bounds__(128)
       }
       const uint32_t fb = smem_u32(&s.full[st]);
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fb),
-                   "r"((uint32_t)(groups * 32 + nn) * WGT_BK * 2)
+                   "r"((uint32_t)(nbox * 32) * WGT_BK * 2)
                    : "memory");
       const uint32_t sa = smem_u32(s.A[st]), sb = smem_u32(s.B[st]);
+      if (warp == 3) {
+        for (int ng = 0; ng < nbox; ng++) tma_load4(sb + ng * LBO, &tg, co0 + 32 * ng, w0, h0, img, fb);
+      } else {
 #pragma unroll
-      for (int gi = 0; gi < 4; gi++)
-        if (gi < groups) tma_load4(sa + gi * LBO, &tx, gc[gi], w0 + gw[gi], h0 + gh[gi], img, fb);
-      for (int ng = 0; ng < nn / 32; ng++) tma_load4(sb + ng * LBO, &tg, co0 + 32 * ng, w0, h0, img, fb);
+        for (int i = 0; i < 2; i++)
+          if (i < nbox) tma_load4(sa + (b0 + i) * LBO, &tx, gc[i], w0 + gw[i], h0 + gh[i], img, fb);
+      }
       w0 += bw;  // the next pixel block
       if (w0 == a.W) {
         w0 = 0;
@@ -894,7 +921,7 @@ __global__ void __launch_bounds__(128)
     }
     if (ok && c1 > c0) tc_commit(smem_u32(&s.done));
   }
-  // The other lanes of warps 0 and 1 wait here, not on the barrier: a try_wait
+  // The other lanes of the warps wait here, not on the barrier: a try_wait
   // suspends the whole warp for a time, the producer's or the issuer's lane with
   // it (2.3 us a pixel block, whatever its size, in place of 0.6).
   __syncwarp();
@@ -1148,11 +1175,19 @@ __global__ void __launch_bounds__(512) wgrad_first8_kernel(const float* x, const
   const long long P = (long long)N * H * W;
   const long long p0 = (long long)blockIdx.x * rows, p1 = p0 + rows < P ? p0 + rows : P;
   auto load = [&](long long p, int b) {
-    T::load(g, C, p, p1, C, t - 256, sh[b]);
-    for (int q = t - 256; q < 3 * (T::RMAX + 2); q += 256) {
-      const int d = q / (T::RMAX + 2), i = q - d * (T::RMAX + 2);
+    constexpr int NX = T::RMAX + 2, NQ = (3 * NX + 255) / 256;
+    float v[NQ];
+#pragma unroll
+    for (int u = 0; u < NQ; u++) {
+      const int q = t - 256 + 256 * u, d = q / NX, i = q - d * NX;
       const long long k = p - 1 + (long long)(d - 1) * W + i;
-      xs[b][d][i] = k >= 0 && k < P ? x[k] : 0.0f;
+      v[u] = d < 3 && k >= 0 && k < P ? x[k] : 0.0f;
+    }
+    T::load(g, C, p, p1, C, t - 256, sh[b]);
+#pragma unroll
+    for (int u = 0; u < NQ; u++) {
+      const int q = t - 256 + 256 * u, d = q / NX;
+      if (d < 3) xs[b][d][q - d * NX] = v[u];
     }
   };
   float s[3] = {};
@@ -1168,17 +1203,19 @@ __global__ void __launch_bounds__(512) wgrad_first8_kernel(const float* x, const
       const bf16* gv = sh[b] + c;
       const float* xr = xs[b][tr];
       for (int r = 0; r < n; r += 4) {
-        if (r + 4 <= n && w >= 1 && w + 4 < W && h + tr >= 1 && h + tr <= H) {  // four pixels with all taps inside
-          const float4 a = *reinterpret_cast<const float4*>(xr + r);
-          const float2 e = *reinterpret_cast<const float2*>(xr + r + 4);
-          const float v[6] = {a.x, a.y, a.z, a.w, e.x, e.y};
+        if (r + 8 <= n && w >= 1 && w + 8 < W && h + tr >= 1 && h + tr <= H) {  // eight pixels with all taps inside
+          const float4 a = *reinterpret_cast<const float4*>(xr + r), e = *reinterpret_cast<const float4*>(xr + r + 4);
+          const float2 f = *reinterpret_cast<const float2*>(xr + r + 8);
+          const float v[10] = {a.x, a.y, a.z, a.w, e.x, e.y, e.z, e.w, f.x, f.y};
+          float gj[8];
 #pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const float gj = __bfloat162float(gv[(r + j) * C]);
+          for (int j = 0; j < 8; j++) gj[j] = __bfloat162float(gv[(r + j) * C]);
 #pragma unroll
-            for (int d = 0; d < 3; d++) s[d] += v[j + d] * gj;
-          }
-          w += 4;
+          for (int j = 0; j < 8; j++)
+#pragma unroll
+            for (int d = 0; d < 3; d++) s[d] += v[j + d] * gj[j];
+          w += 8;
+          r += 4;
           continue;
         }
         for (int j = 0; j < 4 && r + j < n; j++) {
@@ -1264,9 +1301,20 @@ __global__ void __launch_bounds__(512) head_wgrad8_kernel(const bf16* y, int y_c
   const int t = threadIdx.x, R = T::rows(C), ng = (K + 2) / 3;
   const long long p0 = (long long)blockIdx.x * rows, p1 = p0 + rows < P ? p0 + rows : P;
   auto load = [&](long long p, int b) {
-    T::load(y + y_co, y_cs, p, p1, C, t - 256, sh[b]);
+    constexpr int NQ = T::RMAX * 8 / 256;
     const int n = (int)min((long long)R, p1 - p) * K;
-    for (int q = t - 256; q < n; q += 256) gs[b][q % K][q / K] = g[p * K + q];
+    float v[NQ];
+#pragma unroll
+    for (int u = 0; u < NQ; u++) {
+      const int q = t - 256 + 256 * u;
+      if (q < n) v[u] = g[p * K + q];
+    }
+    T::load(y + y_co, y_cs, p, p1, C, t - 256, sh[b]);
+#pragma unroll
+    for (int u = 0; u < NQ; u++) {
+      const int q = t - 256 + 256 * u;
+      if (q < n) gs[b][q % K][q / K] = v[u];
+    }
   };
   float s[3] = {};
   const int kg = t / C, c = t - kg * C;
