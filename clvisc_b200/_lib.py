@@ -84,8 +84,12 @@ _SIGS = {
     'clv_alignment': ([], ctypes.c_int),
     'clv_set_option': ([ctypes.c_int, ctypes.c_int], ctypes.c_int),
     'clv_ideal_stage': ([_P, ctypes.c_int, ctypes.c_double, _VP, _VP, _VP, _VP, ctypes.c_int, _VP, _VP], ctypes.c_int),
+    'clv_ideal_steps': ([_P, ctypes.c_int, ctypes.POINTER(ctypes.c_double), _VP, _VP, _VP, _VP, ctypes.c_double,
+                         ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_int), _VP], ctypes.c_int),
     'clv_visc_stage': ([_P, ctypes.c_int, ctypes.c_double, ctypes.c_int, ctypes.POINTER(ClvViscBuffers), _VP],
                        ctypes.c_int),
+    'clv_visc_steps': ([_P, ctypes.c_int, ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ClvViscBuffers),
+                        ctypes.POINTER(ClvViscBuffers), _VP], ctypes.c_int),
     'clv_visc_initialize': ([_P, _VP, _VP, _VP, _VP, ctypes.c_double, _VP], ctypes.c_int),
     'clv_get_udiff': ([_P, _VP, _VP, _VP, _VP], ctypes.c_int),
     'clv_max_ed_reset': ([_P, _VP, _VP], ctypes.c_int),

@@ -419,6 +419,23 @@ int clv_ideal_stage(const clv_params* pp, int step, double tau, const void* ev_s
   return ideal_stage_t<double>(p, step, tau, ev_st, ev1, ev_new, src, write_src, edmax_key, S(stream));
 }
 
+int clv_ideal_steps(const clv_params* pp, int nsteps, const double* tau, void* ev1, void* ev2, void* src, void* key,
+                    double stop_below, double* edmax, int* done, void* stream) {
+  if (!done || nsteps < 0 || (nsteps > 0 && (!tau || !edmax))) return fail(CLV_ERR_INVALID, "ideal_steps: bad argument%s");
+  *done = 0;
+  if (!key) return fail(CLV_ERR_INVALID, "ideal_steps: null key%s");
+  for (int n = 0; n < nsteps; n++) {
+    int rc = clv_ideal_stage(pp, 1, tau[n], ev1, ev1, ev2, src, 1, nullptr, stream);
+    if (!rc) rc = clv_max_ed_reset(pp, key, stream);
+    if (!rc) rc = clv_ideal_stage(pp, 2, tau[n + 1], ev2, ev1, ev1, src, 1, key, stream);
+    if (!rc) rc = clv_max_ed_read(pp, key, edmax + n, stream);
+    if (rc) return rc;
+    *done = n + 1;
+    if (edmax[n] < stop_below) break;
+  }
+  return CLV_OK;
+}
+
 int clv_visc_stage(const clv_params* pp, int step, double tau, int parts, const clv_visc_buffers* b, void* stream) {
   clv::Params p;
   int rc = to_params(pp, &p);
@@ -427,6 +444,30 @@ int clv_visc_stage(const clv_params* pp, int step, double tau, int parts, const 
   if (!b || !(parts & (CLV_PART_IS | CLV_PART_KT)) || (parts & ~3)) return fail(CLV_ERR_INVALID, "bad parts or buffers%s");
   if (pp->precision == 4) return visc_stage_t<float>(p, step, tau, parts, b, S(stream));
   return visc_stage_t<double>(p, step, tau, parts, b, S(stream));
+}
+
+int clv_visc_steps(const clv_params* pp, int nsteps, const double* tau, const clv_visc_buffers* b1,
+                   const clv_visc_buffers* b2, void* stream) {
+  clv::Params p;
+  int rc = to_params(pp, &p);
+  if (rc) return rc;
+  if (!b1 || !b2 || nsteps < 0 || (nsteps > 0 && !tau)) return fail(CLV_ERR_INVALID, "visc_steps: bad argument%s");
+  const int both = CLV_PART_IS | CLV_PART_KT;
+  clv_visc_buffers s1 = *b1, s2 = *b2;
+  s1.edmax_key = nullptr;
+  auto stage = [&](int step, double t, const clv_visc_buffers* b) {
+    return pp->precision == 4 ? visc_stage_t<float>(p, step, t, both, b, S(stream))
+                              : visc_stage_t<double>(p, step, t, both, b, S(stream));
+  };
+  for (int n = 0; n < nsteps; n++) {
+    rc = stage(1, tau[n], &s1);
+    if (rc) return rc;
+    s2.edmax_key = n == nsteps - 1 ? b2->edmax_key : nullptr;
+    if (s2.edmax_key) cudaMemsetAsync(s2.edmax_key, 0, pp->precision, S(stream));
+    rc = stage(2, tau[n + 1], &s2);
+    if (rc) return rc;
+  }
+  return CLV_OK;
 }
 
 int clv_visc_initialize(const clv_params* pp, void* pi1, unsigned char* goodcell, void* udiff, const void* ev,

@@ -245,15 +245,36 @@ class CLIdeal(object):
     def stepUpdate(self, step, jet_eloss_src=None):
         """One Runge-Kutta stage (ideal.py:211-255): d_ev[3-step] from
         d_ev[step], with d_Src zeroed at step 1 and accumulated at step 2."""
+        self._no_jets(jet_eloss_src)
+        self._stage(step)
+
+    def _no_jets(self, jet_eloss_src):
         if jet_eloss_src is not None and jet_eloss_src.get('switch_on', False):
             raise NotImplementedError('jet energy-loss sources are not part of this backend')
+
+    def _stage(self, step, key=None):
         self._call('clv_ideal_stage', int(step), float(self.tau), _lib.ptr(self.d_ev[step]), _lib.ptr(self.d_ev[1]),
-                   _lib.ptr(self.d_ev[3 - step]), _lib.ptr(self.d_Src), 1, None, self.stream)
+                   _lib.ptr(self.d_ev[3 - step]), _lib.ptr(self.d_Src), 1, _lib.ptr(key), self.stream)
+
+    def _steps(self, loop, n, stop_below=None):
+        """Up to n time steps from `loop` in one call of the library, ending
+        after a step whose maximum energy density is below stop_below: (steps
+        taken, the maximum after each)."""
+        tau = [float(self.tau)] + [float(self.cfg.real(self.cfg.TAU0 + (loop + k + 1) * self.cfg.DT)) for k in range(n)]
+        out = (ctypes.c_double * n)()
+        done = ctypes.c_int()
+        self._call('clv_ideal_steps', int(n), (ctypes.c_double * (n + 1))(*tau), _lib.ptr(self.d_ev[1]),
+                   _lib.ptr(self.d_ev[2]), _lib.ptr(self.d_Src), _lib.ptr(self._key),
+                   float('-inf') if stop_below is None else float(stop_below), out, ctypes.byref(done), self.stream)
+        return done.value, [self.cfg.real(v) for v in out[:done.value]]
 
     def max_energy_density(self):
         """Maximum energy density of d_ev[1] (ideal.py:257-262)."""
         self._call('clv_max_ed_reset', _lib.ptr(self._key), self.stream)
         self._call('clv_max_ed', _lib.ptr(self.d_ev[1]), _lib.ptr(self._key), self.stream)
+        return self._read_key()
+
+    def _read_key(self):
         out = ctypes.c_double()
         self._call('clv_max_ed_read', _lib.ptr(self._key), ctypes.byref(out), self.stream)
         return self.cfg.real(out.value)
@@ -308,8 +329,15 @@ class CLIdeal(object):
     def evolve(self, max_loops=2000, save_hypersf=True, save_bulk=True, plot_bulk=True, to_maxloop=False,
                jet_eloss_src=None):
         """Main loop (ideal.py:322-349)."""
-        for n in range(max_loops):
-            self.edmax = self.max_energy_density()
+        # the steps up to the next output go out in one call, whose second
+        # stages fold the maximum of the state they write (a subclass's own
+        # stages keep the separate calls)
+        own = all(getattr(type(self), f) is getattr(CLIdeal, f)
+                  for f in ('stepUpdate', 'max_energy_density', 'update_time'))
+        ahead = []  # the maxima of the states the last call went through
+        n = 0
+        while n < max_loops:
+            self.edmax = ahead.pop(0) if ahead else self.max_energy_density()
             self.history.append([self.tau, self.edmax])
             is_finished = False
             if save_hypersf:
@@ -318,7 +346,24 @@ class CLIdeal(object):
                 break
             if (save_bulk or plot_bulk) and n % self.cfg.ntskip == 0:
                 self.bulkinfo.get(self.tau, self.d_ev[1], self.edmax)
-            self.stepUpdate(step=1)
-            self.update_time(loop=n)
-            self.stepUpdate(step=2, jet_eloss_src=jet_eloss_src)
+            if not own:
+                self.stepUpdate(step=1)
+                self.update_time(loop=n)
+                self.stepUpdate(step=2, jet_eloss_src=jet_eloss_src)
+                n += 1
+                continue
+            self._no_jets(jet_eloss_src)
+            # a state below the freeze-out energy density is looked at on the host
+            k = min(self.cfg.ntskip - n % self.cfg.ntskip, max_loops - n)
+            if is_finished:
+                k = 1
+            done, maxima = self._steps(n, k, self.efrz if save_hypersf else None)
+            # between outputs only the history grows
+            for q in range(1, done):
+                self.update_time(loop=n + q - 1)
+                self.edmax = maxima[q - 1]
+                self.history.append([self.tau, self.edmax])
+            self.update_time(loop=n + done - 1)
+            ahead = [maxima[done - 1]]
+            n += done
         self.save(save_hypersf=save_hypersf, save_bulk=save_bulk)

@@ -172,11 +172,29 @@ size_t clv_params_size(void);
 int clv_ideal_stage(const clv_params *p, int step, double tau, const void *ev_st, const void *ev1,
                     void *ev_new, void *src, int write_src, void *edmax_key, void *stream);
 
+/* Up to nsteps ideal time steps in one call: stage 1 at tau[n] (ev1 -> ev2),
+ * stage 2 at tau[n + 1] (ev2 -> ev1), n = 0 .. nsteps-1 (tau: nsteps + 1 host
+ * values; ideal.py:322-349 with update_time between the stages). After each
+ * step the maximum energy density of ev1 goes to edmax[n] (host; the call waits
+ * for it), and the run ends when it is below stop_below; *done receives the
+ * steps taken. key: a device word for the maximum (clv_max_ed). */
+int clv_ideal_steps(const clv_params *p, int nsteps, const double *tau, void *ev1, void *ev2, void *src, void *key,
+                    double stop_below, double *edmax, int *done, void *stream);
+
 /* One viscous Runge-Kutta stage, any of CLV_PART_IS (visc_src_christoffel,
  * visc_src_alongx/y/z, update_pimn: kernel_IS.cl:41-709) and CLV_PART_KT
  * (kt_src_christoffel, kt_src_alongx/y/z, update_ev: kernel_visc.cl:11-393).
  * With both parts the new pi feeds update_ev from registers. */
 int clv_visc_stage(const clv_params *p, int step, double tau, int parts, const clv_visc_buffers *b, void *stream);
+
+/* nsteps fused viscous time steps (both parts of both stages) in one call:
+ * stage 1 with b1 at tau[n], stage 2 with b2 at tau[n + 1], n = 0 .. nsteps-1
+ * (tau: nsteps + 1 host values; visc.py:527-544 with update_time between the
+ * stages). The same launches as 2 * nsteps clv_visc_stage calls. b2's edmax_key
+ * (nullable) is reset before the last step's second stage and receives that
+ * step's maximum; b1's is ignored. */
+int clv_visc_steps(const clv_params *p, int nsteps, const double *tau, const clv_visc_buffers *b1,
+                   const clv_visc_buffers *b2, void *stream);
 
 /* visc_initialize (kernel_IS.cl:10-36): Navier-Stokes pi from ev, udiff = 0,
  * goodcell = 1. Components of pi1 other than 11, 22, 33 are left as they are.
