@@ -314,8 +314,8 @@ int ideal_stage_t(const clv::Params& p, int step, double tau, const void* ev_st,
   // bits.
   if (p.nz >= kTiledMinNz && clv::fits_idx32<real>(p)) return launch_ideal_tiled<real>(p, b, step, tau, s);
   if (p.nz == 1 && clv::fits_idx32<real>(p) && (p.nx + 7) / 8 <= 65535) {
-    clv::ideal_stage_patch_kernel<real, 8, 8, 64><<<dim3((p.ny + 7) / 8, (p.nx + 7) / 8), 64, 0, s>>>(
-        p, b, step, tau_const<real>(p, tau));
+    clv::launch_early(clv::ideal_stage_patch_kernel<real, 8, 8, 64>, dim3((p.ny + 7) / 8, (p.nx + 7) / 8), 64, 0, s, p, b,
+                      step, tau_const<real>(p, tau));
     return cuda_check("ideal_stage_patch_kernel");
   }
   const int bs = 128;

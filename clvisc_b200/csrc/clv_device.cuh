@@ -17,6 +17,7 @@
 // the arithmetic (clv::exact or clv::fast), so both builds link into one
 // library; plain structs are shared.
 #pragma once
+#include "clv_launch.cuh"
 #include <cuda_runtime.h>
 #include <stdint.h>
 

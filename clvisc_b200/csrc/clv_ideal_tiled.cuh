@@ -289,6 +289,7 @@ template <class real, int TX, int TY> struct IdealPatchSmem {
 template <class real, int TX, int TY, int NT>
 __global__ void __launch_bounds__(NT)
     ideal_stage_patch_kernel(Params p, IdealBuffers<real> b, int step, TauConst<real> tc) {
+  after_previous();
   typedef PatchGeom<TX, TY> G;
   typedef IdealPatchSmem<real, TX, TY> SM;
   constexpr int NP = SM::NP, RG = SM::RG, SG = SM::SG, NS = G::NSX + G::NSY, NF = G::NFX + G::NFY;

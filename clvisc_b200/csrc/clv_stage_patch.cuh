@@ -173,6 +173,7 @@ __device__ __forceinline__ void patch2d(const Params& p, const GridDims& gd, con
 template <class real, bool BULK, int TX, int TY, int NT, int MINB, int STAGE>
 __global__ void __launch_bounds__(NT, MINB)
     visc_stage_patch_kernel(Params p, ViscBuffers<real> b, int step, TauConst<real> tc) {
+  after_previous();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   PatchSmem<real, BULK, TX, TY>& s = *reinterpret_cast<PatchSmem<real, BULK, TX, TY>*>(smem_raw);
   const GridDims gd{p.nx, p.ny, p.nz, p.ld};
@@ -198,8 +199,7 @@ cudaError_t launch_patch_shape(const Params& p, const ViscBuffers<real>& v, int 
     if (e != cudaSuccess) return e;
     configured[kind][dev] = true;
   }
-  kern<<<dim3((p.ny + TY - 1) / TY, (p.nx + TX - 1) / TX), NT, sizeof(SM), s>>>(p, v, step, tc);
-  return cudaGetLastError();
+  return launch_early(kern, dim3((p.ny + TY - 1) / TY, (p.nx + TX - 1) / TX), NT, sizeof(SM), s, p, v, step, tc);
 }
 template <class real, bool BULK>
 cudaError_t launch_patch(const Params& p, const ViscBuffers<real>& v, int step, const TauConst<real>& tc,

@@ -119,7 +119,8 @@ template <int BN, bool SW> int launch_conv_tma(const ConvArgs& a, int bw, cudaSt
     grid = sms * std::max(per_sm, 1);
   }
   const long long tiles = (long long)a.N * (a.H / (TC_BM / bw)) * (a.W / bw) * (a.Cout / BN);
-  kern<<<(unsigned)std::min<long long>(grid, tiles), tma_threads(BN), sizeof(TmaSmem<BN>), s>>>(ta, tb, a, bw);
+  clv::launch_early(kern, (unsigned)std::min<long long>(grid, tiles), tma_threads(BN), sizeof(TmaSmem<BN>), s, ta, tb,
+                    a, bw);
   return clv_host::check_cuda("conv3x3_tma_kernel");
 }
 
@@ -180,7 +181,7 @@ int wgrad_tma(const WgradArgs& a, float* dw, int accumulate, int max_splits, cud
   const long long cps = (nchunks + want - 1) / want;
   const int splits = (int)((nchunks + cps - 1) / cps);  // every split has pixel blocks
   WgradArgs b = a;
-  wgrad3x3_tma_kernel<<<dim3(blocks, splits), 128, sizeof(WgTmaSmem), s>>>(tg, tx, b, bw, (int)cps);
+  clv::launch_early(wgrad3x3_tma_kernel, dim3(blocks, splits), 128, sizeof(WgTmaSmem), s, tg, tx, b, bw, (int)cps);
   int rc = clv_host::check_cuda("wgrad3x3_tma_kernel");
   if (rc) return rc;
   const long long n = 9LL * a.Cin * a.Cout;
@@ -200,7 +201,7 @@ template <int BN> int launch_conv_tc(const ConvArgs& a, long long P, cudaStream_
     configured[cdev] = true;
   }
   dim3 grid(nb(P, TC_BM), a.Cout / BN);
-  kern<<<grid, 128, sizeof(TcSmem<BN>), s>>>(a);
+  clv::launch_early(kern, grid, 128, sizeof(TcSmem<BN>), s, a);
   return clv_host::check_cuda("conv3x3_tc_kernel");
 }
 }  // namespace
@@ -237,10 +238,10 @@ int clv_unet_conv3x3(const clv_unet_conv* args, void* stream) {
   }
   if (a.Cout % 64 == 0) {
     dim3 grid(nb(P, CONV_BM), a.Cout / 64);
-    conv3x3_kernel<64><<<grid, 256, 0, S(stream)>>>(a);
+    clv::launch_early(conv3x3_kernel<64>, grid, 256, 0, S(stream), a);
   } else {
     dim3 grid(nb(P, CONV_BM), a.Cout / 32);
-    conv3x3_kernel<32><<<grid, 256, 0, S(stream)>>>(a);
+    clv::launch_early(conv3x3_kernel<32>, grid, 256, 0, S(stream), a);
   }
   return clv_host::check_cuda("conv3x3_kernel");
 }
@@ -275,7 +276,7 @@ int clv_unet_wgrad3x3(const void* x, int x_cs, int x_co, const void* g, int N, i
   }
   a.pix_per_split = (P + s - 1) / s;
   dim3 grid((9 * Cin + WG_BM - 1) / WG_BM, (Cout + WG_BN - 1) / WG_BN, s);
-  wgrad3x3_kernel<<<grid, 256, 0, S(stream)>>>(a);
+  clv::launch_early(wgrad3x3_kernel, grid, 256, 0, S(stream), a);
   const long long n = 9LL * Cin * Cout;
   reduce_partials(a.part, s, n, dw, accumulate, S(stream));
   return clv_host::check_cuda("wgrad3x3_kernel");
@@ -289,9 +290,9 @@ int clv_unet_bias_grad(const void* g, int g_cs, long long P, int C, float* db, v
     return clv_host::set_error(CLV_ERR_INVALID, "unet_bias_grad: bad argument");
   const long long rows = (P + kRowBlocks - 1) / kRowBlocks;
   if (vec8_ok(g, g_cs, 0) && group8(C))
-    colsum8_kernel<<<kRowBlocks, 512, 0, S(stream)>>>((const bf16*)g, g_cs, P, C, rows, (float*)scratch);
+    clv::launch_early(colsum8_kernel, kRowBlocks, 512, 0, S(stream), (const bf16*)g, g_cs, P, C, rows, (float*)scratch);
   else
-    colsum_kernel<<<kRowBlocks, 128, 0, S(stream)>>>((const bf16*)g, g_cs, P, C, rows, (float*)scratch);
+    clv::launch_early(colsum_kernel, kRowBlocks, 128, 0, S(stream), (const bf16*)g, g_cs, P, C, rows, (float*)scratch);
   reduce_partials((const float*)scratch, kRowBlocks, C, db, 0, S(stream));
   return clv_host::check_cuda("colsum_kernel");
 }
@@ -301,10 +302,11 @@ int clv_unet_first_fwd(const float* x, const float* w, const float* bias, int N,
   if (!x || !w || !bias || !pre || !out) return clv_host::set_error(CLV_ERR_INVALID, "unet_first_fwd: null");
   const long long n = (long long)N * H * W * C;
   if (vec8_ok(pre, C, 0) && vec8_ok(out, out_cs, out_co) && n < kIndex32)
-    conv_first8_kernel<<<nb(n / 8, 256), 256, 0, S(stream)>>>(x, w, bias, N, H, W, C, (bf16*)pre, (bf16*)out, out_cs,
-                                                              out_co);
+    clv::launch_early(conv_first8_kernel, nb(n / 8, 256), 256, 0, S(stream), x, w, bias, N, H, W, C, (bf16*)pre,
+                      (bf16*)out, out_cs, out_co);
   else
-    conv_first_kernel<<<nb(n, 256), 256, 0, S(stream)>>>(x, w, bias, N, H, W, C, (bf16*)pre, (bf16*)out, out_cs, out_co);
+    clv::launch_early(conv_first_kernel, nb(n, 256), 256, 0, S(stream), x, w, bias, N, H, W, C, (bf16*)pre,
+                      (bf16*)out, out_cs, out_co);
   return clv_host::check_cuda("conv_first_kernel");
 }
 
@@ -315,9 +317,11 @@ int clv_unet_first_wgrad(const float* x, const void* g, int N, int H, int W, int
   const long long P = (long long)N * H * W;
   const long long rows = (P + kRowBlocks - 1) / kRowBlocks;
   if (vec8_ok(g, C, 0) && group8(C) && 3 * C <= 256)
-    wgrad_first8_kernel<<<kRowBlocks, 512, 0, S(stream)>>>(x, (const bf16*)g, N, H, W, C, rows, (float*)scratch);
+    clv::launch_early(wgrad_first8_kernel, kRowBlocks, 512, 0, S(stream), x, (const bf16*)g, N, H, W, C, rows,
+                      (float*)scratch);
   else
-    wgrad_first_kernel<<<kRowBlocks, 288, 0, S(stream)>>>(x, (const bf16*)g, N, H, W, C, rows, (float*)scratch);
+    clv::launch_early(wgrad_first_kernel, kRowBlocks, 288, 0, S(stream), x, (const bf16*)g, N, H, W, C, rows,
+                      (float*)scratch);
   reduce_partials((const float*)scratch, kRowBlocks, 9LL * C, dw, 0, S(stream));
   return clv_host::check_cuda("wgrad_first_kernel");
 }
@@ -325,7 +329,7 @@ int clv_unet_first_wgrad(const float* x, const void* g, int N, int H, int W, int
 int clv_unet_head_fwd(const void* y, int y_cs, int y_co, const float* w, const float* b, long long P, int C, int K,
                       float* out, void* stream) {
   if (!y || !w || !b || !out) return clv_host::set_error(CLV_ERR_INVALID, "unet_head_fwd: null");
-  head_fwd_kernel<<<nb(P * K, 256), 256, 0, S(stream)>>>((const bf16*)y, y_cs, y_co, w, b, P, C, K, out);
+  clv::launch_early(head_fwd_kernel, nb(P * K, 256), 256, 0, S(stream), (const bf16*)y, y_cs, y_co, w, b, P, C, K, out);
   return clv_host::check_cuda("head_fwd_kernel");
 }
 
@@ -335,16 +339,17 @@ int clv_unet_head_bwd(const void* y, int y_cs, int y_co, const void* z, const fl
     return clv_host::set_error(CLV_ERR_INVALID, "unet_head_bwd: bad argument");
   const bool v8 = C % 8 == 0 && K <= 8;
   if (v8 && vec8_ok(z, C, 0) && vec8_ok(gz, C, 0) && P * C < kIndex32)
-    head_dgrad8_kernel<<<nb(P * C / 8, 256), 256, 0, S(stream)>>>(g, w, (const bf16*)z, P, C, K, (bf16*)gz);
+    clv::launch_early(head_dgrad8_kernel, nb(P * C / 8, 256), 256, 0, S(stream), g, w, (const bf16*)z, P, C, K,
+                      (bf16*)gz);
   else
-    head_dgrad_kernel<<<nb(P * C, 256), 256, 0, S(stream)>>>(g, w, (const bf16*)z, P, C, K, (bf16*)gz);
+    clv::launch_early(head_dgrad_kernel, nb(P * C, 256), 256, 0, S(stream), g, w, (const bf16*)z, P, C, K, (bf16*)gz);
   const long long rows = (P + kRowBlocks - 1) / kRowBlocks;
   if (v8 && group8(C) && vec8_ok(y, y_cs, y_co) && C * ((K + 2) / 3) + K <= 256)
-    head_wgrad8_kernel<<<kRowBlocks, 512, 0, S(stream)>>>((const bf16*)y, y_cs, y_co, g, P, C, K, rows,
-                                                           (float*)scratch);
+    clv::launch_early(head_wgrad8_kernel, kRowBlocks, 512, 0, S(stream), (const bf16*)y, y_cs, y_co, g, P, C, K, rows,
+                      (float*)scratch);
   else
-    head_wgrad_kernel<<<kRowBlocks, 224, 0, S(stream)>>>((const bf16*)y, y_cs, y_co, g, P, C, K, rows,
-                                                         (float*)scratch);
+    clv::launch_early(head_wgrad_kernel, kRowBlocks, 224, 0, S(stream), (const bf16*)y, y_cs, y_co, g, P, C, K, rows,
+                      (float*)scratch);
   reduce_partials((const float*)scratch, kRowBlocks, (long long)(C + 1) * K, dwb, 0, S(stream));
   return clv_host::check_cuda("head_bwd");
 }
@@ -353,10 +358,11 @@ int clv_unet_pool(const void* x, int x_cs, int x_co, int N, int H, int W, int C,
   if (!x || !out || H % 2 || W % 2) return clv_host::set_error(CLV_ERR_INVALID, "unet_pool: bad argument");
   const long long n8 = (long long)N * H * W * C;
   if (vec8_ok(x, x_cs, x_co) && vec8_ok(out, C, 0) && n8 < kIndex32)
-    pool8_kernel<<<nb(n8 / 32, 256), 256, 0, S(stream)>>>((const bf16*)x, x_cs, x_co, N, H, W, C, (bf16*)out);
+    clv::launch_early(pool8_kernel, nb(n8 / 32, 256), 256, 0, S(stream), (const bf16*)x, x_cs, x_co, N, H, W, C,
+                      (bf16*)out);
   else
-    pool_kernel<<<nb((long long)N * (H / 2) * (W / 2) * C, 256), 256, 0, S(stream)>>>((const bf16*)x, x_cs, x_co, N, H,
-                                                                                      W, C, (bf16*)out);
+    clv::launch_early(pool_kernel, nb((long long)N * (H / 2) * (W / 2) * C, 256), 256, 0, S(stream), (const bf16*)x,
+                      x_cs, x_co, N, H, W, C, (bf16*)out);
   return clv_host::check_cuda("pool_kernel");
 }
 
@@ -364,10 +370,11 @@ int clv_unet_up(const void* x, int N, int H, int W, int C, void* out, int out_cs
   if (!x || !out) return clv_host::set_error(CLV_ERR_INVALID, "unet_up: null");
   const long long n8 = (long long)N * H * W * C;
   if (vec8_ok(x, C, 0) && vec8_ok(out, out_cs, out_co) && n8 < kIndex32)
-    up8_kernel<<<nb(n8 / 8, 256), 256, 0, S(stream)>>>((const bf16*)x, N, H, W, C, (bf16*)out, out_cs, out_co);
+    clv::launch_early(up8_kernel, nb(n8 / 8, 256), 256, 0, S(stream), (const bf16*)x, N, H, W, C, (bf16*)out, out_cs,
+                      out_co);
   else
-    up_kernel<<<nb((long long)N * 4 * H * W * C, 256), 256, 0, S(stream)>>>((const bf16*)x, N, H, W, C, (bf16*)out,
-                                                                          out_cs, out_co);
+    clv::launch_early(up_kernel, nb((long long)N * 4 * H * W * C, 256), 256, 0, S(stream), (const bf16*)x, N, H, W, C,
+                      (bf16*)out, out_cs, out_co);
   return clv_host::check_cuda("up_kernel");
 }
 
@@ -376,11 +383,11 @@ int clv_unet_skip_grad(const void* gcat, int gcat_cs, int gcat_co, const void* g
   if (!gcat || !z || !gz) return clv_host::set_error(CLV_ERR_INVALID, "unet_skip_grad: null");
   const long long n8 = (long long)N * H * W * C;
   if (vec8_ok(gcat, gcat_cs, gcat_co) && vec8_ok(gpool, C, 0) && vec8_ok(z, C, 0) && vec8_ok(gz, C, 0) && n8 < kIndex32)
-    skip_grad8_kernel<<<nb(n8 / 8, 256), 256, 0, S(stream)>>>((const bf16*)gcat, gcat_cs, gcat_co, (const bf16*)gpool,
-                                                              (const bf16*)z, N, H, W, C, (bf16*)gz);
+    clv::launch_early(skip_grad8_kernel, nb(n8 / 8, 256), 256, 0, S(stream), (const bf16*)gcat, gcat_cs, gcat_co,
+                      (const bf16*)gpool, (const bf16*)z, N, H, W, C, (bf16*)gz);
   else
-    skip_grad_kernel<<<nb((long long)N * H * W * C, 256), 256, 0, S(stream)>>>(
-      (const bf16*)gcat, gcat_cs, gcat_co, (const bf16*)gpool, (const bf16*)z, N, H, W, C, (bf16*)gz);
+    clv::launch_early(skip_grad_kernel, nb((long long)N * H * W * C, 256), 256, 0, S(stream), (const bf16*)gcat,
+                      gcat_cs, gcat_co, (const bf16*)gpool, (const bf16*)z, N, H, W, C, (bf16*)gz);
   return clv_host::check_cuda("skip_grad_kernel");
 }
 
@@ -389,11 +396,11 @@ int clv_unet_up_grad(const void* gcat, int gcat_cs, int gcat_co, const void* z, 
   if (!gcat || !z || !gz) return clv_host::set_error(CLV_ERR_INVALID, "unet_up_grad: null");
   const long long n8 = (long long)N * H * W * C;
   if (vec8_ok(gcat, gcat_cs, gcat_co) && vec8_ok(z, C, 0) && vec8_ok(gz, C, 0) && n8 < kIndex32)
-    up_grad8_kernel<<<nb(n8 / 8, 256), 256, 0, S(stream)>>>((const bf16*)gcat, gcat_cs, gcat_co, (const bf16*)z, N, H,
-                                                            W, C, (bf16*)gz);
+    clv::launch_early(up_grad8_kernel, nb(n8 / 8, 256), 256, 0, S(stream), (const bf16*)gcat, gcat_cs, gcat_co,
+                      (const bf16*)z, N, H, W, C, (bf16*)gz);
   else
-    up_grad_kernel<<<nb((long long)N * H * W * C, 256), 256, 0, S(stream)>>>((const bf16*)gcat, gcat_cs, gcat_co,
-                                                                           (const bf16*)z, N, H, W, C, (bf16*)gz);
+    clv::launch_early(up_grad_kernel, nb((long long)N * H * W * C, 256), 256, 0, S(stream), (const bf16*)gcat,
+                      gcat_cs, gcat_co, (const bf16*)z, N, H, W, C, (bf16*)gz);
   return clv_host::check_cuda("up_grad_kernel");
 }
 
@@ -401,14 +408,14 @@ int clv_unet_mse(const float* out, const float* target, const float* wch, long l
                  float* grad, float* part, int nparts, void* stream) {
   if (!out || !target || !wch || !grad || !part || nparts < 1)
     return clv_host::set_error(CLV_ERR_INVALID, "unet_mse: bad argument");
-  mse_kernel<<<nparts, 256, 0, S(stream)>>>(out, target, wch, P, K, scale, grad, part);
+  clv::launch_early(mse_kernel, nparts, 256, 0, S(stream), out, target, wch, P, K, scale, grad, part);
   return clv_host::check_cuda("mse_kernel");
 }
 
 int clv_unet_adam(float* w, const float* g, float* m, float* v, long long n, float lr_t, float b1, float b2,
                   float eps, void* stream) {
   if (!w || !g || !m || !v) return clv_host::set_error(CLV_ERR_INVALID, "unet_adam: null");
-  adam_kernel<<<nb(n, 256), 256, 0, S(stream)>>>(w, g, m, v, n, lr_t, b1, b2, eps);
+  clv::launch_early(adam_kernel, nb(n, 256), 256, 0, S(stream), w, g, m, v, n, lr_t, b1, b2, eps);
   return clv_host::check_cuda("adam_kernel");
 }
 
@@ -432,7 +439,8 @@ int clv_unet_timeouts(int* count, int reset) {
 
 int clv_unet_pack(const float* wf, int Cin, int Cout, void* w, void* wt, void* stream) {
   if (!wf || !w || !wt) return clv_host::set_error(CLV_ERR_INVALID, "unet_pack: null");
-  pack_weights_kernel<<<nb(9LL * Cin * Cout, 256), 256, 0, S(stream)>>>(wf, Cin, Cout, (bf16*)w, (bf16*)wt);
+  clv::launch_early(pack_weights_kernel, nb(9LL * Cin * Cout, 256), 256, 0, S(stream), wf, Cin, Cout, (bf16*)w,
+                    (bf16*)wt);
   return clv_host::check_cuda("pack_weights_kernel");
 }
 

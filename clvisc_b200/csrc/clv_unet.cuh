@@ -25,6 +25,8 @@
 #include <type_traits>
 #include <stdint.h>
 
+#include "clv_launch.cuh"
+
 namespace clv {
 namespace unet {
 
@@ -84,6 +86,7 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
 constexpr int CONV_BM = 128, CONV_BK = 32, A_LD = CONV_BK + 8;
 
 template <int BN> __global__ void __launch_bounds__(256) conv3x3_kernel(ConvArgs a) {
+  after_previous();
   constexpr int B_LD = BN + 8;
   constexpr int WARPS_M = BN == 64 ? 4 : 8;
   constexpr int WM = CONV_BM / WARPS_M;  // 32 or 16
@@ -336,6 +339,7 @@ template <int BN> struct TcSmem {
 };
 
 template <int BN> __global__ void __launch_bounds__(128) conv3x3_tc_kernel(ConvArgs a) {
+  after_previous();
   static_assert(BN == 32 || BN == 64 || BN == 128, "BN");
   constexpr int TCOLS = BN;                    // tensor-memory columns (a power of two >= 32)
   constexpr uint32_t LBO_A = TC_BM / 8 * 128;  // A: K-adjacent core matrices (8 channels apart)
@@ -506,6 +510,7 @@ __device__ __forceinline__ void tma_load2(uint32_t dst, const void* map, int c0,
 template <int BN, bool SW>
 __global__ void __launch_bounds__(tma_threads(BN))
     conv3x3_tma_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, ConvArgs a, int bw) {
+  after_previous();
   static_assert(BN == 32 || BN == 64 || BN == 128, "BN");
   constexpr int TCOLS = 2 * BN;  // two accumulators
   constexpr bool WIDE = tma_threads(BN) == 224;
@@ -697,6 +702,7 @@ constexpr int WG_BM = 64, WG_BN = 64, WG_BK = 32, WG_LD = 64 + 8;
 
 // grid (ceil(9 Cin / 64), ceil(Cout / 64), S); warps 2 (m) x 4 (n) of 32 x 16
 __global__ void __launch_bounds__(256) wgrad3x3_kernel(WgradArgs a) {
+  after_previous();
   __shared__ __align__(16) bf16 sA[2][WG_BK][WG_LD];  // [pixel][(tap, ci)]
   __shared__ __align__(16) bf16 sB[2][WG_BK][WG_LD];  // [pixel][co]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -815,6 +821,7 @@ struct WgTmaSmem {
 __global__ void __launch_bounds__(128)
     wgrad3x3_tma_kernel(const __grid_constant__ CUtensorMap tg, const __grid_constant__ CUtensorMap tx, WgradArgs a,
                         int bw, int chunks_per_split) {
+  after_previous();
   // MN-major, 64-byte swizzle: 32-channel groups (one box each) WGT_BK x 64 B apart, 8-row atoms 512 B,
   // K step of 16 pixel rows 1024 B
   constexpr uint32_t LBO = WGT_BK * 64, SBO = 512, KSTEP = 1024, LAYOUT = 4;
@@ -964,6 +971,7 @@ __global__ void __launch_bounds__(128)
 // out[i] (+)= the sum over S partials of part[k][i], in order, a thread an output
 __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* part, int S, long long n, float* out,
                                                               int accumulate) {
+  after_previous();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float s = 0.0f;
@@ -979,6 +987,7 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* part,
 constexpr int RED_ROWS = 320;
 __global__ void __launch_bounds__(1024) reduce_few_kernel(const float* part, int S, long long n, float* out,
                                                           int accumulate) {
+  after_previous();
   __shared__ float sh[RED_ROWS][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long long i = (long long)blockIdx.x * 32 + lane;
@@ -1000,8 +1009,10 @@ __global__ void __launch_bounds__(1024) reduce_few_kernel(const float* part, int
   if (w == 0 && i < n) out[i] = accumulate ? out[i] + s : s;
 }
 inline void reduce_partials(const float* part, int S, long long n, float* out, int accumulate, cudaStream_t s) {
-  if (n < 65536) reduce_few_kernel<<<(unsigned int)((n + 31) / 32), 1024, 0, s>>>(part, S, n, out, accumulate);
-  else reduce_partials_kernel<<<(unsigned int)((n + 255) / 256), 256, 0, s>>>(part, S, n, out, accumulate);
+  if (n < 65536) clv::launch_early(reduce_few_kernel, (unsigned int)((n + 31) / 32), 1024, 0, s, part, S, n, out,
+                        accumulate);
+  else clv::launch_early(reduce_partials_kernel, (unsigned int)((n + 255) / 256), 256, 0, s, part, S, n, out,
+                        accumulate);
 }
 
 // Eight neighbouring channels (16 bytes) a thread for the layers below where
@@ -1041,6 +1052,7 @@ inline bool vec8_ok(const void* p, int cs, int co) {
 
 // column sums of g[P][C] (bias gradient): block b sums rows [b*rows, ...) into part[b][C]
 __global__ void colsum_kernel(const bf16* g, int g_cs, long long P, int C, long long rows, float* part) {
+  after_previous();
   const long long p0 = (long long)blockIdx.x * rows;
   const long long p1 = p0 + rows < P ? p0 + rows : P;
   for (int c = threadIdx.x; c < C; c += blockDim.x) {
@@ -1080,6 +1092,7 @@ template <int NV> struct RowTile {
 };
 __global__ void __launch_bounds__(512) colsum8_kernel(const bf16* g, int g_cs, long long P, int C, long long rows,
                                                       float* part) {
+  after_previous();
   typedef RowTile<4> T;
   __shared__ __align__(16) bf16 sh[2][T::NE];
   const int t = threadIdx.x, R = T::rows(C);
@@ -1105,6 +1118,7 @@ __global__ void __launch_bounds__(512) colsum8_kernel(const bf16* g, int g_cs, l
 // first layer: 1 input channel (FP32 image) -> C channels, bias, GELU
 __global__ void conv_first_kernel(const float* x, const float* w /*[9][C]*/, const float* bias, int N, int H, int W,
                                   int C, bf16* pre, bf16* out, int out_cs, int out_co) {
+  after_previous();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long P = (long long)N * H * W;
   if (t >= P * C) return;
@@ -1123,6 +1137,7 @@ __global__ void conv_first_kernel(const float* x, const float* w /*[9][C]*/, con
 // its weight gradient: part[b][tap][c] = sum over pixel block b of x[p + tap] g[p][c]
 __global__ void wgrad_first_kernel(const float* x, const bf16* g, int N, int H, int W, int C, long long rows,
                                    float* part) {
+  after_previous();
   const long long P = (long long)N * H * W;
   const long long p0 = (long long)blockIdx.x * rows, p1 = p0 + rows < P ? p0 + rows : P;
   for (int q = threadIdx.x; q < 9 * C; q += blockDim.x) {
@@ -1143,6 +1158,7 @@ __global__ void wgrad_first_kernel(const float* x, const bf16* g, int N, int H, 
 __global__ void __launch_bounds__(256) conv_first8_kernel(const float* x, const float* w, const float* bias, int N,
                                                           int H, int W, int C, bf16* pre, bf16* out, int out_cs,
                                                           int out_co) {
+  after_previous();
   const unsigned int t = blockIdx.x * 256u + threadIdx.x, cg = (unsigned int)C / 8u;
   const unsigned int p = t / cg, c = 8u * (t % cg);
   if (p >= (unsigned int)(N * H * W)) return;
@@ -1168,6 +1184,7 @@ __global__ void __launch_bounds__(256) conv_first8_kernel(const float* x, const 
 // inputs are too: x[p + dr W + ds].
 __global__ void __launch_bounds__(512) wgrad_first8_kernel(const float* x, const bf16* g, int N, int H, int W, int C,
                                                            long long rows, float* part) {
+  after_previous();
   typedef RowTile<2> T;
   __shared__ __align__(16) bf16 sh[2][T::NE];
   __shared__ __align__(16) float xs[2][3][T::RMAX + 4];  // x[p - 1 + dr W + i]
@@ -1240,6 +1257,7 @@ __global__ void __launch_bounds__(512) wgrad_first8_kernel(const float* x, const
 // head: 1x1 convolution C -> K (FP32 out)
 __global__ void head_fwd_kernel(const bf16* y, int y_cs, int y_co, const float* w /*[C][K]*/, const float* b,
                                 long long P, int C, int K, float* out) {
+  after_previous();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= P * K) return;
   const long long p = t / K;
@@ -1250,6 +1268,7 @@ __global__ void head_fwd_kernel(const bf16* y, int y_cs, int y_co, const float* 
 }
 // head backward to its input, times GELU'(z): gy[p][c] = gelu'(z[p][c]) sum_k g[p][k] w[c][k]
 __global__ void head_dgrad_kernel(const float* g, const float* w, const bf16* z, long long P, int C, int K, bf16* gz) {
+  after_previous();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= P * C) return;
   const long long p = t / C;
@@ -1261,6 +1280,7 @@ __global__ void head_dgrad_kernel(const float* g, const float* w, const bf16* z,
 // head weight and bias gradients: part[b][c][k] and part[b][C][k] over pixel block b
 __global__ void head_wgrad_kernel(const bf16* y, int y_cs, int y_co, const float* g, long long P, int C, int K,
                                   long long rows, float* part) {
+  after_previous();
   const long long p0 = (long long)blockIdx.x * rows, p1 = p0 + rows < P ? p0 + rows : P;
   for (int q = threadIdx.x; q < (C + 1) * K; q += blockDim.x) {
     const int c = q / K, k = q % K;
@@ -1274,6 +1294,7 @@ __global__ void head_wgrad_kernel(const bf16* y, int y_cs, int y_co, const float
 // head backward with 8 channels a thread (K <= 8); per output the same order
 __global__ void __launch_bounds__(256) head_dgrad8_kernel(const float* g, const float* w, const bf16* z, long long P,
                                                           int C, int K, bf16* gz) {
+  after_previous();
   const unsigned int t = blockIdx.x * 256u + threadIdx.x, cg = (unsigned int)C / 8u;
   const unsigned int p = t / cg, c = 8u * (t % cg);
   if (p >= (unsigned int)P) return;
@@ -1295,6 +1316,7 @@ __global__ void __launch_bounds__(256) head_dgrad8_kernel(const float* g, const 
 // K <= 8)
 __global__ void __launch_bounds__(512) head_wgrad8_kernel(const bf16* y, int y_cs, int y_co, const float* g,
                                                           long long P, int C, int K, long long rows, float* part) {
+  after_previous();
   typedef RowTile<2> T;
   __shared__ __align__(16) bf16 sh[2][T::NE];
   __shared__ __align__(16) float gs[2][9][T::RMAX];  // g[p + r][k] at [k][r]
@@ -1366,6 +1388,7 @@ __global__ void __launch_bounds__(512) head_wgrad8_kernel(const bf16* y, int y_c
 
 // 2x2 average pooling of a channel slice
 __global__ void pool_kernel(const bf16* x, int x_cs, int x_co, int N, int H, int W, int C, bf16* out) {
+  after_previous();
   const int Ho = H / 2, Wo = W / 2;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)N * Ho * Wo * C) return;
@@ -1381,6 +1404,7 @@ __global__ void pool_kernel(const bf16* x, int x_cs, int x_co, int N, int H, int
 }
 // nearest 2x upsampling into a channel slice
 __global__ void up_kernel(const bf16* x, int N, int H, int W, int C, bf16* out, int out_cs, int out_co) {
+  after_previous();
   const int Ho = 2 * H, Wo = 2 * W;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)N * Ho * Wo * C) return;
@@ -1393,6 +1417,7 @@ __global__ void up_kernel(const bf16* x, int N, int H, int W, int C, bf16* out, 
 // and input of the pooling): gz = (gcat[p][co + c] + gpool[p/2][c] / 4) gelu'(z)
 __global__ void skip_grad_kernel(const bf16* gcat, int gcat_cs, int gcat_co, const bf16* gpool, const bf16* z, int N,
                                  int H, int W, int C, bf16* gz) {
+  after_previous();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)N * H * W * C) return;
   const int c = (int)(t % C);
@@ -1405,6 +1430,7 @@ __global__ void skip_grad_kernel(const bf16* gcat, int gcat_cs, int gcat_co, con
 // upsampling backward (sum of the 4 children of a channel slice) times gelu'(z)
 __global__ void up_grad_kernel(const bf16* gcat, int gcat_cs, int gcat_co, const bf16* z, int N, int H, int W, int C,
                                bf16* gz) {
+  after_previous();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)N * H * W * C) return;
   const int c = (int)(t % C);
@@ -1422,6 +1448,7 @@ __global__ void up_grad_kernel(const bf16* gcat, int gcat_cs, int gcat_co, const
 // is the one-channel kernels' expression
 __global__ void __launch_bounds__(256) pool8_kernel(const bf16* x, int x_cs, int x_co, int N, int H, int W, int C,
                                                     bf16* out) {
+  after_previous();
   const unsigned int t = blockIdx.x * 256u + threadIdx.x, cg = (unsigned int)C / 8u, Ho = H / 2, Wo = W / 2;
   const unsigned int q = t / cg, c = 8u * (t % cg);
   if (q >= N * Ho * Wo) return;
@@ -1440,6 +1467,7 @@ __global__ void __launch_bounds__(256) pool8_kernel(const bf16* x, int x_cs, int
 }
 __global__ void __launch_bounds__(256) up8_kernel(const bf16* x, int N, int H, int W, int C, bf16* out, int out_cs,
                                                   int out_co) {
+  after_previous();
   const unsigned int t = blockIdx.x * 256u + threadIdx.x, cg = (unsigned int)C / 8u;
   const unsigned int q = t / cg, c = 8u * (t % cg);
   if (q >= (unsigned int)(N * H * W)) return;  // an input pixel: read once, written four times
@@ -1453,6 +1481,7 @@ __global__ void __launch_bounds__(256) up8_kernel(const bf16* x, int N, int H, i
 }
 __global__ void __launch_bounds__(256) skip_grad8_kernel(const bf16* gcat, int gcat_cs, int gcat_co, const bf16* gpool,
                                                          const bf16* z, int N, int H, int W, int C, bf16* gz) {
+  after_previous();
   const unsigned int t = blockIdx.x * 256u + threadIdx.x, cg = (unsigned int)C / 8u;
   const unsigned int p = t / cg, c = 8u * (t % cg);
   if (p >= (unsigned int)(N * H * W)) return;
@@ -1470,6 +1499,7 @@ __global__ void __launch_bounds__(256) skip_grad8_kernel(const bf16* gcat, int g
 }
 __global__ void __launch_bounds__(256) up_grad8_kernel(const bf16* gcat, int gcat_cs, int gcat_co, const bf16* z, int N,
                                                        int H, int W, int C, bf16* gz) {
+  after_previous();
   const unsigned int t = blockIdx.x * 256u + threadIdx.x, cg = (unsigned int)C / 8u;
   const unsigned int q = t / cg, c = 8u * (t % cg);
   if (q >= (unsigned int)(N * H * W)) return;
@@ -1491,6 +1521,7 @@ __global__ void __launch_bounds__(256) up_grad8_kernel(const bf16* gcat, int gca
 // weighted squared error: loss partials per block, gradient dL/dout
 __global__ void mse_kernel(const float* out, const float* target, const float* wch, long long P, int K, float scale,
                            float* grad, float* part) {
+  after_previous();
   __shared__ float sh[256];
   const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   float s = 0.0f;
@@ -1512,6 +1543,7 @@ __global__ void mse_kernel(const float* out, const float* target, const float* w
 // Adam on FP32 master weights (Kingma and Ba, 2015), bias-corrected step size given
 __global__ void adam_kernel(float* w, const float* g, float* m, float* v, long long n, float lr_t, float b1, float b2,
                             float eps) {
+  after_previous();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float gi = g[i];
@@ -1525,6 +1557,7 @@ __global__ void adam_kernel(float* w, const float* g, float* m, float* v, long l
 // BF16 weights of a 3x3 layer from FP32 [9][Cin][Cout]: w (same layout) and,
 // for the input gradient, wt[tap][co][ci] = w[8 - tap][ci][co]
 __global__ void pack_weights_kernel(const float* wf, int Cin, int Cout, bf16* w, bf16* wt) {
+  after_previous();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 9LL * Cin * Cout) return;
   const int co = (int)(t % Cout);
