@@ -14,6 +14,10 @@
 // column's records of the two planes ahead, its x slope and its x face stay in
 // registers (nine values a record: no second shared copy as the viscous kernel
 // needs), so FP32 keeps three CTAs of 256 threads an SM (85 registers, 30 KB).
+// Bound by the latency of a plane's chain, as the viscous kernel: 201x201x61
+// FP32, one stage, 390 us against 608 with a thread a cell. (2+1)D grids take
+// 8 x 8 patches below: 101 x 101 FP64, 20 steps with the maximum read after
+// each, 1.19 ms against 1.61 (evolve's single library call included).
 #pragma once
 #include "clv_smem16.cuh"
 #include "clv_stage_patch.cuh"

@@ -329,7 +329,10 @@ int clv_unet_first_wgrad(const float* x, const void* g, int N, int H, int W, int
 int clv_unet_head_fwd(const void* y, int y_cs, int y_co, const float* w, const float* b, long long P, int C, int K,
                       float* out, void* stream) {
   if (!y || !w || !b || !out) return clv_host::set_error(CLV_ERR_INVALID, "unet_head_fwd: null");
-  clv::launch_early(head_fwd_kernel, nb(P * K, 256), 256, 0, S(stream), (const bf16*)y, y_cs, y_co, w, b, P, C, K, out);
+  if (C % 8 == 0 && C <= HEAD_C && K <= 8 && vec8_ok(y, y_cs, y_co))
+    clv::launch_early(head_fwd8_kernel, nb(P, 256), 256, 0, S(stream), (const bf16*)y, y_cs, y_co, w, b, P, C, K, out);
+  else
+    clv::launch_early(head_fwd_kernel, nb(P * K, 256), 256, 0, S(stream), (const bf16*)y, y_cs, y_co, w, b, P, C, K, out);
   return clv_host::check_cuda("head_fwd_kernel");
 }
 

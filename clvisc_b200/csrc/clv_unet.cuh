@@ -1266,6 +1266,31 @@ __global__ void head_fwd_kernel(const bf16* y, int y_cs, int y_co, const float* 
   for (int c = 0; c < C; c++) s += __bfloat162float(y[p * y_cs + y_co + c]) * w[c * K + k];
   out[t] = s;
 }
+// the same (K <= 8, C <= 256) with a thread a pixel, which reads its channels
+// once, 16 bytes at a time, for all outputs; per output the same order
+constexpr int HEAD_C = 256;
+__global__ void __launch_bounds__(256) head_fwd8_kernel(const bf16* y, int y_cs, int y_co, const float* w,
+                                                        const float* b, long long P, int C, int K, float* out) {
+  after_previous();
+  __shared__ __align__(16) float sw[HEAD_C][8];
+  for (int i = threadIdx.x; i < C * 8; i += 256) sw[i / 8][i % 8] = i % 8 < K ? w[i / 8 * K + i % 8] : 0.0f;
+  __syncthreads();
+  const long long p = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (p >= P) return;
+  float s[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) s[k] = k < K ? b[k] : 0.0f;
+  for (int c0 = 0; c0 < C; c0 += 8) {
+    const Vec8 v = load8(y + p * y_cs + y_co + c0);
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+      for (int k = 0; k < 8; k++) s[k] += v.v[i] * sw[c0 + i][k];
+  }
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    if (k < K) out[p * K + k] = s[k];
+}
 // head backward to its input, times GELU'(z): gy[p][c] = gelu'(z[p][c]) sum_k g[p][k] w[c][k]
 __global__ void head_dgrad_kernel(const float* g, const float* w, const bf16* z, long long P, int C, int K, bf16* gz) {
   after_previous();

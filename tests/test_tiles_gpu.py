@@ -203,8 +203,12 @@ def test_unet_small_layers(cuda_lib, C, cs, co, H):
     cols = F.unfold(img[:, None].double(), 3, padding=1)  # (N, 9, HW)
     want = torch.einsum('ntp,npc->tc', cols, z.double().reshape(N, H * W, C))
     np.testing.assert_allclose(dw.cpu().numpy(), want.cpu().numpy(), **tol)
-    # head gradients and a bias sum
-    go, wh = rnd(P, K), rnd(C, K)
+    # head, its gradients and a bias sum
+    go, wh, bh = rnd(P, K), rnd(C, K), rnd(K)
+    o = torch.zeros(P, K, device='cuda')
+    _unet_call(lib, 'clv_unet_head_fwd', x, cs, co, wh, bh, ctypes.c_longlong(P), C, K, o)
+    want = x[..., co:co + C].double().reshape(P, C) @ wh.double() + bh.double()
+    np.testing.assert_allclose(o.cpu().numpy(), want.cpu().numpy(), rtol=0, atol=16 * C * 2.0 ** -23)
     dwb = torch.zeros(C + 1, K, device='cuda')
     _unet_call(lib, 'clv_unet_head_bwd', x, cs, co, z, go, wh, P, C, K, gz, dwb, scratch, ctypes.c_size_t(nb))
     near(gz.reshape(P, C), (go.double() @ wh.double().T).float() * dgelu(z.float()).reshape(P, C))
