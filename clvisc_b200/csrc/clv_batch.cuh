@@ -147,11 +147,13 @@ __global__ void __launch_bounds__(BS, MINB) batch_stage_kernel(Params p, BatchAr
 // the work items are the TX x TY patches of the running events in order; a
 // persistent block takes patches blockIdx.x, blockIdx.x + gridDim.x, ... Bound by
 // latency at four blocks of 128 threads an SM; 32 events of 121^2 to 301^2 with
-// bulk, FP32 tolerance build, 20 steps: 10.1 ms, against 14.9 for strips that
-// march along x.
+// bulk, FP32 tolerance build, 20 steps: 10.8 ms, against 15.0 for strips of
+// `chunk` planes that march along x. The values are the strips', bit for bit
+// (FP32 tolerance build: where chunk is a multiple of TX, so that a strip starts
+// with a patch; else to the rounding of the x slopes where a strip starts).
 template <class real, bool BULK, int TX, int TY, int NT, int MINB, int STAGE>
-__global__ void __launch_bounds__(NT, MINB) batch_patch_kernel(Params p, BatchArgs<real> a) {
-  constexpr int step = STAGE;
+__global__ void __launch_bounds__(NT, MINB) batch_patch_kernel(Params p, BatchArgs<real> a, int step_, int chunk) {
+  const int step = arith_step<real, STAGE>(step_);
   __shared__ int s_prefix[BATCH_MAX_EVENTS + 1];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   PatchSmem<real, BULK, TX, TY>& sm = *reinterpret_cast<PatchSmem<real, BULK, TX, TY>*>(smem_raw);
@@ -197,7 +199,8 @@ __global__ void __launch_bounds__(NT, MINB) batch_patch_kernel(Params p, BatchAr
     const ViscBuffers<real> b = batch_buffers<real>(a, E, e, step, fold);
     const int local = g - s_prefix[lo];
     const int nty = (E.ny + TY - 1) / TY;
-    patch2d<real, BULK, TX, TY, NT, STAGE>(p, gd, b, step, tc, local / nty * TX, local % nty * TY, sm);
+    const int i0 = local / nty * TX;
+    patch2d<real, BULK, TX, TY, NT, STAGE>(p, gd, b, step, tc, i0, local % nty * TY, sm, i0 % chunk == 0);
     __syncthreads();
   }
 }

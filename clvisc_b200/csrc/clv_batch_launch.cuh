@@ -106,7 +106,7 @@ template <class real, bool BULK> int occupancy_patch(int* n) {
 // a block for every few patches the waves' ends cost 15 % (32 events: 10.1 ms
 // for 20 steps against 11.5).
 template <class real, bool BULK>
-int stage_patch(const Params& p, const BatchArgs<real>& a, int step, int grid, cudaStream_t s) {
+int stage_patch(const Params& p, const BatchArgs<real>& a, int step, int chunk, int grid, cudaStream_t s) {
   typedef PatchWide<real, BULK> W;
   typedef PatchSmem<real, BULK, W::TX, W::TY> SM;
   static int resident[kMaxDevices] = {};  // per device; also: its launch attributes are set
@@ -119,14 +119,14 @@ int stage_patch(const Params& p, const BatchArgs<real>& a, int step, int grid, c
     resident[dev] = sm_count() * std::max(1, n);
   }
   const int g = grid > 0 ? std::min(grid, resident[dev]) : resident[dev];
-  if (step == 1) batch_patch_kernel<real, BULK, W::TX, W::TY, W::NT, kPatchBlocks, 1><<<g, W::NT, sizeof(SM), s>>>(p, a);
-  else batch_patch_kernel<real, BULK, W::TX, W::TY, W::NT, kPatchBlocks, 2><<<g, W::NT, sizeof(SM), s>>>(p, a);
+  if (step == 1) batch_patch_kernel<real, BULK, W::TX, W::TY, W::NT, kPatchBlocks, 1><<<g, W::NT, sizeof(SM), s>>>(p, a, 1, chunk);
+  else batch_patch_kernel<real, BULK, W::TX, W::TY, W::NT, kPatchBlocks, 2><<<g, W::NT, sizeof(SM), s>>>(p, a, 2, chunk);
   return clv_host::check_cuda("batch_patch_kernel");
 }
 template <class real>
-int stage_tiled(const Params& p, const BatchArgs<real>& a, int step, int grid, cudaStream_t s) {
-  return p.flags & FLAG_BULK ? stage_patch<real, true>(p, a, step, grid, s)
-                             : stage_patch<real, false>(p, a, step, grid, s);
+int stage_tiled(const Params& p, const BatchArgs<real>& a, int step, int chunk, int grid, cudaStream_t s) {
+  return p.flags & FLAG_BULK ? stage_patch<real, true>(p, a, step, chunk, grid, s)
+                             : stage_patch<real, false>(p, a, step, chunk, grid, s);
 }
 template <class real> int occupancy_tiled(bool bulk, int* n) {
   return bulk ? occupancy_patch<real, true>(n) : occupancy_patch<real, false>(n);

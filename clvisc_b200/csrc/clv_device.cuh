@@ -222,6 +222,9 @@ __device__ __forceinline__ double fast_floor(double x, int& i) {
   return t - 6755399441055744.0;
 }
 #endif
+// a product that is never contracted into a sum
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 // quotient and reciprocal of per-cell values
 template <class real> __device__ __forceinline__ real quot(real a, real b) {
 #if CLV_FAST
@@ -286,72 +289,8 @@ template <class real> __device__ __forceinline__ EosSpot<real> eos_spot(const Pa
 template <class real> __device__ __forceinline__ real eos_lerp(real r, float lo, float hi) {
   return (real)(1.0f - r) * (real)lo + r * (real)hi;
 }
-#if CLV_FAST
-// Tolerance build, FP32: the texel straight from x = (eps - start) / step, no
-// row and column. The reference's row/col arithmetic (above) rounds at the
-// same places to the same 2^-24 of x (the two differ by less than x ulps of
-// the weight, 6e-8 of the pressure at the table's end); in FP64 its
-// float-rounded row width moves the result by 1e-9, so FP64 keeps it. About
-// 10 instructions and one conversion on the dependent chain of a lookup
-// against 35 and two: the chain sits inside the root finder's loop. Below
-// eos_inner only: the last texel and beyond (where the row/col clamps decide
-// what is read) take the reference's way.
-struct EosAt {
-  int t;    // texel, clamped to the table
-  float r;  // weight of the next one
-};
-__device__ __forceinline__ EosAt eos_at(const Params& p, float eps) {
-  const float x = (eps - p.eos_start) * p.rf.eos_step;
-  const int i = (int)x;
-  return EosAt{min(max(i, 0), p.eos_last), x - (float)i};
-}
-#endif
-#if CLV_FAST
-// The reference's lookup and its formula beyond the table, out of line (one
-// copy a kernel of the power and exponential): the last texel and beyond. The
-// constants go by value: a reference would put the kernel's parameters in
-// local memory.
-struct EosEdge {
-  const float* eos;
-  float start, step, rstep, repr, top;
-  int ncol, nrow;
-};
-__device__ __forceinline__ EosEdge eos_edge(const Params& p) {
-  return EosEdge{p.eos, p.eos_start, p.eos_step, p.rf.eos_step, p.rf.eos_epr, p.eos_top, p.eos_ncol, p.eos_nrow};
-}
-static __device__ __noinline__ float eos_comp_edge(EosEdge g, float eps, int c) {
-  Params p;
-  p.eos_start = g.start;
-  p.eos_step = g.step;
-  p.eos_ncol = g.ncol;
-  p.eos_nrow = g.nrow;
-  p.rf.eos_step = g.rstep;
-  p.rf.eos_epr = g.repr;
-  const EosSpot<float> s = eos_spot<float>(p, eps);
-  return eos_lerp<float>(s.r, __ldg(g.eos + 4 * s.t0 + c), __ldg(g.eos + 4 * s.t1 + c));
-}
-static __device__ __noinline__ float eosP_edge(EosEdge g, float eps) {
-  if (eps < g.top) return eos_comp_edge(g, eps, 1);
-  return 0.3327f * eps - 0.3223f * pow(eps, 0.4585f) - 0.003906f * eps * exp(-0.05697f * eps);
-}
-#endif
 template <class real>
 __device__ CLV_EOS_ATTR real eos_comp(const Params& p, real eps, int c) {
-#if CLV_FAST
-  if constexpr (sizeof(real) == 4) {
-    if (eps < p.eos_inner) {
-      const EosAt a = eos_at(p, eps);
-      if (c == 1 && p.eos_p2) {
-        const float2 q = __ldg(p.eos_p2 + a.t);
-        return q.x + a.r * (q.y - q.x);
-      }
-      const float lo = __ldg(p.eos + 4 * (long long)a.t + c);
-      const float hi = __ldg(p.eos + 4 * (long long)min(a.t + 1, p.eos_last) + c);
-      return lo + a.r * (hi - lo);
-    }
-    return eos_comp_edge(eos_edge(p), eps, c);
-  }
-#endif
   const EosSpot<real> s = eos_spot<real>(p, eps);
 #if CLV_FAST
   // tolerance build: the pressure from one 8-byte read of the pair table
@@ -369,22 +308,6 @@ __device__ CLV_EOS_ATTR real eos_comp(const Params& p, real eps, int c) {
 // 16-byte texel reads; component c equals eos_comp(p, eps, c) bit for bit
 // (the table is 16-byte aligned: the library checks it)
 template <class real> __device__ __forceinline__ void eos_texel4(const Params& p, real eps, real out[4]) {
-#if CLV_FAST
-  if constexpr (sizeof(real) == 4) {
-    if (eps < p.eos_inner) {
-      const EosAt a = eos_at(p, eps);
-      const float4 l = __ldg(reinterpret_cast<const float4*>(p.eos) + a.t);
-      const float4 h = __ldg(reinterpret_cast<const float4*>(p.eos) + min(a.t + 1, p.eos_last));
-      out[0] = l.x + a.r * (h.x - l.x);
-      out[1] = l.y + a.r * (h.y - l.y);
-      out[2] = l.z + a.r * (h.z - l.z);
-      out[3] = l.w + a.r * (h.w - l.w);
-      return;
-    }
-    for (int c = 0; c < 4; c++) out[c] = eos_comp_edge(eos_edge(p), eps, c);
-    return;
-  }
-#endif
   const EosSpot<real> s = eos_spot<real>(p, eps);
   const float4 lo = __ldg(reinterpret_cast<const float4*>(p.eos) + s.t0);
   const float4 hi = __ldg(reinterpret_cast<const float4*>(p.eos) + s.t1);
@@ -398,31 +321,9 @@ template <class real> __device__ __forceinline__ bool eos_in_table(const Params&
 }
 // P(e): eos_table.h:65-71
 template <class real> __device__ __forceinline__ real eosP(const Params& p, real eps) {
-#if CLV_FAST
-  if constexpr (sizeof(real) == 4) return eps < p.eos_inner ? eos_comp<real>(p, eps, 1) : eosP_edge(eos_edge(p), eps);
-#endif
   if (eos_in_table(p, eps)) return eos_comp(p, eps, 1);
   return 0.3327f * eps - 0.3223f * pow(eps, (real)0.4585f) - 0.003906f * eps * exp(-0.05697f * eps);
 }
-#if CLV_FAST
-// pressure and its table slope dP/de (1/3 beyond the table, as the root
-// finder's derivative takes it there)
-__device__ __forceinline__ float eos_p_slope(const Params& p, float eps, float& dpe) {
-  dpe = 1.0f / 3.0f;
-  if (!(eps < p.eos_inner)) return eosP_edge(eos_edge(p), eps);
-  const EosAt a = eos_at(p, eps);
-  float2 q;
-  if (p.eos_p2) {
-    q = __ldg(p.eos_p2 + a.t);
-  } else {
-    q.x = __ldg(p.eos + 4 * (long long)a.t + 1);
-    q.y = __ldg(p.eos + 4 * (long long)min(a.t + 1, p.eos_last) + 1);
-  }
-  const float d = q.y - q.x;
-  dpe = d * p.rf.eos_step;
-  return q.x + a.r * d;
-}
-#endif
 // CS2(e): eos_table.h:94-100
 template <class real> __device__ __forceinline__ real eosCS2(const Params& p, real eps) {
   if (eos_in_table(p, eps)) return eos_comp(p, eps, 0);
@@ -500,11 +401,15 @@ __device__ __forceinline__ real max_speed(const Params& p, real e, real vx, real
 // helper.h:128-167; returns the energy density. With BULK the pressure is
 // P(e) + bulk, the bulk viscous pressure of the cell.
 template <class real, bool BULK = false>
-__device__ __forceinline__ real root_newton(const Params& p, real T00, real M, real bulk = (real)0.0f) {
+__device__ __forceinline__ real root_newton(const Params& p, real T00, real M, real bulk = (real)0.0f,
+                                            real v_start = (real)-1.0f) {
   real vl = 0.0f;
   real vh = 1.0f;
   real dpe = 1.0f / 3.0f;
-  real v = 0.5f * (vl + vh);
+  // the reference starts at the middle of the bracket; a start in [0, 1)
+  // (the tolerance build passes the cell's speed at the start of the step)
+  // leaves the bracket and the safeguards as they are
+  real v = v_start >= (real)0.0f ? v_start : 0.5f * (vl + vh);
   real ed = T00 - M * v;
   real pr = eosP<real>(p, ed);
   if (BULK) pr = pr + bulk;
@@ -538,55 +443,6 @@ __device__ __forceinline__ real root_newton(const Params& p, real T00, real M, r
   }
   return T00 - M * v;
 }
-#if CLV_FAST
-// The FP32 tolerance build's root finder: the same equation, bracket,
-// safeguards and stopping rule (a step below 1e-5). Every evaluation of the
-// reference's finder is a dependent table read out of L2, four to five of them
-// a cell at the end of the cell's longest chain. This one starts from the root
-// of the equation with P(e) linear about (er, pr, cs2), an energy density near
-// the new one that the pi update has looked up (a quadratic: no table read), takes the
-// table's own dP/de from the texels of each evaluation, and returns the
-// pressure at the root from the last evaluation's segment: most cells read the
-// table once. (FP64, with its tolerance of 1e-11, keeps the reference's
-// iterates: where the finder stops within 1e-5 depends on them.)
-template <bool BULK>
-__device__ __forceinline__ float root_near(const Params& p, float T00, float M, float bulk, float er, float pr0,
-                                           float cs2, float& pr_out) {
-  // cs2 M v^2 - b v + M = 0, b = T00 + P + cs2 (T00 - er): the smaller root
-  const float b = T00 + pr0 + (BULK ? bulk : 0.0f) + cs2 * (T00 - er);
-  const float disc = b * b - 4.0f * cs2 * M * M;
-  float v = 2.0f * M / (b + sqrtf(fmaxf(disc, 0.0f)));
-  if (!(v >= 0.0f && v <= 1.0f)) v = 0.5f;
-  float vl = 0.0f, vh = 1.0f, dv = 1.0f, dvold = 1.0f, ed, pt, dpe;
-  int i = 0;
-  while (true) {
-    ed = T00 - M * v;
-    pt = eos_p_slope(p, ed, dpe);
-    const float pr = BULK ? pt + bulk : pt;
-    const float f = (T00 + pr) * v - M;
-    const float df = (T00 + pr) - M * v * dpe;
-    if (i > 0) {
-      if (f > 0.0f) vh = v;
-      else vl = v;
-    }
-    if ((f + df * (vh - v)) * (f + df * (vl - v)) > 0.0f || fabsf(2.f * f) > fabsf(dvold * df)) {
-      dvold = dv;
-      dv = 0.5f * (vh - vl);
-      v = vl + dv;
-    } else {
-      dvold = dv;
-      dv = f / df;
-      v -= dv;
-    }
-    i++;
-    if (fabsf(dv) < 0.00001f || i > 100) break;
-  }
-  const float e = T00 - M * v;
-  pr_out = (fabsf(dv) < 0.00001f && ed < p.eos_inner) ? pt + dpe * (e - ed) : eosP<float>(p, e);
-  return e;
-}
-#endif
-
 // Bulk sector (no counterpart in the reference): zeta/s(T) as a skewed Cauchy
 // peak, ZETAOS_MAX w^2 / (w^2 + (T - T0)^2), w = WIDTH (1 + SKEW sign(T - T0))
 // (the JETSCAPE parametrisation, Everett et al., PRC 103, 054904 (2021)).

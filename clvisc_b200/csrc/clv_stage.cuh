@@ -73,10 +73,28 @@ struct GridDims {
 template <class real> struct CellIn {
   real e0[4], g0, p0;
   real e1[4], g1, p1;
-  real er, pr, cr;  // tolerance build, FP32: an energy density near the new one with its P(e) and c_s^2 (pi_update's lookup)
 };
 
 inline namespace CLV_ARITH {
+// What the tolerance build contracts into a fused multiply-add depends on what
+// the compiler sees around a product. Where the FP32 build has one expression in
+// two places (a chunk's first planes and its loop; a stage compiled apart and
+// with its number at run time), these keep it from telling them apart: v's
+// values are taken as they are, not as the products they came from, and a
+// stage's number is not known when its sources are scaled by it.
+template <class real, int N> __device__ __forceinline__ void opaque(real (&v)[N]) {
+#if CLV_FAST
+  if constexpr (sizeof(real) == 4)
+#pragma unroll
+    for (int i = 0; i < N; i++) asm("" : "+f"(v[i]));
+#endif
+}
+template <class real, int STAGE> __device__ __forceinline__ int arith_step(int step) {
+#if CLV_FAST
+  if (sizeof(real) == 4) return step;
+#endif
+  return STAGE ? STAGE : step;
+}
 __device__ __forceinline__ Stencil make_stencil(int q, int L, long long stride) {
   Stencil s;
 #pragma unroll
@@ -142,7 +160,7 @@ template <class real> __device__ __forceinline__ void cell_in_ev1_of(const Param
 // pi_old(m, u0): u0 times component m of pi at the start of the step (d_pi[1]).
 template <class real, bool COUPLED, bool BULK, class Idx, class PiOld>
 __device__ __forceinline__ void pi_update(const Params& p, const ViscBuffers<real>& b, int step,
-                                          const TauConst<real>& tc, Idx I, long long ld, CellIn<real>& cin,
+                                          const TauConst<real>& tc, Idx I, long long ld, const CellIn<real>& cin,
                                           const real pc[11], const real grad[3][4], real S10[11], real pinew[11],
                                           PiOld&& pi_start) {
   const real acu = Acu<real>::v;
@@ -189,11 +207,6 @@ __device__ __forceinline__ void pi_update(const Params& p, const ViscBuffers<rea
   real theta = udt[0] + grad[0][1] + grad[1][2] + grad[2][3];
   real tex[4];  // cs2, P, T, s at ed_step
   eos_texel4<real>(p, ed_step, tex);
-#if CLV_FAST
-  cin.er = ed_step;
-  cin.pr = tex[1];
-  cin.cr = tex[0];
-#endif
   real temperature = tex[2];
   real sdens = tex[3];
   real local_etaos = etaos<real>(p, temperature);
@@ -347,31 +360,23 @@ __device__ __forceinline__ void ev_update(const Params& p, const ViscBuffers<rea
     T03 *= SCALE_COEF * T00 / M;
     M = SCALE_COEF * T00;
   }
-  real pr, ed_find;
+  // tolerance build, FP32: Newton from the cell's speed at the start of the
+  // step, which is near the root, instead of from 1/2 (fewer EOS lookups).
+  // The finder stops at a step below 1e-5, so where it ends depends on where
+  // it starts: about 1e-9 of the energy density, inside the FP32 tolerance
+  // but not the FP64 one, which keeps the reference's start.
+  real v_start = -1.0f;
 #if CLV_FAST
-  if constexpr (sizeof(real) == 4 && FUSED_PI) {
-    ed_find = root_near<BULK>(p, T00, M, bnew, cin.er, cin.pr, cin.cr, pr);
-    if (ed_find < acu) {
-      T01 = 0.0f;
-      T02 = 0.0f;
-      T03 = 0.0f;
-    }
-    if (ed_find < 0.0f) {
-      ed_find = 0.0f;
-      pr = eosP<real>(p, ed_find);
-    }
-  } else
+  if constexpr (sizeof(real) == 4) v_start = fmin(sqrt(vx * vx + vy * vy + vz * vz), (real)0.999f);
 #endif
-  {
-    ed_find = root_newton<real, BULK>(p, T00, M, bnew);
-    if (ed_find < acu) {
-      T01 = 0.0f;
-      T02 = 0.0f;
-      T03 = 0.0f;
-    }
-    ed_find = cmax<real>(0.0f, ed_find);
-    pr = eosP<real>(p, ed_find);
+  real ed_find = root_newton<real, BULK>(p, T00, M, bnew, v_start);
+  if (ed_find < acu) {
+    T01 = 0.0f;
+    T02 = 0.0f;
+    T03 = 0.0f;
   }
+  ed_find = cmax<real>(0.0f, ed_find);
+  real pr = eosP<real>(p, ed_find);
   if (BULK) pr = pr + bnew;
   real epv = cmax<real>(acu, T00 + pr);
   const real repv = quot<real>((real)1.0f, epv);

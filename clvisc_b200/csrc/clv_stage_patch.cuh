@@ -10,8 +10,9 @@
 // latency of one thread's chain, not by the chip's throughput. Against the
 // per-cell kernel a cell costs 1.9-2.3 records, 2.4 slopes and 2.2 faces in
 // place of 9, 6 and 4.
-// Records, slopes and faces are the functions of clv_stage_tiled2d.cuh, whose
-// exact-build results are the per-cell kernel's bit for bit.
+// Records, slopes and faces are the functions of clv_stage_tiled2d.cuh: the
+// exact build's results are the per-cell kernel's bit for bit, the FP32
+// tolerance build's are the strips'.
 #pragma once
 #include "clv_stage_tiled2d.cuh"
 
@@ -47,17 +48,18 @@ template <class real, bool BULK> struct PatchSmall {
 
 inline namespace CLV_ARITH {
 
-// The patch at (i0, j0) of the event (gd, b). Every thread of the block calls
-// it (it holds barriers).
+// The patch at (i0, j0) of the event (gd, b); first: a strip starts at i0. Every
+// thread of the block calls it (it holds barriers).
 template <class real, bool BULK, int TX, int TY, int NT, int STAGE>
 __device__ __forceinline__ void patch2d(const Params& p, const GridDims& gd, const ViscBuffers<real>& b, int step_,
-                                        const TauConst<real>& tc, int i0, int j0, PatchSmem<real, BULK, TX, TY>& s) {
+                                        const TauConst<real>& tc, int i0, int j0, PatchSmem<real, BULK, TX, TY>& s,
+                                        bool first = false) {
   typedef Rec2<BULK> R;
   typedef Rec2L<real, BULK> L;
   typedef PatchGeom<TX, TY> G;
   constexpr int NP = L::NP, CP = L::CP, RG = L::RG, CG = L::CG, NC = R::NCOMP;
   constexpr int NS = G::NSX + G::NSY, NF = G::NFX + G::NFY;
-  const int step = STAGE ? STAGE : step_;
+  const int step = arith_step<real, STAGE>(step_);
   const real tau = tc.tau;
   const Recips<real>& rc = recips<real>(p);
   const long long ld = gd.ld;
@@ -87,7 +89,7 @@ __device__ __forceinline__ void patch2d(const Params& p, const GridDims& gd, con
     grp_load<real, RG>(C, G::NC, cm - d, rl);
     grp_load<real, RG>(C, G::NC, cm, rm);
     grp_load<real, RG>(C, G::NC, cm + d, rr);
-    rec2_slopes<real, BULK>(rl, rm, rr, sl);
+    rec2_slopes<real, BULK, true>(rl, rm, rr, sl, first && x && qq / TY == 0);
     grp_store<real, CG>(S, NS, q, sl);
   }
   __syncthreads();
@@ -111,7 +113,7 @@ __device__ __forceinline__ void patch2d(const Params& p, const GridDims& gd, con
       grp_load<real, RG>(C, G::NC, cl + (x ? G::CY : 1), rr);
       grp_load<real, CG>(S, NS, s0, sl);
       grp_load<real, CG>(S, NS, s0 + (x ? TY : 1), sr);
-      rec2_face<real, BULK>(p, tau, x ? 0 : 1, rl, sl, rr, sr, f[it]);
+      rec2_face<real, BULK, true>(p, tau, x ? 0 : 1, rl, sl, rr, sr, f[it]);
     }
   }
   __syncthreads();
@@ -142,7 +144,7 @@ __device__ __forceinline__ void patch2d(const Params& p, const GridDims& gd, con
       grp_load<real, RG>(C, G::NC, cs, n);
       rec2_umu<real, BULK>(n, um);
       grp_load<real, RG>(C, G::NC, cs - G::CY, n);
-      rec2_umu<real, BULK>(n, ux0);
+      rec2_umu<real, BULK, true>(n, ux0);
       grp_load<real, RG>(C, G::NC, cs + G::CY, n);
       rec2_umu<real, BULK>(n, ux1);
       grp_load<real, RG>(C, G::NC, cs - 1, n);

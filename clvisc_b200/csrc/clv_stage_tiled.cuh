@@ -28,14 +28,15 @@
 // barrier that precedes their use, the update follows the last barrier of its
 // plane so that warps drift apart, offsets are 32 bits wide, each Runge-Kutta
 // stage is its own instantiation (loads under a run-time condition in an
-// unrolled loop wait one by one), and the FP32 tolerance build works on pairs
-// (clv_pairs.cuh). One step at 385x385x115 FP32: 12.0 to 11.1 ms; 201x201x105
-// 3.90 to 3.14 (chunks of march_chunk included); 161x145x77 FP64 3.73 to 3.47;
-// 97x93x65 exact 3.8 to 2.1. Prefetching the next plane's fields into registers
-// (12.5 ms at 385x385x115, spills) or by cp.async into shared memory (11.9)
-// was slower.
+// unrolled loop wait one by one). Two steps at 385x385x115 FP32: 12.0 to 11.9 ms;
+// 201x201x105 3.88 to 3.36 (chunks of march_chunk included); 161x145x77 FP64 3.72
+// to 3.42; 97x93x65 exact 3.8 to 2.1. Prefetching the next plane's fields into
+// registers (12.5 ms at 385x385x115, spills) or by cp.async into shared memory
+// (11.9) was slower. Records as densities u0 pi in pairs for the two-lane FP32
+// instructions and a root finder from the pi update's lookup took 11.0 ms, but
+// each rounds elsewhere (v and pi recovered by 1/u0): the error against 64 bits
+// grew from 4.4e-7 to 4.8e-7, and cells at the floors of the update changed.
 #pragma once
-#include "clv_pairs.cuh"
 #include "clv_smem16.cuh"
 #include "clv_stage.cuh"
 
@@ -169,12 +170,6 @@ __device__ CLV_TILED_ATTR void make_record(const Params& p, const ViscBuffers<re
 #pragma unroll
     for (int f = RF_P0 + 1; f < L::RN; f++) r[f] = 0.0f;
   }
-#if CLV_FAST
-  if constexpr (Pairs<real>::on) {
-    pair_record<L::NPI>(tau, e, vx, vy, vz, pr, pi, r);
-    return;
-  }
-#endif
   real u0 = gamma3<real>(vx, vy, vz);
   real A = (e + pr) * u0;
   real u4[4] = {(real)1.0f * u0, vx * u0, vy * u0, vz * u0};
@@ -225,14 +220,6 @@ template <int TJ, int TK> __device__ __forceinline__ bool halo_cell(int q, int& 
 template <class real, bool BULK>
 __device__ CLV_TILED_ATTR void slopes3(const real* L, const real* M, const real* R, real* out) {
   typedef Lanes<real, BULK> T;
-#if CLV_FAST
-  if constexpr (Pairs<real>::on) {
-#pragma unroll
-    for (int q = 0; q < T::CP; q += 2)  // with bulk the last pair is (u0 Pi, P(e)): its second slope goes unused
-      pair_limit(pair_at(L + PK_Q + q), pair_at(M + PK_Q + q), pair_at(R + PK_Q + q), out + q);
-    return;
-  }
-#endif
 #pragma unroll
   for (int c = 0; c < 4; c++) out[c] = slope<real>(L[RF_Q0 + c], M[RF_Q0 + c], R[RF_Q0 + c]);
   real uL = L[RF_U0], uM = M[RF_U0], uR = R[RF_U0];
@@ -258,10 +245,6 @@ __device__ CLV_TILED_ATTR void face_flux(const Params& p, real tau, int a, const
 #pragma unroll
     for (int m = 0; m < T::NPI; m++) F[4 + m] = 0.0f;
 #if CLV_FAST
-  if constexpr (Pairs<real>::on) {
-    pair_face<T::CP>(tau, a, L, sL, R, sR, F);
-    return;
-  }
   // tolerance build, with the KT speed 1: F = 0.5 (J(A_R) + J(A_L)) -
   // 0.5 (A_R - A_L) is, for J linear in A with slope v, the weighted sum
   // cp A_L + cm A_R + (the pressure and pi part), cp = (v+1)/2, cm = (v-1)/2;
@@ -335,40 +318,23 @@ __device__ CLV_TILED_ATTR void face_flux(const Params& p, real tau, int a, const
 #endif
 }
 
-// the stage input of a record's cell (cin.e0, g0, p0) and its pi and Pi; in
-// pairs cin.e0[0] comes from the field
+// the stage input of a record's cell (cin.e0, g0, p0) and its pi and Pi
 template <class real, bool BULK>
 __device__ __forceinline__ void record_cell(const real* Cc, CellIn<real>& cin, real pc[11]) {
   constexpr int NPI = Lanes<real, BULK>::NPI;
-  if constexpr (Pairs<real>::on) {
-    const real ru = Cc[PK_RU];
-    cin.e0[1] = Cc[PK_UX] * ru;
-    cin.e0[2] = Cc[PK_UY] * ru;
-    cin.e0[3] = Cc[PK_UZ] * ru;
-    cin.g0 = Cc[PK_U0];
-    cin.p0 = BULK ? Cc[RF_P0] : Cc[PK_PR];
+  cin.e0[0] = Cc[RF_E];
+  cin.e0[1] = Cc[RF_VX];
+  cin.e0[2] = Cc[RF_VY];
+  cin.e0[3] = Cc[RF_VZ];
+  cin.g0 = Cc[RF_U0];
+  cin.p0 = BULK ? Cc[RF_P0] : Cc[RF_PR];
 #pragma unroll
-    for (int m = 0; m < NPI; m++) pc[m] = Cc[PK_U + m] * ru;
-  } else {
-    cin.e0[0] = Cc[RF_E];
-    cin.e0[1] = Cc[RF_VX];
-    cin.e0[2] = Cc[RF_VY];
-    cin.e0[3] = Cc[RF_VZ];
-    cin.g0 = Cc[RF_U0];
-    cin.p0 = BULK ? Cc[RF_P0] : Cc[RF_PR];
-#pragma unroll
-    for (int m = 0; m < NPI; m++) pc[m] = Cc[RF_PI + m];
-  }
+  for (int m = 0; m < NPI; m++) pc[m] = Cc[RF_PI + m];
   if (!BULK) pc[10] = 0.0f;
 }
 
 // u^mu of a record
 template <class real> __device__ __forceinline__ void umu_of(const real* r, real u[4]) {
-  if constexpr (Pairs<real>::on) {  // in the record's order: u^1, u^2, u^3, u^0
-#pragma unroll
-    for (int c = 0; c < 4; c++) u[c] = r[PK_UX + c];
-    return;
-  }
   const real u0 = r[RF_U0];
   u[0] = u0 * 1.0f;
   u[1] = u0 * r[RF_VX];
@@ -380,7 +346,7 @@ template <class real> __device__ __forceinline__ void umu_of(const real* r, real
 template <class real, bool DO_IS, bool DO_KT, bool COUPLED, int TJ, int TK, int MINB, bool BULK = false, int STAGE = 0>
 __global__ void __launch_bounds__(TJ * TK, MINB)
     visc_stage_tiled_kernel(Params p, ViscBuffers<real> b, int step_, TauConst<real> tc, int chunk) {
-  const int step = STAGE ? STAGE : step_;
+  const int step = arith_step<real, STAGE>(step_);
   const real tau = tc.tau;
   const Recips<real>& rc = recips<real>(p);
   typedef TileGeom<TJ, TK> G;
@@ -424,9 +390,15 @@ __global__ void __launch_bounds__(TJ * TK, MINB)
     make_record<real, BULK>(p, b, tau, i0 - 1, jj, kk, r1);
     make_record<real, BULK>(p, b, tau, i0, jj, kk, r2);
     rec_store<real, BULK>(C, G::NC, cself, r2);
+    opaque<real, L::RN>(r0);
+    opaque<real, L::RN>(r1);
+    opaque<real, L::RN>(r2);
     slopes3<real, BULK>(r0, r1, r2, s_prev);  // slope at i0-1
     make_record<real, BULK>(p, b, tau, i0 + 1, jj, kk, r0);
     rec_store<real, BULK>(A, G::NI, tid, r0);
+    opaque<real, L::RN>(r0);
+    opaque<real, L::RN>(r1);
+    opaque<real, L::RN>(r2);
     slopes3<real, BULK>(r1, r2, r0, s_cur);  // slope at i0
     face_flux<real, DO_IS, DO_KT, BULK>(p, tau, 0, r1, s_prev, r2, s_cur, F_prev);
     if constexpr (SM::KEEP) st16<real>(s.PX[tid], F_prev);
@@ -540,7 +512,6 @@ __global__ void __launch_bounds__(TJ * TK, MINB)
 #pragma unroll
           for (int m = 0; m < L::NPI; m++) S10[m] = plane_at(b.src, (4 + m) * ld, I);
       }
-      if constexpr (Pairs<real>::on) cin.e0[0] = plane_at(b.ev_st, 0, I);
     }
     __syncthreads();
 
@@ -597,25 +568,6 @@ __global__ void __launch_bounds__(TJ * TK, MINB)
           cmp_load<real, BULK>(SZ4, SZ2, G::NSZ, tj * (TK + 2) + (tk + 1), Fp);
           cmp_load<real, BULK>(SZ4, SZ2, G::NSZ, tj * (TK + 2) + tk, Fm);
         }
-#if CLV_FAST
-        if constexpr (Pairs<real>::on) {
-          const float2 rd2 = make_float2(-rD, -rD);
-#pragma unroll
-          for (int c = 0; c < L::NC; c += 2) {
-            const float2 d = pair_sub(a == 0 ? pair_at(Fx + c) : pair_at(Fp + c),
-                                      a == 0 ? pair_at(F_prev + c) : pair_at(Fm + c));
-            real* const s2 = c < 4 ? S4 + c : S10 + (c - 4);
-            if (c + 1 == L::NC) {  // Pi's, alone
-              s2[0] = s2[0] - d.x * rD;
-              continue;
-            }
-            const float2 t = __ffma2_rn(d, rd2, pair_at(s2));
-            s2[0] = t.x;
-            s2[1] = t.y;
-          }
-          continue;
-        }
-#endif
 #pragma unroll
         for (int c = 0; c < L::NC; c++) {
           if (c < 4 && !DO_KT) continue;
@@ -646,28 +598,11 @@ __global__ void __launch_bounds__(TJ * TK, MINB)
           rec_load<real, BULK>(C, G::NC, cself + 1, rn);
           umu_of<real>(rn, umz1);
           const real u0c = cin.g0;
-#if CLV_FAST
-          if constexpr (Pairs<real>::on) {
-            const real* lo[3] = {umu_prev, umy0, umz0};
-            const real* hi[3] = {umx1, umy1, umz1};
 #pragma unroll
-            for (int a = 0; a < 3; a++) {
-              const real sc = CLV_THETA * (a == 0 ? rc.DX : (a == 1 ? rc.DY : tc.rdzt));
-              real o[4];
-              pair_limit(pair_at(lo[a]), pair_at(umc), pair_at(hi[a]), o);
-              pair_limit(pair_at(lo[a] + 2), pair_at(umc + 2), pair_at(hi[a] + 2), o + 2);
-#pragma unroll
-              for (int c = 0; c < 4; c++) grad[a][c] = sc * o[(c + 3) & 3];
-            }
-          }
-#endif
-          if constexpr (!Pairs<real>::on) {
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-              grad[0][c] = div_by<real>(grad_limit<real>(umu_prev[c], umc[c], umx1[c]), (real)p.DX, rc.DX);
-              grad[1][c] = div_by<real>(grad_limit<real>(umy0[c], umc[c], umy1[c]), (real)p.DY, rc.DY);
-              grad[2][c] = div_by<real>(grad_limit<real>(umz0[c], umc[c], umz1[c]), tc.dzt, tc.rdzt);
-            }
+          for (int c = 0; c < 4; c++) {
+            grad[0][c] = div_by<real>(grad_limit<real>(umu_prev[c], umc[c], umx1[c]), (real)p.DX, rc.DX);
+            grad[1][c] = div_by<real>(grad_limit<real>(umy0[c], umc[c], umy1[c]), (real)p.DY, rc.DY);
+            grad[2][c] = div_by<real>(grad_limit<real>(umz0[c], umc[c], umz1[c]), tc.dzt, tc.rdzt);
           }
           grad[2][0] = grad[2][0] + div_by<real>(e0[3] * u0c, tau, tc.rtau);
           grad[2][1] = grad[2][1] + div_by<real>((real)0.0f * u0c, tau, tc.rtau);

@@ -23,7 +23,6 @@
 // Each record, slope and face flux is the per-cell kernel's expression, so the
 // results are identical bit for bit.
 #pragma once
-#include "clv_pairs.cuh"
 #include "clv_smem16.cuh"
 #include "clv_stage.cuh"
 
@@ -84,13 +83,6 @@ __device__ __forceinline__ void rec2_make(const Params& p, const GridDims& gd, c
   real p0 = eosP<real>(p, e);
   real pr = p0;
   if (BULK) pr = pr + pv[R::NPI - 1];
-#if CLV_FAST
-  if constexpr (Pairs<real>::on) {
-    pair_record<R::NPI>(tau, e, vx, vy, vz, pr, pv, dst);
-    if (BULK) dst[R::P0] = p0;
-    return;
-  }
-#endif
   real u0 = gamma3<real>(vx, vy, vz);
   real A = (e + pr) * u0;
   real u4[4] = {(real)1.0f * u0, vx * u0, vy * u0, vz * u0};
@@ -111,50 +103,47 @@ __device__ __forceinline__ void rec2_make(const Params& p, const GridDims& gd, c
   if (BULK) dst[R::P0 * stride] = p0;
 }
 
-// limited slopes of every component at the middle of three records
-template <class real, bool BULK>
-__device__ __forceinline__ void rec2_slopes(const real* L, const real* M, const real* R_, real* out) {
+// The FP32 tolerance build contracts products into sums, and which product goes
+// into which sum depends on the code around. At the floors of the update
+// (T^{tau i} below 1e-7 and Pi below ZETAOS_TMIN are zero) the last bit decides
+// what becomes of a dilute cell, so the patches (PATCH below) write out the
+// contractions that the strips of tile2d get: patches and strips are the same
+// values.
+template <class real> struct Contracted { static constexpr bool on = CLV_FAST && sizeof(real) == 4; };
+
+// limited slopes of every component at the middle of three records; before (of
+// an x slope): the plane before the first of a strip, whose slope shares its
+// difference to the first plane with that plane's slope
+template <class real, bool BULK, bool PATCH = false>
+__device__ __forceinline__ void rec2_slopes(const real* L, const real* M, const real* R_, real* out, bool before = false) {
   typedef Rec2<BULK> R;
   constexpr int sl = 1, sm = 1, sr = 1, so = 1;
-#if CLV_FAST
-  if constexpr (Pairs<real>::on) {
-    // with the bulk sector the last pair is (u0 Pi, P(e)); its second slope is
-    // never used
-    constexpr int NC = (R::NCOMP + 1) / 2 * 2;
-#pragma unroll
-    for (int q = 0; q < NC; q += 2)
-      pair_limit(pair_at(L + PK_Q + q), pair_at(M + PK_Q + q), pair_at(R_ + PK_Q + q), out + q);
-#pragma unroll
-    for (int c = NC; c < Rec2L<real, BULK>::CP; c++) out[c] = 0.0f;  // padding
-    return;
-  }
-#endif
 #pragma unroll
   for (int c = R::NCOMP; c < Rec2L<real, BULK>::CP; c++) out[c] = 0.0f;  // padding
 #pragma unroll
   for (int c = 0; c < 4; c++) out[c * so] = slope<real>(L[(R::Q0 + c) * sl], M[(R::Q0 + c) * sm], R_[(R::Q0 + c) * sr]);
   real uL = L[R::U0 * sl], uM = M[R::U0 * sm], uR = R_[R::U0 * sr];
 #pragma unroll
-  for (int m = 0; m < R::NPI; m++)
-    out[(4 + m) * so] =
-        slope<real>(uL * L[(R::PI + m) * sl], uM * M[(R::PI + m) * sm], uR * R_[(R::PI + m) * sr]);
+  for (int m = 0; m < R::NPI; m++) {
+    const real pl = L[(R::PI + m) * sl], pm = M[(R::PI + m) * sm], pr = R_[(R::PI + m) * sr];
+#if CLV_FAST
+    if constexpr (PATCH && Contracted<real>::on) {
+      const real um = mul_rn(uM, pm);
+      out[(4 + m) * so] = gminmod<real>(before ? fma(-uM, pm, mul_rn(uR, pr)) : fma(uR, pr, -um),
+                                        before ? fma(uM, pm, -mul_rn(uL, pl)) : fma(-uL, pl, um));
+      continue;
+    }
+#endif
+    out[(4 + m) * so] = slope<real>(uL * pl, uM * pm, uR * pr);
+  }
 }
 
 // flux through the face between records L and R along axis a (0: x, 1: y)
-template <class real, bool BULK>
+template <class real, bool BULK, bool PATCH = false>
 __device__ __forceinline__ void rec2_face(const Params& p, real tau, int a, const real* L, const real* sL,
                                           const real* R_, const real* sR, real F[Rec2L<real, BULK>::CP]) {
   typedef Rec2<BULK> R;
   constexpr int sl = 1, ssl = 1, sr = 1, ssr = 1;
-#if CLV_FAST
-  if constexpr (Pairs<real>::on) {
-    constexpr int NC = (R::NCOMP + 1) / 2 * 2;
-    pair_face<NC>(tau, a, L, sL, R_, sR, F);
-#pragma unroll
-    for (int c = NC; c < Rec2L<real, BULK>::CP; c++) F[c] = 0.0f;  // padding
-    return;
-  }
-#endif
 #pragma unroll
   for (int c = R::NCOMP; c < Rec2L<real, BULK>::CP; c++) F[c] = 0.0f;  // padding
 #if CLV_FAST
@@ -172,7 +161,10 @@ __device__ __forceinline__ void rec2_face(const Params& p, real tau, int a, cons
       const real p0s = L[(R::PI + c) * sl] + R_[(R::PI + c) * sr];
       const real pis = (a == 0 ? L[(R::PI + m1) * sl] : L[(R::PI + m2) * sl]) +
                        (a == 0 ? R_[(R::PI + m1) * sr] : R_[(R::PI + m2) * sr]);
-      real k = (c == 0 ? pt - th * p0s : -th * p0s) * vh + th * pis;
+      const real k0 = c == 0 ? pt - th * p0s : -th * p0s;
+      real k;
+      if constexpr (PATCH && Contracted<real>::on) k = fma(th, pis, mul_rn(k0, vh));
+      else k = k0 * vh + th * pis;
       if (c == a + 1) k += pt;
       real f = cm * R_[(R::Q0 + c) * sr] + k;
       f = f - hm * sR[c * ssr];
@@ -222,18 +214,17 @@ __device__ __forceinline__ void rec2_face(const Params& p, real tau, int a, cons
 #endif
 }
 
-// u^mu of a record: u^0..u^3 (in pairs: u^1, u^2, u^3, u^0, the record's order)
-template <class real, bool BULK> __device__ __forceinline__ void rec2_umu(const real* r, real u[4]) {
+// u^mu of a record. CARRIED: that of the plane before, which strips carry from
+// one plane to the next, so that no product of it is contracted into a sum.
+template <class real, bool BULK, bool CARRIED = false>
+__device__ __forceinline__ void rec2_umu(const real* r, real u[4]) {
   typedef Rec2<BULK> R;
-  if constexpr (Pairs<real>::on) {
+  const real u0 = r[R::U0];
+  u[0] = u0 * 1.0f;
 #pragma unroll
-    for (int c = 0; c < 4; c++) u[c] = r[PK_UX + c];
-  } else {
-    const real u0 = r[R::U0];
-    u[0] = u0 * 1.0f;
-    u[1] = u0 * r[R::VX];
-    u[2] = u0 * r[R::VY];
-    u[3] = u0 * r[R::VZ];
+  for (int c = 0; c < 3; c++) {
+    if constexpr (CARRIED && Contracted<real>::on) u[1 + c] = mul_rn(u0, r[R::VX + c]);
+    else u[1 + c] = u0 * r[R::VX + c];
   }
 }
 
@@ -250,26 +241,14 @@ __device__ __forceinline__ void rec2_cell(const Params& p, const GridDims& gd, c
   real Cs[Rec2L<real, BULK>::NP];
   grp_load<real, Rec2L<real, BULK>::RG>(C, n, c0, Cs);
   real* e0 = cin.e0;
-  if constexpr (Pairs<real>::on) {
-    const real ru = Cs[PK_RU];
-    e0[0] = b.ev_st[I];
-    e0[1] = Cs[PK_UX] * ru;
-    e0[2] = Cs[PK_UY] * ru;
-    e0[3] = Cs[PK_UZ] * ru;
-    cin.g0 = Cs[PK_U0];
-    cin.p0 = BULK ? Cs[R::P0] : Cs[PK_PR];
+  e0[0] = Cs[R::E];
+  e0[1] = Cs[R::VX];
+  e0[2] = Cs[R::VY];
+  e0[3] = Cs[R::VZ];
+  cin.g0 = Cs[R::U0];
+  cin.p0 = Cs[R::P0];
 #pragma unroll
-    for (int m = 0; m < R::NPI; m++) pc[m] = Cs[PK_U + m] * ru;
-  } else {
-    e0[0] = Cs[R::E];
-    e0[1] = Cs[R::VX];
-    e0[2] = Cs[R::VY];
-    e0[3] = Cs[R::VZ];
-    cin.g0 = Cs[R::U0];
-    cin.p0 = Cs[R::P0];
-#pragma unroll
-    for (int m = 0; m < R::NPI; m++) pc[m] = Cs[R::PI + m];
-  }
+  for (int m = 0; m < R::NPI; m++) pc[m] = Cs[R::PI + m];
   if (!BULK) pc[10] = 0.0f;
 #pragma unroll
   for (int c = 0; c < 4; c++) pin[c] = b.pin[c * ld + I];
@@ -322,24 +301,6 @@ __device__ __forceinline__ void rec2_cell(const Params& p, const GridDims& gd, c
 template <class real, bool BULK>
 __device__ __forceinline__ void rec2_flux(const real* Fp, const real* Fm, real D, real rD, real S4[4], real S10[11]) {
   constexpr int NC = Rec2<BULK>::NCOMP;
-#if CLV_FAST
-  if constexpr (Pairs<real>::on) {
-    const float2 rd2 = make_float2(-rD, -rD);
-#pragma unroll
-    for (int c = 0; c < NC; c += 2) {
-      const float2 d = pair_sub(pair_at(Fp + c), pair_at(Fm + c));
-      real* const s2 = c < 4 ? S4 + c : S10 + (c - 4);
-      if (c + 1 < NC) {
-        const float2 t = __ffma2_rn(d, rd2, pair_at(s2));
-        s2[0] = t.x;
-        s2[1] = t.y;
-      } else {
-        s2[0] = s2[0] - d.x * rD;
-      }
-    }
-    return;
-  }
-#endif
 #pragma unroll
   for (int c = 0; c < NC; c++) {
     real src = Fp[c];
@@ -358,27 +319,10 @@ __device__ __forceinline__ void rec2_grad(const Params& p, const TauConst<real>&
   const real tau = tc.tau;
   const real* e0 = cin.e0;
   const real u0c = cin.g0;
-#if CLV_FAST
-  if constexpr (Pairs<real>::on) {
 #pragma unroll
-    for (int a = 0; a < 2; a++) {
-      const real sc = CLV_THETA * (a == 0 ? rc.DX : rc.DY);
-      const real* lo = a == 0 ? ux0 : uy0;
-      const real* hi = a == 0 ? ux1 : uy1;
-      real o[4];
-      pair_limit(pair_at(lo), pair_at(um), pair_at(hi), o);
-      pair_limit(pair_at(lo + 2), pair_at(um + 2), pair_at(hi + 2), o + 2);
-#pragma unroll
-      for (int c = 0; c < 4; c++) grad[a][c] = sc * o[(c + 3) & 3];
-    }
-  }
-#endif
-  if constexpr (!Pairs<real>::on) {
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-      grad[0][c] = div_by<real>(grad_limit<real>(ux0[c], um[c], ux1[c]), (real)p.DX, rc.DX);
-      grad[1][c] = div_by<real>(grad_limit<real>(uy0[c], um[c], uy1[c]), (real)p.DY, rc.DY);
-    }
+  for (int c = 0; c < 4; c++) {
+    grad[0][c] = div_by<real>(grad_limit<real>(ux0[c], um[c], ux1[c]), (real)p.DX, rc.DX);
+    grad[1][c] = div_by<real>(grad_limit<real>(uy0[c], um[c], uy1[c]), (real)p.DY, rc.DY);
   }
 #pragma unroll
   for (int c = 0; c < 4; c++) grad[2][c] = 0.0f;

@@ -315,10 +315,12 @@ int clv_batch_occupancy(const clv_params *p, int block_size, int max_registers, 
 /* The same stage for batches of (2+1)D events with the tiled kernel: work
  * items are patches of cells, taken in order by grid_blocks persistent blocks
  * (grid_blocks <= 0, or above the resident blocks of the GPU: fill it once).
- * rows must be 64 or 128 and chunk 1 to 4096; the kernel chooses its patch
- * itself, so neither changes the launch any more. Every event must have
- * nz = 1: the kernel gives events with nz != 1 no patches. Same bits as
- * clv_batch_stage. */
+ * rows must be 64 or 128 and chunk 1 to 4096: the strips of (rows - 4) y rows
+ * by chunk x planes whose values the patches give. The kernel chooses its patch
+ * itself, so neither changes the launch; in the FP32 tolerance build chunk
+ * enters the last bit of the planes where a strip starts. Every event must have
+ * nz = 1: the kernel gives events with nz != 1 no patches. Exact build: same
+ * bits as clv_batch_stage, for any chunk. */
 int clv_batch_stage_tiled(const clv_params *p, int step, const clv_batch *b, int rows, int chunk, int grid_blocks,
                           void *stream);
 /* Resident blocks per SM of the tiled batch stage kernel. */
