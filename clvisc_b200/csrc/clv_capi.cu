@@ -76,7 +76,7 @@ int to_params(const clv_params* in, clv::Params* out) {
   p.eos_num = in->eos_num_ed; p.eos_nrow = in->eos_nrow; p.eos_ncol = in->eos_ncol;
   p.eos_last = (int)std::min((long long)in->eos_nrow * in->eos_ncol, 1ll << 30) - 1;
   p.eos_top = in->eos_ed_start + in->eos_num_ed * in->eos_ed_step;
-  p.eos_inner = std::min(p.eos_top, in->eos_ed_start + (float)p.eos_last * in->eos_ed_step);
+  p.eos_inner = in->eos_ed_start == 0.0f ? std::min(p.eos_top, (float)(p.eos_last - 1) * in->eos_ed_step) : -1.0f;
   p.eos = in->eos_table;
   p.eos_p2 = reinterpret_cast<const float2*>(in->eos_p2);
   if (in->eos_p2 && (reinterpret_cast<uintptr_t>(in->eos_p2) % 8))

@@ -51,7 +51,7 @@ struct Params {
   int eos_num, eos_nrow, eos_ncol;
   int eos_last;    // nrow*ncol - 1, the last texel
   float eos_top;   // start + num*step as the kernels form it: the table's end
-  float eos_inner; // start + (last texel)*step: below it a lookup's two texels are neighbours
+  float eos_inner; // energy density of the last texel but one, below which a lookup's two texels are neighbours; -1 unless start is 0
   const float* eos;  // nrow*ncol texels of (cs2, p, T, s)
   const float2* eos_p2;  // optional: pairs (p[t], p[t+1]) of the pressure column (tolerance build)
   int flags;
@@ -213,11 +213,10 @@ __device__ __forceinline__ double fast_rsqrt(double a) {
   return fma(0.5 * x, fma(-a * x, x, 1.0), x);
 }
 __device__ __forceinline__ float fast_rsqrt(float a) { return rsqrt(a); }
-// the integer below x (as an int and as a double) for |x| < 2^31, by adding
-// 3 * 2^51 to x - 1/2: no conversion instructions. At an integer x either
-// neighbour may come out, where a piecewise linear function has one value.
+// the integer at or below x (as an int and as a double) for |x| < 2^31, by
+// adding 3 * 2^51 rounded down: no conversion instructions
 __device__ __forceinline__ double fast_floor(double x, int& i) {
-  const double t = (x - 0.5) + 6755399441055744.0;
+  const double t = __dadd_rd(x, 6755399441055744.0);
   i = __double2loint(t);
   return t - 6755399441055744.0;
 }
@@ -253,10 +252,12 @@ template <class real> __device__ __forceinline__ EosSpot<real> eos_spot(const Pa
   if constexpr (sizeof(real) == 8) {
     // the same row, column and weight, the reference's float roundings of the
     // row width and of col * step included, from two additions each in place of
-    // the double conversions; inside the table t1 is the texel after t0 (the
+    // the double conversions. Tables that start at zero and energies from zero
+    // (eos_inner is negative for other tables), where rounding down is the
+    // reference's truncation; inside the table t1 is the texel after t0 (the
     // last column's next is the next row's first), except where the rounded row
     // width leaves a column beyond the last, which reads the last twice
-    if (eps < p.eos_inner) {
+    if (eps >= 0.0 && eps < p.eos_inner) {
       int row, col;
       const double rowd = fast_floor(eps * rc.eos_epr, row);
       const double x = eps - p.eos_start - rowd * ed_per_row;
