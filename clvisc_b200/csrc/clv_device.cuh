@@ -193,26 +193,6 @@ template <class real> __device__ __forceinline__ real div_step(real x, int step)
 }
 
 #if CLV_FAST
-// FP64 quotient, reciprocal square root and square root of the tolerance
-// build: the hardware's approximation (20 bits or more) and two Newton-Raphson
-// steps, x <- x + x (1 - b x) and x <- x + x (1 - a x^2) / 2, each doubling the
-// correct bits (about 1e-16 of the result; the tolerance is 1e-11), without
-// the branches of the library's correctly rounded forms. Arguments are
-// normal numbers away from the range's ends: energy densities, velocities and
-// their sums, floored where they can vanish.
-__device__ __forceinline__ double fast_rcp(double b) {
-  double x;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(b));
-  x = fma(x, fma(-b, x, 1.0), x);
-  return fma(x, fma(-b, x, 1.0), x);
-}
-__device__ __forceinline__ double fast_rsqrt(double a) {
-  double x;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
-  x = fma(0.5 * x, fma(-a * x, x, 1.0), x);
-  return fma(0.5 * x, fma(-a * x, x, 1.0), x);
-}
-__device__ __forceinline__ float fast_rsqrt(float a) { return rsqrt(a); }
 // the integer at or below x (as an int and as a double) for |x| < 2^31, by
 // adding 3 * 2^51 rounded down: no conversion instructions
 __device__ __forceinline__ double fast_floor(double x, int& i) {
@@ -224,14 +204,6 @@ __device__ __forceinline__ double fast_floor(double x, int& i) {
 // a product that is never contracted into a sum
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-// quotient and reciprocal of per-cell values
-template <class real> __device__ __forceinline__ real quot(real a, real b) {
-#if CLV_FAST
-  if constexpr (sizeof(real) == 8) return a * fast_rcp(b);
-#endif
-  return a / b;
-}
-
 // ------------------------------------------------------------------ EOS
 // Table lookup of eos_table.h:39-62: row/col from the energy density, two
 // nearest texels (the second wraps to the next row), clamp-to-edge, lerp.
@@ -334,7 +306,7 @@ template <class real> __device__ __forceinline__ real eosCS2(const Params& p, re
 // ---------------------------------------------------------------- helper.h
 template <class real> __device__ __forceinline__ real gamma3(real vx, real vy, real vz) {  // helper.h:46-48
 #if CLV_FAST
-  return fast_rsqrt(cmax<real>(1.0f - vx * vx - vy * vy - vz * vz, Acu<real>::v));
+  return rsqrt(cmax<real>(1.0f - vx * vx - vy * vy - vz * vz, Acu<real>::v));
 #else
   return 1.0f / sqrt(cmax<real>(1.0f - vx * vx - vy * vy - vz * vz, Acu<real>::v));
 #endif
@@ -426,7 +398,7 @@ __device__ __forceinline__ real root_newton(const Params& p, real T00, real M, r
       v = vl + dv;
     } else {
       dvold = dv;
-      dv = quot<real>(f, df);
+      dv = f / df;
       v -= dv;
     }
     i++;

@@ -226,7 +226,7 @@ __device__ __forceinline__ void pi_update(const Params& p, const ViscBuffers<rea
 
   // the implicit update's denominator, shared by the ten components
   const real den = u_new[0] + p.DT * one_over_taupi;
-  const real rden = quot<real>((real)1.0f, den);
+  const real rden = (real)1.0f / den;
   real max_pimn_abs = 0.0f;
 #if CLV_FAST
   // tolerance build: the transversality terms of every component,
@@ -379,7 +379,7 @@ __device__ __forceinline__ void ev_update(const Params& p, const ViscBuffers<rea
   real pr = eosP<real>(p, ed_find);
   if (BULK) pr = pr + bnew;
   real epv = cmax<real>(acu, T00 + pr);
-  const real repv = quot<real>((real)1.0f, epv);
+  const real repv = (real)1.0f / epv;
   real en[4] = {ed_find, div_by<real>(T01, epv, repv), div_by<real>(T02, epv, repv), div_by<real>(T03, epv, repv)};
 #pragma unroll
   for (int c = 0; c < 4; c++) plane_at(b.evnew, c * ld, I) = en[c];

@@ -30,7 +30,7 @@
 // stage is its own instantiation (loads under a run-time condition in an
 // unrolled loop wait one by one). Two steps at 385x385x115 FP32: 12.0 to 11.8 ms;
 // 201x201x105 3.88 to 3.34 (chunks of march_chunk included); 161x145x77 FP64 3.73
-// to 3.45; 97x93x65 exact 3.8 to 2.1. Prefetching the next plane's fields into
+// to 3.58; 97x93x65 exact 3.8 to 2.1. Prefetching the next plane's fields into
 // registers (12.5 ms at 385x385x115, spills) or by cp.async into shared memory
 // (11.9) was slower. Records as densities u0 pi in pairs for the two-lane FP32
 // instructions and a root finder from the pi update's lookup took 11.0 ms, but
