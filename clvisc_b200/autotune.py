@@ -1,9 +1,14 @@
 """Autotuner of the fused viscous stage's launch shape for one event.
 
-The tiled stage kernel takes its (y, eta) tile from a compile-time set
-(8 x 32, 16 x 16 or 8 x 16, CLV_OPT_TILE) and its x extent per block at run time
-(CLV_OPT_CHUNK); the per-cell kernel is the alternative on any grid. Every
-variant computes the same bits (in either arithmetic). tune_visc() times each
+The first candidate is the library's own choice (kernel 0, chunk 0): patches on
+(2+1)D grids, tiles with the x planes per block chosen from the grid where eta
+has 24 cells or more, one thread per cell between. The others: the tiled kernel's
+(y, eta) tiles from its compile-time set (8 x 32, 16 x 16, 8 x 16, CLV_OPT_TILE)
+and x extents per block (CLV_OPT_CHUNK), the marching (2+1)D kernel, and one
+thread per cell. In the exact build every variant computes the same bits; in the
+tolerance build the variants differ within its tolerance (1e-5 FP32, 1e-11 FP64),
+so there the choice, which hangs on timings, enters the last bits of a run.
+tune_visc() times each
 candidate for a few fused steps on the run's own state, saved before and
 restored after each, and leaves the fastest selected for that run only: the
 choice goes into the run's own clv_params (opt_* fields), so other CLVisc
@@ -31,14 +36,16 @@ def _apply(v, c):
 
 def candidates(nz, use_float32=True, fast=False):
     """(kernel, tile, chunk, blocks) choices worth timing on a grid with nz
-    cells along eta (the 16 x 32 tile exists in the FP32 tolerance build)."""
-    out = [dict(DEFAULTS, kernel=1)]
-    blocks = (2, 1) if use_float32 else (1,)
+    cells along eta (the 16 x 32 tile exists in the FP32 tolerance build); chunk
+    0 leaves the x planes per block to the library."""
+    out = [dict(DEFAULTS, chunk=0), dict(DEFAULTS, kernel=1)]
+    if nz == 1:
+        return out + [dict(DEFAULTS, kernel=3)]
     tiles = (0, 1, 2, 3) if (fast and use_float32) else (0, 1, 2)
+    blocks = 2 if use_float32 else 1
     for tile in tiles:
-        for chunk in (16, 24, 32, 48):
-            for b in blocks[:1]:
-                out.append({'kernel': 2, 'tile': tile, 'chunk': chunk, 'blocks': b})
+        for chunk in (0, 5, 8, 12, 16, 24, 32, 48):
+            out.append({'kernel': 2, 'tile': tile, 'chunk': chunk, 'blocks': blocks})
     if use_float32:
         out.append({'kernel': 2, 'tile': 0, 'chunk': 32, 'blocks': 1})
     return out
