@@ -21,8 +21,10 @@ replays it until every event has stopped.
 
 The stage kernel is either one thread per cell for any grids
 (clv_batch_stage) or, for batches of (2+1)D events, the tiled kernel
-(clv_batch_stage_tiled: patches of cells, of the kernel's own size); both give
-the same bits. autotune() times both families over their launch shapes.
+(clv_batch_stage_tiled: patches of cells, of the kernel's own size). In the exact
+build both give the same bits, in the tolerance build the same values within its
+tolerance (1e-5 FP32, 1e-11 FP64). autotune() times both families over their
+launch shapes; its choice, which hangs on timings, enters the last bits there.
 
 Only the viscous path is batched (no Gubser, coupling or Riemann test flags);
 freeze-out surfaces are not extracted.
@@ -270,7 +272,7 @@ class CLViscBatch(object):
         return n.value
 
     def tiles(self, rows, chunk):
-        """Work items of the tiled kernel at a (rows, chunk) shape."""
+        """Strips of (rows - 4) x chunk cells of the batch, the unit of a tiled launch shape's grid."""
         ti = rows - 4
         return sum(((ny + ti - 1) // ti) * ((nx + chunk - 1) // chunk) for nx, ny, _ in self.grids)
 
@@ -408,9 +410,10 @@ class CLViscBatch(object):
         """Launch shapes autotune() times. One thread per cell: every block
         size with persistent grids of 1..occupancy blocks per SM and the
         one-cell-per-thread grid, without and (FP32) with a 128-register cap
-        (and a 168-register cap below 256 threads). Tiled ((2+1)D batches only): rows x chunks, each with the grid
-        that fills the GPU once and the one-tile-per-block grid (the kernel chooses its patch itself, and a grid
-        above one resident wave counts as one)."""
+        (and a 168-register cap below 256 threads). Tiled ((2+1)D batches
+        only): one shape, that fills the GPU once (the kernel's patches do not
+        depend on rows and chunk; 16 planes a strip where chunks has it, else
+        its first)."""
         sms = torch.cuda.get_device_properties(self.device).multi_processor_count
         out = []
         total = sum(self.sizes)
@@ -423,11 +426,8 @@ class CLViscBatch(object):
                 for grid in sorted({sms * k for k in range(1, occ + 1)} | {(total + bs - 1) // bs}):
                     out.append(('cell', bs, grid, regs))
         if self.all_2d:
-            for r in rows:
-                fill = sms * max(1, self.occupancy_tiled(r))
-                for ch in chunks:
-                    for grid in sorted({fill, self.tiles(r, ch)}):
-                        out.append(('tile', r, ch, grid))
+            fill = sms * max(1, self.occupancy_tiled(rows[0]))
+            out.append(('tile', rows[0], 16 if 16 in chunks else chunks[0], fill))
         return out
 
     def autotune(self, steps=4, cands=None):

@@ -90,8 +90,8 @@ int batch_stage_tiled_t(const clv_params* pp, int step, const clv_batch* b, int 
     return clv_host::set_error(CLV_ERR_INVALID, "batch: test flags (Gubser, couplings, Riemann) are not batched");
   if (chunk < 1 || chunk > 4096) return clv_host::set_error(CLV_ERR_INVALID, "batch: chunk must be in 1..4096");
   if (rows != 64 && rows != 128) return clv_host::set_error(CLV_ERR_INVALID, "batch: rows must be 64 or 128");
-  if (p.flags & clv::FLAG_FAST) return clv_fastpath::batch_stage_tiled<real>(p, a, step, chunk, grid, s);
-  return clv::batch_launch::stage_tiled<real>(p, a, step, chunk, grid, s);
+  if (p.flags & clv::FLAG_FAST) return clv_fastpath::batch_stage_tiled<real>(p, a, step, rows, chunk, grid, s);
+  return clv::batch_launch::stage_tiled<real>(p, a, step, rows, chunk, grid, s);
 }
 
 template <class real> int batch_advance_t(const clv_params* pp, const clv_batch* b, int first, cudaStream_t s) {

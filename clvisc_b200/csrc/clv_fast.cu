@@ -148,8 +148,9 @@ int batch_stage(const clv::Params& p, const clv::BatchArgs<real>& a, int step, i
 }
 
 template <class real>
-int batch_stage_tiled(const clv::Params& p, const clv::BatchArgs<real>& a, int step, int chunk, int grid, cudaStream_t s) {
-  return clv::batch_launch::stage_tiled<real>(p, a, step, chunk, grid, s);
+int batch_stage_tiled(const clv::Params& p, const clv::BatchArgs<real>& a, int step, int rows, int chunk, int grid,
+                      cudaStream_t s) {
+  return clv::batch_launch::stage_tiled<real>(p, a, step, rows, chunk, grid, s);
 }
 
 template <class real> int batch_occupancy(bool bulk, int bs, int cap, int* n) {
@@ -166,8 +167,10 @@ template int batch_occupancy_tiled<double>(bool, int*);
 
 template int batch_stage<float>(const clv::Params&, const clv::BatchArgs<float>&, int, int, int, int, cudaStream_t);
 template int batch_stage<double>(const clv::Params&, const clv::BatchArgs<double>&, int, int, int, int, cudaStream_t);
-template int batch_stage_tiled<float>(const clv::Params&, const clv::BatchArgs<float>&, int, int, int, cudaStream_t);
-template int batch_stage_tiled<double>(const clv::Params&, const clv::BatchArgs<double>&, int, int, int, cudaStream_t);
+template int batch_stage_tiled<float>(const clv::Params&, const clv::BatchArgs<float>&, int, int, int, int,
+                                      cudaStream_t);
+template int batch_stage_tiled<double>(const clv::Params&, const clv::BatchArgs<double>&, int, int, int, int,
+                                       cudaStream_t);
 
 template int visc_stage<float>(const clv::Params&, const clv::ViscBuffers<float>&, int, const clv::TauConst<float>&,
                                const clv::StageOpts&, cudaStream_t);

@@ -313,14 +313,13 @@ int clv_batch_advance(const clv_params *p, const clv_batch *b, int first, void *
 /* Resident blocks per SM of the batch stage kernel at block_size threads. */
 int clv_batch_occupancy(const clv_params *p, int block_size, int max_registers, int *blocks_per_sm);
 /* The same stage for batches of (2+1)D events with the tiled kernel: work
- * items are patches of cells, taken in order by grid_blocks persistent blocks
- * (grid_blocks <= 0, or above the resident blocks of the GPU: fill it once).
- * rows must be 64 or 128 and chunk 1 to 4096: the strips of (rows - 4) y rows
- * by chunk x planes whose values the patches give. The kernel chooses its patch
- * itself, so neither changes the launch; in the FP32 tolerance build chunk
+ * items are patches of cells, taken in order by persistent blocks, as many as
+ * the patches of grid_blocks strips of (rows - 4) y rows by chunk x planes, at
+ * most one wave (grid_blocks <= 0: one wave). rows must be 64 or 128 and chunk 1
+ * to 4096. The patches give the strips' values: in the FP32 tolerance build chunk
  * enters the last bit of the planes where a strip starts. Every event must have
  * nz = 1: the kernel gives events with nz != 1 no patches. Exact build: same
- * bits as clv_batch_stage, for any chunk. */
+ * bits as clv_batch_stage, for any launch shape. */
 int clv_batch_stage_tiled(const clv_params *p, int step, const clv_batch *b, int rows, int chunk, int grid_blocks,
                           void *stream);
 /* Resident blocks per SM of the tiled batch stage kernel. */
