@@ -463,7 +463,8 @@ int clv_visc_steps(const clv_params* pp, int nsteps, const double* tau, const cl
     rc = stage(1, tau[n], &s1);
     if (rc) return rc;
     s2.edmax_key = n == nsteps - 1 ? b2->edmax_key : nullptr;
-    if (s2.edmax_key) cudaMemsetAsync(s2.edmax_key, 0, pp->precision, S(stream));
+    if (s2.edmax_key && cudaMemsetAsync(s2.edmax_key, 0, pp->precision, S(stream)) != cudaSuccess)
+      return cuda_check("cudaMemsetAsync");
     rc = stage(2, tau[n + 1], &s2);
     if (rc) return rc;
   }

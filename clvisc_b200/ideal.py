@@ -104,6 +104,11 @@ def load_eos(cfg, handcrafted_eos, device):
     return eos, torch.from_numpy(table.reshape(-1)).to(device), meta, eos.f_ed(cfg.TFRZ)
 
 
+def stock(obj, cls, names):
+    """Whether the methods of obj named are cls's own, in its class and on the object."""
+    return all(getattr(type(obj), f) is getattr(cls, f) and f not in vars(obj) for f in names)
+
+
 class CLIdeal(object):
     """Ideal hydro (pyvisc/ideal.py:28)."""
 
@@ -120,6 +125,7 @@ class CLIdeal(object):
         self.size = self.cfg.NX * self.cfg.NY * self.cfg.NZ
         self.ld = plane_stride(self.size)
         self.tau = self.cfg.real(self.cfg.TAU0)
+        self._times = self._maxima = None  # host arrays of the library's step calls
 
         self.eos, self.eos_table, meta, self.efrz = load_eos(self.cfg, handcrafted_eos, self.device)
         # effective chemical potentials on the freeze-out surface (ideal.py:65)
@@ -252,20 +258,32 @@ class CLIdeal(object):
         if jet_eloss_src is not None and jet_eloss_src.get('switch_on', False):
             raise NotImplementedError('jet energy-loss sources are not part of this backend')
 
-    def _stage(self, step, key=None):
+    def _stage(self, step):
         self._call('clv_ideal_stage', int(step), float(self.tau), _lib.ptr(self.d_ev[step]), _lib.ptr(self.d_ev[1]),
-                   _lib.ptr(self.d_ev[3 - step]), _lib.ptr(self.d_Src), 1, _lib.ptr(key), self.stream)
+                   _lib.ptr(self.d_ev[3 - step]), _lib.ptr(self.d_Src), 1, None, self.stream)
+
+    def times(self, loop, n):
+        """The present tau and update_time's after each of n steps from `loop`,
+        as the array the library takes (one a run, kept: building a ctypes array
+        type costs up to 50 us after a garbage collection)."""
+        if self._times is None or len(self._times) < n + 1:
+            self._times = (ctypes.c_double * max(n + 1, 64))()
+        self._times[0] = float(self.tau)
+        for k in range(n):
+            self._times[k + 1] = float(self.cfg.real(self.cfg.TAU0 + (loop + k + 1) * self.cfg.DT))
+        return self._times
 
     def _steps(self, loop, n, stop_below=None):
         """Up to n time steps from `loop` in one call of the library, ending
         after a step whose maximum energy density is below stop_below: (steps
         taken, the maximum after each)."""
-        tau = [float(self.tau)] + [float(self.cfg.real(self.cfg.TAU0 + (loop + k + 1) * self.cfg.DT)) for k in range(n)]
-        out = (ctypes.c_double * n)()
-        done = ctypes.c_int()
-        self._call('clv_ideal_steps', int(n), (ctypes.c_double * (n + 1))(*tau), _lib.ptr(self.d_ev[1]),
-                   _lib.ptr(self.d_ev[2]), _lib.ptr(self.d_Src), _lib.ptr(self._key),
-                   float('-inf') if stop_below is None else float(stop_below), out, ctypes.byref(done), self.stream)
+        tau = self.times(loop, n)
+        if self._maxima is None or len(self._maxima) < n:
+            self._maxima = (ctypes.c_double * max(n, 64))()
+        out, done = self._maxima, ctypes.c_int()
+        self._call('clv_ideal_steps', int(n), tau, _lib.ptr(self.d_ev[1]), _lib.ptr(self.d_ev[2]),
+                   _lib.ptr(self.d_Src), _lib.ptr(self._key), float('-inf') if stop_below is None else float(stop_below),
+                   out, ctypes.byref(done), self.stream)
         return done.value, [self.cfg.real(v) for v in out[:done.value]]
 
     def max_energy_density(self):
@@ -331,9 +349,8 @@ class CLIdeal(object):
         """Main loop (ideal.py:322-349)."""
         # the steps up to the next output go out in one call, whose second
         # stages fold the maximum of the state they write (a subclass's own
-        # stages keep the separate calls)
-        own = all(getattr(type(self), f) is getattr(CLIdeal, f)
-                  for f in ('stepUpdate', 'max_energy_density', 'update_time'))
+        # stages, times or surface keep the separate calls)
+        own = stock(self, CLIdeal, ('stepUpdate', '_stage', 'max_energy_density', 'update_time', 'get_hypersf'))
         ahead = []  # the maxima of the states the last call went through
         n = 0
         while n < max_loops:

@@ -27,7 +27,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .ideal import CLIdeal, add_visc_params
+from .ideal import CLIdeal, add_visc_params, stock
 
 
 class CLVisc(object):
@@ -129,7 +129,20 @@ class CLVisc(object):
     def step(self, loop, edmax=False):
         """One fused time step: both Runge-Kutta stages, pi and T^{tau mu}
         together (visc.py:527-544)."""
-        self._steps(loop, 1, edmax)
+        if self._own('update_time', '_stage', '_buffers'):
+            return self._steps(loop, 1, edmax)
+        both = _lib.CLV_PART_IS | _lib.CLV_PART_KT
+        self._stage(1, both, fused=True)
+        self.update_time(loop)
+        if edmax:
+            self._call('clv_max_ed_reset', _lib.ptr(self._key), self.stream)
+        self._stage(2, both, fused=True, edmax=edmax)
+
+    def _own(self, *names):
+        """Whether these methods are this class's (a subclass's or an object's
+        own are called stage by stage, where the steps are not handed over
+        together), and the time is CLIdeal's."""
+        return stock(self, CLVisc, names) and stock(self.ideal, CLIdeal, ('update_time',))
 
     def _steps(self, loop, n, edmax=False):
         """Fused time steps loop .. loop+n-1 in one call of the library, which
@@ -137,15 +150,14 @@ class CLVisc(object):
         than a small (2+1)D stage takes on the device (121 x 121 cells, 20
         steps: 485 us with a call a stage, 434 with one call). The last step
         folds the maximum energy density into the key with edmax=True."""
-        tau = (ctypes.c_double * (n + 1))(float(self.ideal.tau))
-        for k in range(n):
-            self.update_time(loop + k)
-            tau[k + 1] = float(self.ideal.tau)
+        tau = self.ideal.times(loop, n)
         both = _lib.CLV_PART_IS | _lib.CLV_PART_KT
         b1 = self._buffers(1, both, fused=True)
         b2 = self._buffers(2, both, fused=True, edmax=edmax)
         _lib.check(self.lib.clv_visc_steps(ctypes.byref(self.params), n, tau, ctypes.byref(b1), ctypes.byref(b2),
                                            self.stream), 'clv_visc_steps')
+        if n:
+            self.update_time(loop + n - 1)
 
     def read_edmax_key(self):
         out = ctypes.c_double()
@@ -243,12 +255,14 @@ class CLVisc(object):
             n = c.ntskip - loop % c.ntskip
             if is_finished and save_hypersf:
                 n = 1  # a forced run looks for the surface at every step from here on
+            if save_hypersf and not self._own('get_hypersf'):
+                n = 1  # a subclass's own surface is asked for at every step
             if force_run_to_maxloop and max_loops > loop:
                 n = min(n, max_loops - loop)
             edmax_pending = (loop + n) % c.ntskip == 0
-            if type(self).step is CLVisc.step:
+            if self._own('step', 'update_time', '_stage', '_buffers'):
                 self._steps(loop, n, edmax=edmax_pending)
-            else:  # a subclass's own step
+            else:
                 for k in range(n):
                     self.step(loop + k, edmax=edmax_pending and k == n - 1)
             loop = loop + n
