@@ -984,32 +984,28 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* part,
 // was one chain of S dependent reads on a nearly empty chip (20 us a launch, 29
 // launches a training step). A block takes 32 outputs: its 32 warps bring
 // the partials to shared memory, one adds them.
-constexpr int RED_ROWS = 320;
+constexpr int RED_ROWS = 320;  // partials at most (the callers have up to 296)
 __global__ void __launch_bounds__(1024) reduce_few_kernel(const float* part, int S, long long n, float* out,
                                                           int accumulate) {
   after_previous();
   __shared__ float sh[RED_ROWS][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long long i = (long long)blockIdx.x * 32 + lane;
+  float v[RED_ROWS / 32];
+#pragma unroll
+  for (int q = 0; q < RED_ROWS / 32; q++)
+    v[q] = i < n && w + 32 * q < S ? part[(long long)(w + 32 * q) * n + i] : 0.0f;
+#pragma unroll
+  for (int q = 0; q < RED_ROWS / 32; q++) sh[w + 32 * q][lane] = v[q];
+  __syncthreads();
+  if (w != 0 || i >= n) return;
   float s = 0.0f;
-  for (int k0 = 0; k0 < S; k0 += RED_ROWS) {
-    const int m = min(RED_ROWS, S - k0);
-    float v[RED_ROWS / 32];
-#pragma unroll
-    for (int q = 0; q < RED_ROWS / 32; q++)
-      v[q] = i < n && w + 32 * q < m ? part[(long long)(k0 + w + 32 * q) * n + i] : 0.0f;
-    if (k0) __syncthreads();
-#pragma unroll
-    for (int q = 0; q < RED_ROWS / 32; q++) sh[w + 32 * q][lane] = v[q];
-    __syncthreads();
-    if (w == 0 && i < n)
 #pragma unroll 16
-      for (int k = 0; k < m; k++) s += sh[k][lane];
-  }
-  if (w == 0 && i < n) out[i] = accumulate ? out[i] + s : s;
+  for (int k = 0; k < S; k++) s += sh[k][lane];
+  out[i] = accumulate ? out[i] + s : s;
 }
 inline void reduce_partials(const float* part, int S, long long n, float* out, int accumulate, cudaStream_t s) {
-  if (n < 65536) clv::launch_early(reduce_few_kernel, (unsigned int)((n + 31) / 32), 1024, 0, s, part, S, n, out,
+  if (n < 65536 && S <= RED_ROWS) clv::launch_early(reduce_few_kernel, (unsigned int)((n + 31) / 32), 1024, 0, s, part, S, n, out,
                         accumulate);
   else clv::launch_early(reduce_partials_kernel, (unsigned int)((n + 255) / 256), 256, 0, s, part, S, n, out,
                         accumulate);
