@@ -312,7 +312,7 @@ int ideal_stage_t(const clv::Params& p, int step, double tau, const void* ev_st,
   // FP32, one stage: 608 us per cell, 390 tiled), patches on (2+1)D grids, the
   // per-cell kernel on the short eta axes between (2 to 23 cells): the same
   // bits.
-  if (p.nz >= kTiledMinNz && clv::fits_idx32<real>(p)) return launch_ideal_tiled<real>(p, b, step, tau, s);
+  if (p.nz >= kTiledMinNz && clv::fits_idx32<real>(p) && (p.ny + 7) / 8 <= 65535) return launch_ideal_tiled<real>(p, b, step, tau, s);
   if (p.nz == 1 && clv::fits_idx32<real>(p) && (p.nx + 7) / 8 <= 65535) {
     clv::launch_early(clv::ideal_stage_patch_kernel<real, 8, 8, 64>, dim3((p.ny + 7) / 8, (p.nx + 7) / 8), 64, 0, s, p, b,
                       step, tau_const<real>(p, tau));

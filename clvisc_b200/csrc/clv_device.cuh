@@ -103,17 +103,18 @@ template <> struct Acu<double> { static constexpr double v = 1.0E-14; };
 // fill the chip, where a fixed 32 left small grids half empty. From 5 to 32
 // planes, with four waves of CTAs or more, the one with the least planes in
 // whole waves (0.7 of a plane more each); 5 where the grid has no four waves.
-// B200, two steps: 97x93x65 exact 5 planes 2.14 ms, 32 3.84; 201x201x105 FP32
-// 12 planes 3.10, 8 3.15, 13 3.22, 32 3.85; 161x145x77 FP64 9 planes 3.42, 10
-// 3.63; 385x385x115 FP32 22 planes 11.02, 30 11.25, 129 11.96.
+// B200, two steps: 97x93x65 exact 5 planes 2.20 ms, 8 2.41, 32 4.02; 201x201x105
+// FP32 12 planes 3.38, 8 3.43, 13 3.49, 32 3.97; 161x145x77 FP64 9 planes 3.56, 10
+// 3.79, 32 3.64; 385x385x115 FP32 22 planes 11.9, 30 12.1, 129 12.2.
 inline int march_chunk(int nx, long long columns, int slots) {
-  int best = 5;
+  const int from = nx > 5 * 65535 ? (nx + 65534) / 65535 : 5;  // grid.z
+  int best = from;
   double least = 0.0;
-  for (int c = 5; c <= 32; c++) {
+  for (int c = from; c <= 32; c++) {
     const long long blocks = columns * ((nx + c - 1) / c);
     if (blocks < 4ll * slots) break;
     const double cost = (double)((blocks + slots - 1) / slots) * (c + 0.7);
-    if (c == 5 || cost < least) best = c, least = cost;
+    if (c == from || cost < least) best = c, least = cost;
   }
   return best;
 }
