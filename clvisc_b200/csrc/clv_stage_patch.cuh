@@ -33,17 +33,17 @@ template <class real, bool BULK, int TX, int TY> struct PatchSmem {
 // Patch shapes. FP32: 8 x 16 cells on 128 threads, four or five blocks an SM;
 // where that leaves SMs without a block (fewer patches than SMs: a single event
 // below about 150 x 150 cells), 4 x 8 cells on 96 threads. FP64: 8 x 8 on 64.
-// B200, 20 steps of one event, tolerance build, FP32: 301 x 301 0.67 ms (8 x 16)
-// against 0.88 (8 x 8), 0.93 (4 x 8) and 1.19 (one thread a cell); 61 x 61 0.36
-// (4 x 8) against 0.43 (8 x 16) and 0.59; FP64 301 x 301 1.57 (8 x 8, 64
-// threads) against 1.92 (96 threads) and 2.18.
+// B200, 20 steps of one event, tolerance build, FP32: 301 x 301 0.70 ms (one
+// thread a cell 1.30, strips that march 2.2), 145 x 145 0.59 (0.72), 121 x 121 0.39
+// (0.66), 61 x 61 0.37 (0.61); FP64 301 x 301 1.57 (2.30). Measured against each
+// other with another record, the shapes were: 301 x 301 8 x 16 0.67, 8 x 8 0.88,
+// 4 x 8 0.93; 61 x 61 4 x 8 0.36, 8 x 16 0.43; FP64 64 threads 1.57, 96 1.92.
 template <class real, bool BULK> struct PatchWide {
   static constexpr int TX = 8, TY = sizeof(real) == 4 ? 16 : 8, NT = sizeof(real) == 4 ? 128 : 64;
   static constexpr int MINB = sizeof(real) == 4 ? (BULK ? 4 : 5) : 4;
 };
-template <class real, bool BULK> struct PatchSmall {
-  static constexpr int TX = sizeof(real) == 4 ? 4 : 8, TY = 8, NT = sizeof(real) == 4 ? 96 : 64;
-  static constexpr int MINB = sizeof(real) == 4 ? 5 : 4;
+struct PatchSmall {  // FP32
+  static constexpr int TX = 4, TY = 8, NT = 96, MINB = 5;
 };
 
 inline namespace CLV_ARITH {
@@ -207,8 +207,10 @@ template <class real, bool BULK>
 cudaError_t launch_patch(const Params& p, const ViscBuffers<real>& v, int step, const TauConst<real>& tc,
                          cudaStream_t s) {
   typedef PatchWide<real, BULK> W;
-  const long long wide = (long long)((p.ny + W::TY - 1) / W::TY) * ((p.nx + W::TX - 1) / W::TX);
-  if (wide < sm_count()) return launch_patch_shape<real, BULK, PatchSmall<real, BULK>>(p, v, step, tc, s);
+  if constexpr (sizeof(real) == 4) {
+    const long long wide = (long long)((p.ny + W::TY - 1) / W::TY) * ((p.nx + W::TX - 1) / W::TX);
+    if (wide < sm_count()) return launch_patch_shape<real, BULK, PatchSmall>(p, v, step, tc, s);
+  }
   return launch_patch_shape<real, BULK, W>(p, v, step, tc, s);
 }
 // grid.y of the patch launches: patches of 4 cells along x

@@ -349,13 +349,12 @@ __device__ __forceinline__ void rec2_start(const ViscBuffers<real>& b, long long
 
 // One tile: rows j0 .. j0+TB-5 of planes i0 .. i1-1 of the event (gd, b).
 // Every thread of the block calls it (it holds barriers).
-template <class real, bool BULK, int TB, int STAGE = 0>
-__device__ __forceinline__ void tile2d(const Params& p, const GridDims& gd, const ViscBuffers<real>& b, int step_,
+template <class real, bool BULK, int TB>
+__device__ __forceinline__ void tile2d(const Params& p, const GridDims& gd, const ViscBuffers<real>& b, int step,
                                        const TauConst<real>& tc, int j0, int i0, int i1, Tile2Smem<real, BULK, TB>& s) {
   typedef Rec2<BULK> R;
   typedef Rec2L<real, BULK> L;
   constexpr int NC = R::NCOMP, NP = L::NP, CP = L::CP, RG = L::RG, CG = L::CG;
-  const int step = STAGE ? STAGE : step_;
   const real tau = tc.tau;
   const Recips<real>& rc = recips<real>(p);
   const long long ld = gd.ld;
@@ -459,7 +458,7 @@ __device__ __forceinline__ void tile2d(const Params& p, const GridDims& gd, cons
       real pinew[11];
       cell_in_ev1<real>(p, b, I, ld, cin);
       real pstart[R::NPI];  // pi at the start of the step: at stage 1 the stage input's
-      rec2_start<real, BULK, STAGE>(b, I, ld, pc, pstart);
+      rec2_start<real, BULK, 0>(b, I, ld, pc, pstart);
       pi_update<real, false, BULK>(p, b, step, tc, I, ld, cin, pc, grad, S10, pinew,
                                    [&](int m, real u) { return pstart[m] * u; });
       ev_update<real, true, BULK>(p, b, step, tc, I, ld, cin, pin, S4, pinew);
