@@ -8,8 +8,10 @@ Runge-Kutta stage. Per event it reproduces CLVisc exactly: the construction
 sequence (pi initialised from the empty state, one ideal stage on it,
 visc.py:101-102), load_ini, and evolve's loop (visc.py:473-560) with the
 fused stages, the maximum energy density recorded with tau every ntskip steps
-and the stop when it falls below the freeze-out energy density, so each
-event's fields are bit-identical to a CLVisc run of that event alone. The stop
+and the stop when it falls below the freeze-out energy density. In the exact
+build each event's fields are bit-identical to a CLVisc run of that event alone;
+in the tolerance build a step agrees within its tolerance, and a run may stop a
+check earlier or later. The stop
 test runs on the device; evolve() captures ntskip steps in a CUDA graph and
 replays it until every event has stopped.
 

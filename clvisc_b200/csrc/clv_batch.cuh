@@ -7,8 +7,8 @@
 // ld_e. A persistent kernel walks the flattened cells of the events that are
 // still running (a compacted list and a prefix of their cell counts, rebuilt on
 // the device after each step) and applies to each cell the same fused stage as
-// the single-event kernel (visc_stage_cell), so every event evolves bit for bit
-// as it would alone. tau, the step counter, the stop test and the per-event
+// the single-event kernel (visc_stage_cell), so in the exact build every event
+// evolves bit for bit as it would alone. tau, the step counter, the stop test and the per-event
 // history live in device memory, so a block of steps can be captured in one CUDA
 // graph and replayed without host work between steps.
 //

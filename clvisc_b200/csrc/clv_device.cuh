@@ -204,7 +204,7 @@ __device__ __forceinline__ double fast_floor(double x, int& i) {
 #endif
 // a product that is never contracted into a sum
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
 // ------------------------------------------------------------------ EOS
 // Table lookup of eos_table.h:39-62: row/col from the energy density, two
 // nearest texels (the second wraps to the next row), clamp-to-edge, lerp.

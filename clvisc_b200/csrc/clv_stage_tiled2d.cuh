@@ -20,8 +20,8 @@
 //     x face and slope travel in registers from one plane to the next.
 //   * Along eta (one cell) nothing but the Christoffel part of the velocity
 //     gradient remains, as in visc_stage_cell's one-cell-axis branch.
-// Each record, slope and face flux is the per-cell kernel's expression, so the
-// results are identical bit for bit.
+// In the exact build each record, slope and face flux is the per-cell kernel's
+// expression, so the results are identical bit for bit.
 #pragma once
 #include "clv_smem16.cuh"
 #include "clv_stage.cuh"

@@ -126,8 +126,9 @@ typedef struct clv_visc_buffers {
  * thread block marches through (the process-wide default, 32, lets the grid
  * decide; a run's own opt_chunk is taken as it is), and the number of tiled
  * blocks kept resident per SM in
- * FP32 (1 or 2; FP64 uses 1). Every variant computes the same values bit for
- * bit. */
+ * FP32 (1 or 2; FP64 uses 1). In the exact build every variant computes the
+ * same values bit for bit; in the tolerance build the variants agree within its
+ * tolerance (1e-5 FP32, 1e-11 FP64 of each field's scale). */
 #define CLV_OPT_STAGE_KERNEL 1
 #define CLV_OPT_CHUNK 2
 #define CLV_OPT_TILED_BLOCKS 3
@@ -259,7 +260,8 @@ int clv_hypersf_append_noalloc(const clv_params *p, int visc, double tau_old, do
  * with CLV_FLAG_BULK), the sources at off_src (14, or 15), goodcell at byte
  * off_cell. The clv_params of a batch carry the shared constants; its nx, ny,
  * nz, ld describe no event (set them to the largest event). Each event evolves
- * bit for bit as CLVisc.evolve would evolve it alone (visc.py:473-560):
+ * as CLVisc.evolve would evolve it alone (visc.py:473-560; exact build: bit for
+ * bit, tolerance build: within its tolerance a step):
  * both Runge-Kutta stages fused, the maximum energy density recorded with tau
  * at every multiple of ntskip steps, the event stopping when that maximum is
  * below efrz. Gubser, coupling and Riemann test flags are not batched. */
